@@ -51,6 +51,37 @@ RT_DEV float slab_near(F3 o, F3 inv, F3 lo, F3 hi, float tmin, float tmax) {
   return near <= far ? near : BIG;
 }
 
+// Two f32 lanes of one 64-bit register pair (sm_100's packed f32 instructions): each lane rounds on
+// its own exactly as __fmul_rn, __fadd_rn and __fmaf_rn do, at one issue slot for both. The compiler
+// fuses a mul2 whose only use is an add2 (checked on the device: .rn does not stop it), so where
+// the product and the sum must round apart, the products are taken one by one (pack2 of two mul).
+struct P2 {
+  unsigned long long v;
+};
+RT_DEV P2 pack2(float a, float b) {
+  P2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+RT_DEV P2 both(float a) { return pack2(a, a); }
+RT_DEV float first(P2 p) { return __uint_as_float((uint32_t)p.v); }
+RT_DEV float second(P2 p) { return __uint_as_float((uint32_t)(p.v >> 32)); }
+RT_DEV P2 mul2(P2 a, P2 b) {
+  P2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+RT_DEV P2 add2(P2 a, P2 b) {
+  P2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+RT_DEV P2 fma2(P2 a, P2 b, P2 c) {
+  P2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
 RT_DEV uint32_t ld(const uint32_t* __restrict__ w, size_t i) { return __ldg(w + i); }
 RT_DEV float ldf(const uint32_t* __restrict__ w, size_t i) { return __uint_as_float(__ldg(w + i)); }
 RT_DEV F3 ld3(const uint32_t* __restrict__ w, size_t i) { return {ldf(w, i), ldf(w, i + 1), ldf(w, i + 2)}; }
@@ -64,6 +95,26 @@ RT_DEV uint4 ld4(const uint32_t* __restrict__ w, size_t i) {
 RT_DEV uint4 ld4u(const uint32_t* __restrict__ w, size_t i) {
   if ((i & 3) == 0) return __ldg(reinterpret_cast<const uint4*>(w + i));
   return make_uint4(__ldg(w + i), __ldg(w + i + 1), __ldg(w + i + 2), __ldg(w + i + 3));
+}
+
+// The sixteen words of a node record at any word offset. On a 16-byte boundary: four 16-byte loads.
+// Elsewhere (a GI mesh that follows another): the four that begin at or before it and the last one
+// to three words, shifted into place by the offset's low bits, instead of sixteen word loads.
+RT_DEV void ld16(const uint32_t* __restrict__ w, size_t i, uint4 (&n)[4]) {
+  const uint32_t m = (uint32_t)i & 3u;
+  const uint4* p = reinterpret_cast<const uint4*>(w + (i - m));
+  n[0] = __ldg(p), n[1] = __ldg(p + 1), n[2] = __ldg(p + 2), n[3] = __ldg(p + 3);
+  if (m == 0) return;
+  const uint32_t* tail = reinterpret_cast<const uint32_t*>(p + 4);
+  uint32_t x[19] = {n[0].x, n[0].y, n[0].z, n[0].w, n[1].x, n[1].y, n[1].z, n[1].w, n[2].x, n[2].y,
+                    n[2].z, n[2].w, n[3].x, n[3].y, n[3].z, n[3].w, __ldg(tail), m > 1 ? __ldg(tail + 1) : 0u,
+                    m > 2 ? __ldg(tail + 2) : 0u};
+#pragma unroll
+  for (int k = 0; k < 18; ++k) x[k] = (m & 1u) ? x[k + 1] : x[k];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) x[k] = (m & 2u) ? x[k + 2] : x[k];
+  n[0] = make_uint4(x[0], x[1], x[2], x[3]), n[1] = make_uint4(x[4], x[5], x[6], x[7]);
+  n[2] = make_uint4(x[8], x[9], x[10], x[11]), n[3] = make_uint4(x[12], x[13], x[14], x[15]);
 }
 
 struct Ray {
@@ -85,6 +136,16 @@ RT_DEV Ray load_ray_cs(const float4* __restrict__ rays, uint32_t i) {
 template <bool CS>
 RT_DEV Ray load_ray_as(const float4* __restrict__ rays, uint32_t i) {
   return CS ? load_ray_cs(rays, i) : load_ray(rays, i);
+}
+
+// The world ray in object space, by an instance record's three rows (world to object).
+RT_DEV void to_object(uint4 q0, uint4 q1, uint4 q2, const Ray& ray, F3& o, F3& d) {
+  const F3 r0 = {__uint_as_float(q0.x), __uint_as_float(q0.y), __uint_as_float(q0.z)};
+  const F3 r1 = {__uint_as_float(q1.x), __uint_as_float(q1.y), __uint_as_float(q1.z)};
+  const F3 r2 = {__uint_as_float(q2.x), __uint_as_float(q2.y), __uint_as_float(q2.z)};
+  o = {dot4p(r0.x, r0.y, r0.z, __uint_as_float(q0.w), ray.o), dot4p(r1.x, r1.y, r1.z, __uint_as_float(q1.w), ray.o),
+       dot4p(r2.x, r2.y, r2.z, __uint_as_float(q2.w), ray.o)};
+  d = {dot3(r0, ray.d), dot3(r1, ray.d), dot3(r2, ray.d)};
 }
 
 // One ray batch of a many-batch launch, as the device reads it (32 bytes).

@@ -1,36 +1,43 @@
 // FAST traversal kernels: the PLAIN per-ray arithmetic and visit order, rescheduled.
 //
 // Each ray performs exactly the operations of rs_trace / gi_traverse in the same order (so its
-// hit is bit-identical), but the loop is flattened into a per-lane state machine -- one node,
-// one leaf or one top-level step per iteration -- inside persistent warps that refill a lane
-// with the next ray as soon as its ray ends (warp-aggregated atomics on a global ray counter).
-// Lanes therefore stop idling behind the longest ray of their warp, and the divergent nested
-// loops of the direct transcription become one reconverging loop.
+// hit is bit-identical), but the loop is flattened into a per-lane state machine -- one top-level
+// node, instance entry, BLAS node or leaf a step -- inside persistent warps that refill lanes with
+// new rays as rays end (warp-aggregated atomics on a global ray counter).
 //
-// Quantised planes are decoded without integer-to-float conversions: for a byte q,
-// as_float(0x4B000000 | q) - 2^23 is q exactly, an integer OR and one FP32 subtract.
+// What bounds them: instruction issue. Lanes of one warp wait for different kinds of step, and a
+// warp that runs every kind each time around executes each for a fourth of its lanes (6.7 of 32
+// active on 1.05M gather rays over 400 instances, 59 % of issue slots taken, 6.3 G instructions).
+// So the warp votes and runs the one step that most lanes wait for, the others keep theirs
+// (vote_phase): 11.9 lanes active, 4.3 G instructions. Running every step with at least 6, 8 or 12
+// lanes waiting as well was slower (6.78, 6.35 and 6.23 against 6.08 ms there), and so were weights
+// by a step's length. Each is resident 7 times an SM (72 registers): 4, 5, 6 and 8 blocks gave 6.65,
+// 6.63, 6.10 and 6.12 against 6.09 ms; the closest hit therefore keeps no more than t, u, v and where
+// its triangle is, and the record is made when the ray ends. Together, before and after (us):
+//   gather of 16,384 cells over 400 instances, closest   9,530 -> 6,160
+//   16,384 cells x 40 lights, 250k triangles, any hit      508 ->   438
+//   1M GI rays, 250k triangles, GI / reflection          1,876 / 1,455 -> 1,320 / 1,000
+//   1M camera rays, the same scene                         989 /   765 ->   765 /   600
 #pragma once
 #include "plain.cuh"
 
 namespace rtk {
 
-// q as float, exactly (q <= 255 < 2^23).
-RT_DEV float byte_f(uint32_t word, uint32_t shift) {
-  return __fsub_rn(__uint_as_float(0x4B000000u | ((word >> shift) & 0xffu)), 8388608.0f);
-}
+constexpr int FAST_MIN_BLOCKS = 7;  // of 128 threads an SM (72 registers)
 
 // Persistent-kernel ray distribution: every lane that needs a ray takes the next index of the
 // launch; one atomic per warp per refill round.
 struct RayQueue {
   unsigned int* next;  // global counter, zeroed before the launch
   uint32_t n;
-  uint32_t refill;     // idle lanes a warp waits for before taking more rays (1-32)
+  uint32_t refill;     // idle lanes a warp waits for before taking more rays (1-width)
+  uint32_t width;      // lanes of a warp that take rays (1-32): fewer than 32 where n rays do not fill the GPU
 };
 
 // Called by all 32 lanes together. `drained` (warp-uniform) stops the requests once the
 // counter has passed the end, so finished warps add no atomic traffic.
 RT_DEV uint32_t take_ray(const RayQueue& q, bool need, bool& drained) {
-  const unsigned idle = __ballot_sync(0xffffffffu, need);
+  const unsigned idle = __ballot_sync(0xffffffffu, need && (threadIdx.x & 31) < q.width);
   const unsigned want = (!drained && (uint32_t)__popc(idle) >= q.refill) ? idle : 0u;
   if (!want) return EMPTY;
   const int lane = threadIdx.x & 31;
@@ -40,12 +47,57 @@ RT_DEV uint32_t take_ray(const RayQueue& q, bool need, bool& drained) {
   base = __shfl_sync(0xffffffffu, base, leader);
   if (base + (uint32_t)__popc(want) >= q.n) drained = true;
   const uint32_t idx = base + __popc(want & ((1u << lane) - 1u));
-  return (need && (want >> lane & 1u) && idx < q.n) ? idx : EMPTY;
+  return ((want >> lane & 1u) && idx < q.n) ? idx : EMPTY;
+}
+
+// ---------------------------------------------------------------- the walk's schedule
+
+// What a lane does next. PH_DONE: its ray has ended and its result is not stored yet.
+enum : uint32_t { PH_IDLE = 0, PH_TOP = 1, PH_ENTER = 2, PH_NODE = 3, PH_LEAF = 4, PH_DONE = 5 };
+
+// The step that the warp runs next: the one that most of its lanes wait for (PH_IDLE: none does).
+// Called by all 32 lanes; the same answer in each.
+RT_DEV uint32_t vote_phase(uint32_t phase) {
+  const bool waits = phase - PH_TOP <= PH_LEAF - PH_TOP;
+  const uint32_t votes = __reduce_add_sync(0xffffffffu, waits ? 1u << (8 * (phase - PH_TOP)) : 0u);
+  uint32_t best = PH_IDLE, most = 0;
+#pragma unroll
+  for (uint32_t p = PH_TOP; p <= PH_LEAF; ++p) {
+    const uint32_t c = (votes >> (8 * (p - PH_TOP))) & 0xffu;
+    if (c > most) most = c, best = p;
+  }
+  return best;
+}
+
+// Byte c of `word` as a float, exactly: as_float(0x4B000000 | q) - 2^23.
+RT_DEV float byte_f(uint32_t word, uint32_t c) {
+  return __fsub_rn(__uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540u | c)), 8388608.0f);
+}
+
+// slab_near of a BVH4-Q8 node's four children, planes decoded as base + q * step with each product
+// and sum rounded on its own (see P2: the products are taken one by one), the sums and the rest two
+// children to an instruction. 1M GI rays, reflection: 1,000 us against 1,050 one child at a time.
+RT_DEV void child_slabs(F3 base, F3 step, uint32_t lx, uint32_t ly, uint32_t lz, uint32_t hx, uint32_t hy, uint32_t hz, F3 o,
+                        F3 inv, float tmin, float tmax, float (&dist)[4]) {
+#pragma unroll
+  for (uint32_t c = 0; c < 4; c += 2) {
+    auto plane = [&](uint32_t word, float b, float s, float at, float iv) {
+      return mul2(add2(add2(pack2(mul(byte_f(word, c), s), mul(byte_f(word, c + 1), s)), both(b)), both(-at)), both(iv));
+    };
+    const P2 ax = plane(lx, base.x, step.x, o.x, inv.x), bx = plane(hx, base.x, step.x, o.x, inv.x);
+    const P2 ay = plane(ly, base.y, step.y, o.y, inv.y), by = plane(hy, base.y, step.y, o.y, inv.y);
+    const P2 az = plane(lz, base.z, step.z, o.z, inv.z), bz = plane(hz, base.z, step.z, o.z, inv.z);
+    auto entry = [&](float x0, float x1, float y0, float y1, float z0, float z1) {
+      const float near = fmaxf(fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fminf(z0, z1)), tmin);
+      const float far = fminf(fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fmaxf(z0, z1)), tmax);
+      return near <= far ? near : BIG;
+    };
+    dist[c] = entry(first(ax), first(bx), first(ay), first(by), first(az), first(bz));
+    dist[c + 1] = entry(second(ax), second(bx), second(ay), second(by), second(az), second(bz));
+  }
 }
 
 // ---------------------------------------------------------------- reflection layout
-
-enum : uint32_t { PH_IDLE = 0, PH_TOP = 1, PH_BLAS = 2 };
 
 template <int AM>
 struct RsLane {
@@ -56,27 +108,50 @@ struct RsLane {
   uint32_t entry;  // batch entry (many-batch launches)
   bool any;        // any-hit ray (AM 2)
   uint32_t phase;
-  // top level (or flat list position)
-  uint32_t tsp;
-  uint32_t flat_i;
-  // current instance
+  uint32_t top_at;  // items on the top level's stack, or the next instance of a flat list
   uint32_t inst, slot;
   F3 o, d, inv;
   uint32_t nodes, tris;
-  uint32_t cur;  // child to process next, EMPTY: pop
+  uint32_t cur;  // what the next step works on: top-level node, instance, BLAS node or leaf
   uint32_t sp;
 };
 
+// The next item of the top level (or of the flat instance list).
+template <class Lane>
+RT_DEV void next_top(Lane& L, const uint32_t* top_stack, bool flat, uint32_t instances) {
+  if (flat) {
+    if (L.top_at >= instances) {
+      L.phase = PH_DONE;
+    } else {
+      L.cur = L.top_at++;
+      L.phase = PH_ENTER;
+    }
+    return;
+  }
+  if (L.top_at == 0) {
+    L.phase = PH_DONE;
+    return;
+  }
+  const uint32_t item = top_stack[--L.top_at];
+  L.cur = item & ~LEAF;
+  L.phase = (item & LEAF) ? PH_ENTER : PH_TOP;
+}
+
+template <class Lane>
+RT_DEV void set_child(Lane& L, uint32_t child) {
+  L.cur = child;
+  L.phase = (child & LEAF) ? PH_LEAF : PH_NODE;
+}
+
 template <int AM, class Src>
-RT_DEV void rs_finish(RsLane<AM>& L, const Src& src) {
+RT_DEV void rs_finish(const RsLane<AM>& L, const Src& src) {
   if (any_of<AM>(L)) {
     put_flag(src, L.entry, L.ray_id, L.ray, L.best.rec[0] != 0);
-  } else {
-    uint32_t* o = reinterpret_cast<uint32_t*>(out_of(src, L.entry)) + 5 * (size_t)L.ray_id;
-    o[0] = __float_as_uint(L.best.t), o[1] = L.best.rec[0], o[2] = L.best.rec[1], o[3] = L.best.rec[2];
-    o[4] = L.best.rec[3];
+    return;
   }
-  L.phase = PH_IDLE;
+  uint32_t* o = reinterpret_cast<uint32_t*>(out_of(src, L.entry)) + 5 * (size_t)L.ray_id;
+  o[0] = __float_as_uint(L.best.t), o[1] = L.best.rec[0], o[2] = L.best.rec[1], o[3] = L.best.rec[2];
+  o[4] = L.best.rec[3];
 }
 
 // rs_instance's entry (reflections_software_bvh4.wgsl:50-67): true when the lane now walks the
@@ -91,22 +166,14 @@ RT_DEV bool rs_enter(const uint32_t* __restrict__ w, RsLane<AM>& L, uint32_t i) 
   const F3 lo = {__uint_as_float(b0.x), __uint_as_float(b0.y), __uint_as_float(b0.z)};
   const F3 hi = {__uint_as_float(b0.w), __uint_as_float(b1.x), __uint_as_float(b1.y)};
   if (slab_near(L.ray.o, L.world_inv, lo, hi, L.ray.tmin, bound) > bound) return false;
-  const uint4 q0 = ld4(w, R), q1 = ld4(w, R + 4), q2 = ld4(w, R + 8);
-  const F3 ro = L.ray.o, rd = L.ray.d;
-  L.o = {dot4p(__uint_as_float(q0.x), __uint_as_float(q0.y), __uint_as_float(q0.z), __uint_as_float(q0.w), ro),
-         dot4p(__uint_as_float(q1.x), __uint_as_float(q1.y), __uint_as_float(q1.z), __uint_as_float(q1.w), ro),
-         dot4p(__uint_as_float(q2.x), __uint_as_float(q2.y), __uint_as_float(q2.z), __uint_as_float(q2.w), ro)};
-  L.d = {dot3({__uint_as_float(q0.x), __uint_as_float(q0.y), __uint_as_float(q0.z)}, rd),
-         dot3({__uint_as_float(q1.x), __uint_as_float(q1.y), __uint_as_float(q1.z)}, rd),
-         dot3({__uint_as_float(q2.x), __uint_as_float(q2.y), __uint_as_float(q2.z)}, rd)};
+  to_object(ld4(w, R), ld4(w, R + 4), ld4(w, R + 8), L.ray, L.o, L.d);
   L.inv = safe_inverse(L.d);
   L.nodes = b1.z & ~3u;
   L.tris = b1.w & ~3u;
   L.inst = i;
   L.slot = tail.y;
-  L.cur = tail.x;
   L.sp = 0;
-  L.phase = PH_BLAS;
+  set_child(L, tail.x);
   return true;
 }
 
@@ -117,7 +184,7 @@ RT_DEV bool rs_leaf(const uint32_t* __restrict__ w, RsLane<AM>& L, uint32_t chil
   const F3 o = L.o, d = L.d;
   for (uint32_t k = 0; k < count; ++k) {
     const size_t X = L.tris + (size_t)(start + k) * 12;
-    const uint4 w0 = ld4u(w, X), w1 = ld4u(w, X + 4), w2 = ld4u(w, X + 8);
+    const uint4 w0 = ld4(w, X), w1 = ld4(w, X + 4), w2 = ld4(w, X + 8);
     const F3 a = {__uint_as_float(w0.x), __uint_as_float(w0.y), __uint_as_float(w0.z)};
     const F3 e1 = {__uint_as_float(w0.w), __uint_as_float(w1.x), __uint_as_float(w1.y)};
     const F3 e2 = {__uint_as_float(w1.z), __uint_as_float(w1.w), __uint_as_float(w2.x)};
@@ -145,27 +212,21 @@ RT_DEV bool rs_leaf(const uint32_t* __restrict__ w, RsLane<AM>& L, uint32_t chil
   return false;
 }
 
-// One BLAS node (reflections_software_bvh4.wgsl:99-125): children sorted, the nearest kept.
+// One BLAS node (reflections_software_bvh4.wgsl:99-125): children sorted, the nearest returned
+// (EMPTY: none survives), the rest pushed far to near.
 template <int AM>
-RT_DEV void rs_node(const uint32_t* __restrict__ w, RsLane<AM>& L, uint32_t child, uint32_t* stack, DevStatus* st) {
+RT_DEV uint32_t rs_node(const uint32_t* __restrict__ w, RsLane<AM>& L, uint32_t child, uint32_t* stack, DevStatus* st) {
   const size_t N = L.nodes + (size_t)child * 16;
-  const uint4 n0 = ld4u(w, N), n1 = ld4u(w, N + 4), n2 = ld4u(w, N + 8), n3 = ld4u(w, N + 12);
+  const uint4 n0 = ld4(w, N), n1 = ld4(w, N + 4), n2 = ld4(w, N + 8), n3 = ld4(w, N + 12);
   const float lim = rs_limit(L.best, L.inst);
-  const F3 base = {__uint_as_float(n0.x), __uint_as_float(n0.y), __uint_as_float(n0.z)};
-  const F3 step = {__uint_as_float(n0.w), __uint_as_float(n1.x), __uint_as_float(n1.y)};
   uint32_t ids[4] = {n1.z, n1.w, n2.x, n2.y};
   float dist[4];
+  child_slabs({__uint_as_float(n0.x), __uint_as_float(n0.y), __uint_as_float(n0.z)},
+              {__uint_as_float(n0.w), __uint_as_float(n1.x), __uint_as_float(n1.y)}, n2.z, n2.w, n3.x, n3.y, n3.z, n3.w, L.o,
+              L.inv, L.ray.tmin, lim, dist);
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    dist[c] = BIG;
-    if (ids[c] == EMPTY) continue;
-    const uint32_t sh = 8 * c;
-    const F3 lo = {add(mul(byte_f(n2.z, sh), step.x), base.x), add(mul(byte_f(n2.w, sh), step.y), base.y),
-                   add(mul(byte_f(n3.x, sh), step.z), base.z)};
-    const F3 hi = {add(mul(byte_f(n3.y, sh), step.x), base.x), add(mul(byte_f(n3.z, sh), step.y), base.y),
-                   add(mul(byte_f(n3.w, sh), step.z), base.z)};
-    dist[c] = slab_near(L.o, L.inv, lo, hi, L.ray.tmin, lim);
-  }
+  for (int c = 0; c < 4; ++c)
+    if (ids[c] == EMPTY) dist[c] = BIG;
 #define RT_SW(a, b)                                      \
   if (dist[b] < dist[a]) {                               \
     float x = dist[a]; dist[a] = dist[b]; dist[b] = x;   \
@@ -180,24 +241,27 @@ RT_DEV void rs_node(const uint32_t* __restrict__ w, RsLane<AM>& L, uint32_t chil
       else atomicAdd(&st->stack_drops, 1ull);
     }
   }
-  L.cur = (dist[0] <= lim && ids[0] != EMPTY) ? ids[0] : EMPTY;
+  return dist[0] <= lim ? ids[0] : EMPTY;
 }
 
 template <int AM, int BLOCK, class Src>
-__global__ void __launch_bounds__(BLOCK) k_rs_fast(const uint32_t* __restrict__ w, const Src src, RayQueue queue,
-                                                   DevStatus* st) {
+__global__ void __launch_bounds__(BLOCK, FAST_MIN_BLOCKS)
+    k_rs_fast(const uint32_t* __restrict__ w, const Src src, RayQueue queue, DevStatus* st) {
   uint32_t stack[STACK];
   uint32_t top_stack[STACK];
   RsLane<AM> L;
   L.phase = PH_IDLE;
   const uint4 head = ld4(w, 0);
   const size_t bounds = ld(w, 4) & ~3u;
+  const size_t top = head.y & ~3u;
   bool drained = false;
   for (;;) {
-    // Refill idle lanes; a warp leaves when none of its lanes holds a ray.
+    // Every lane reaches the votes below once per iteration (no exit above them); the warp leaves
+    // only when no lane holds a ray and the queue is drained.
     __syncwarp();
-    const uint32_t id = take_ray(queue, L.phase == PH_IDLE, drained);
-    if (L.phase == PH_IDLE && id != EMPTY) {
+    const uint32_t id = take_ray(queue, L.phase == PH_IDLE || L.phase == PH_DONE, drained);
+    if (id != EMPTY) {
+      if (L.phase == PH_DONE) rs_finish<AM>(L, src);
       L.ray = fetch(src, id, L);
       L.world_inv = safe_inverse(L.ray.d);
       L.best.t = L.ray.tmax, L.best.rec[0] = L.best.rec[1] = L.best.rec[2] = L.best.rec[3] = 0, L.best.inst = EMPTY;
@@ -213,119 +277,114 @@ __global__ void __launch_bounds__(BLOCK) k_rs_fast(const uint32_t* __restrict__ 
         live = !(near > far);
         if (live) L.best.t = fminf(L.ray.tmax, __uint_as_float(__float_as_uint(far) + 2u));
       }
+      L.phase = PH_DONE;  // misses the scene box
       if (live) {
-        L.phase = PH_TOP;
-        L.flat_i = 0;
-        L.tsp = 1;
+        L.top_at = head.y == 0 ? 0 : 1;
         top_stack[0] = head.z;
-      } else {
-        rs_finish<AM>(L, src);  // misses the scene box: done, refilled next iteration
+        next_top(L, top_stack, head.y == 0, head.x);
       }
     }
-    // Every lane reaches this vote once per iteration (no exit above it); the warp leaves only
-    // when no lane holds a ray and the queue is drained.
-    if (!__any_sync(0xffffffffu, L.phase != PH_IDLE)) {
+    const uint32_t run = vote_phase(L.phase);
+    if (run == PH_IDLE) {
       if (drained) break;
       continue;
     }
-    if (L.phase == PH_BLAS) {
-      if (L.cur == EMPTY) {
-        if (L.sp == 0) {
-          L.phase = PH_TOP;  // instance done
-        } else {
-          L.cur = stack[--L.sp];
-        }
-      }
-      if (L.phase == PH_BLAS) {
-        const uint32_t child = L.cur;
-        if (child & LEAF) {
-          if (rs_leaf<AM>(w, L, child)) {
-            rs_finish<AM>(L, src);
-            continue;
-          }
-          L.cur = EMPTY;
-        } else {
-          rs_node<AM>(w, L, child, stack, st);
-        }
-        continue;
-      }
-    }
-    if (L.phase == PH_TOP) {
-      if (head.y == 0) {  // flat instance list
-        if (L.flat_i >= head.x) {
-          rs_finish<AM>(L, src);
-          continue;
-        }
-        rs_enter<AM>(w, L, L.flat_i++);
-        continue;
-      }
-      if (L.tsp == 0) {
-        rs_finish<AM>(L, src);
-        continue;
-      }
-      const uint32_t item = top_stack[--L.tsp];
-      if (item & LEAF) {
-        rs_enter<AM>(w, L, item & ~LEAF);
-        continue;
-      }
+    if (L.phase != run) continue;
+    if (run == PH_NODE) {
+      const uint32_t c = rs_node<AM>(w, L, L.cur, stack, st);
+      if (c != EMPTY) set_child(L, c);
+      else if (L.sp) set_child(L, stack[--L.sp]);
+      else next_top(L, top_stack, head.y == 0, head.x);
+    } else if (run == PH_LEAF) {
+      if (rs_leaf<AM>(w, L, L.cur)) L.phase = PH_DONE;
+      else if (L.sp) set_child(L, stack[--L.sp]);
+      else next_top(L, top_stack, head.y == 0, head.x);
+    } else if (run == PH_ENTER) {
+      if (!rs_enter<AM>(w, L, L.cur)) next_top(L, top_stack, head.y == 0, head.x);
+    } else {
       const float bound = L.best.rec[0] != 0 ? next_up(L.best.t) : L.best.t;
-      top_step(w, (head.y & ~3u) + (size_t)item * 32, L.ray, L.world_inv, bound, top_stack, L.tsp, st);
+      top_step(w, top + (size_t)L.cur * 32, L.ray, L.world_inv, bound, top_stack, L.top_at, st);
+      next_top(L, top_stack, false, 0);
     }
   }
+  if (L.phase == PH_DONE) rs_finish<AM>(L, src);
 }
 
 // ---------------------------------------------------------------- GI layout
+
+// The closest hit so far: the record's identity words and normal are made once, when the ray ends.
+struct GiNear {
+  float t, u, v;
+  uint32_t inst;  // EMPTY: none
+  uint32_t at;    // word of the triangle's three indices
+};
+RT_DEV float gi_limit(const GiNear& b, uint32_t i) { return (b.inst != EMPTY && i < b.inst) ? next_up(b.t) : b.t; }
 
 template <int AM>
 struct GiLane {
   Ray ray;
   F3 world_inv;
-  GiBest best;
+  GiNear best;
   uint32_t ray_id;
   uint32_t entry;
   bool any;
   uint32_t phase;
-  uint32_t tsp, flat_i;
+  uint32_t top_at;
   uint32_t inst;
-  float r[12];
   F3 o, d, inv;
-  uint32_t nodes, leaves, positions, indices, prim_base;
+  uint32_t nodes, leaves, positions, indices;
   uint32_t cur, sp;
 };
 
+// The record of an ended ray (gi_rays_software.wgsl:141-169): a hit's primitive or position
+// indices, and the world normal of its source winding.
 template <int AM, class Src>
-RT_DEV void gi_finish(GiLane<AM>& L, const Src& src) {
-  const GiBest& b = L.best;
+RT_DEV void gi_finish(const uint32_t* __restrict__ w, const GiLane<AM>& L, const Src& src) {
+  const GiNear& b = L.best;
   if (any_of<AM>(L)) {
-    put_flag(src, L.entry, L.ray_id, L.ray, b.hit);
-  } else {
-    uint32_t* o = reinterpret_cast<uint32_t*>(out_of(src, L.entry)) + 10 * (size_t)L.ray_id;
-    o[0] = __float_as_uint(b.t), o[1] = b.inst, o[2] = b.tri[0], o[3] = b.tri[1], o[4] = b.tri[2];
-    o[5] = __float_as_uint(b.u), o[6] = __float_as_uint(b.v);
-    o[7] = __float_as_uint(b.n.x), o[8] = __float_as_uint(b.n.y), o[9] = __float_as_uint(b.n.z);
+    put_flag(src, L.entry, L.ray_id, L.ray, b.inst != EMPTY);
+    return;
   }
-  L.phase = PH_IDLE;
+  uint32_t* o = reinterpret_cast<uint32_t*>(out_of(src, L.entry)) + 10 * (size_t)L.ray_id;
+  uint32_t tri[3] = {0, 0, 0};
+  F3 n = {0.0f, 0.0f, 0.0f};
+  if (b.inst != EMPTY) {
+    const size_t r = 16 + (size_t)b.inst * 32;
+    const uint32_t positions = ld(w, r + 20), indices = ld(w, r + 21), prim_base = ld(w, r + 28);
+    tri[0] = ld(w, b.at), tri[1] = ld(w, (size_t)b.at + 1), tri[2] = ld(w, (size_t)b.at + 2);
+    const F3 a = ld3(w, positions + (size_t)tri[0] * 3), bb = ld3(w, positions + (size_t)tri[1] * 3),
+             c = ld3(w, positions + (size_t)tri[2] * 3);
+    const F3 cr = cross3(sub3(bb, a), sub3(c, a));
+    const uint4 q0 = ld4(w, r), q1 = ld4(w, r + 4), q2 = ld4(w, r + 8);
+    n = unit_normal({add(add(mul(__uint_as_float(q0.x), cr.x), mul(__uint_as_float(q1.x), cr.y)), mul(__uint_as_float(q2.x), cr.z)),
+                     add(add(mul(__uint_as_float(q0.y), cr.x), mul(__uint_as_float(q1.y), cr.y)), mul(__uint_as_float(q2.y), cr.z)),
+                     add(add(mul(__uint_as_float(q0.z), cr.x), mul(__uint_as_float(q1.z), cr.y)), mul(__uint_as_float(q2.z), cr.z))});
+    if (prim_base != 0) tri[0] = ld(w, prim_base + (b.at - indices) / 3), tri[1] = 0, tri[2] = 0;
+  }
+  o[0] = __float_as_uint(b.t), o[1] = b.inst, o[2] = tri[0], o[3] = tri[1], o[4] = tri[2];
+  o[5] = __float_as_uint(b.u), o[6] = __float_as_uint(b.v);
+  o[7] = __float_as_uint(n.x), o[8] = __float_as_uint(n.y), o[9] = __float_as_uint(n.z);
 }
 
-// gi_instance's entry (gi_rays_software.wgsl:100-113)
+// gi_instance's entry (gi_rays_software.wgsl:100-113): true when the lane now walks the
+// instance's BLAS.
 template <int AM>
-RT_DEV void gi_enter(const uint32_t* __restrict__ w, GiLane<AM>& L, uint32_t i) {
-  const size_t r = 16 + (size_t)i * 32;
-  if (any_of<AM>(L) && (ld(w, r + 27) & 1u) != 0) return;
+RT_DEV bool gi_enter(const uint32_t* __restrict__ w, GiLane<AM>& L, uint32_t i) {
+  const size_t r = 16 + (size_t)i * 32;  // records start on 16 bytes
+  if (any_of<AM>(L) && (ld(w, r + 27) & 1u) != 0) return false;
+  const uint4 b0 = ld4(w, r + 12), b1 = ld4(w, r + 16);
   const float lim = gi_limit(L.best, i);
-  if (!(slab_near(L.ray.o, L.world_inv, ld3(w, r + 12), ld3(w, r + 15), L.ray.tmin, lim) <= lim)) return;
-  for (int k = 0; k < 12; ++k) L.r[k] = ldf(w, r + k);
-  const F3 ro = L.ray.o, rd = L.ray.d;
-  L.o = {dot4p(L.r[0], L.r[1], L.r[2], L.r[3], ro), dot4p(L.r[4], L.r[5], L.r[6], L.r[7], ro),
-         dot4p(L.r[8], L.r[9], L.r[10], L.r[11], ro)};
-  L.d = {dot3({L.r[0], L.r[1], L.r[2]}, rd), dot3({L.r[4], L.r[5], L.r[6]}, rd), dot3({L.r[8], L.r[9], L.r[10]}, rd)};
+  const F3 lo = {__uint_as_float(b0.x), __uint_as_float(b0.y), __uint_as_float(b0.z)};
+  const F3 hi = {__uint_as_float(b0.w), __uint_as_float(b1.x), __uint_as_float(b1.y)};
+  if (!(slab_near(L.ray.o, L.world_inv, lo, hi, L.ray.tmin, lim) <= lim)) return false;
+  const uint4 b2 = ld4(w, r + 20);
+  to_object(ld4(w, r), ld4(w, r + 4), ld4(w, r + 8), L.ray, L.o, L.d);
   L.inv = safe_inverse(L.d);
-  L.nodes = ld(w, r + 18), L.leaves = ld(w, r + 19), L.positions = ld(w, r + 20), L.indices = ld(w, r + 21);
-  L.prim_base = ld(w, r + 28);
+  L.nodes = b1.z, L.leaves = b1.w, L.positions = b2.x, L.indices = b2.y;
   L.inst = i;
-  L.cur = ld(w, r + 22);
   L.sp = 0;
-  L.phase = PH_BLAS;
+  set_child(L, b2.z);
+  return true;
 }
 
 // One GI leaf (gi_rays_software.wgsl:117-169). True when an any-hit ray is blocked.
@@ -334,17 +393,10 @@ RT_DEV bool gi_leaf(const uint32_t* __restrict__ w, GiLane<AM>& L, uint32_t chil
   const size_t l = L.leaves + (size_t)(child & ~LEAF) * 2;
   const uint32_t first = ld(w, l), count = ld(w, l + 1);
   const uint32_t i = L.inst;
-  auto normal_of = [&](F3 a, F3 b, F3 c) {
-    F3 cr = cross3(sub3(b, a), sub3(c, a));
-    F3 n = {add(add(mul(L.r[0], cr.x), mul(L.r[4], cr.y)), mul(L.r[8], cr.z)),
-            add(add(mul(L.r[1], cr.x), mul(L.r[5], cr.y)), mul(L.r[9], cr.z)),
-            add(add(mul(L.r[2], cr.x), mul(L.r[6], cr.y)), mul(L.r[10], cr.z))};
-    return unit_normal(n);
-  };
   for (uint32_t k = 0; k < count; k += 6) {
-    const size_t x = (size_t)L.indices + first + k;
+    const uint32_t x = L.indices + first + k;
     const bool two = k + 3 < count;
-    const size_t y = two ? x + 3 : x;
+    const uint32_t y = two ? x + 3 : x;
     const uint32_t ia = ld(w, x), ib = ld(w, x + 1), ic = ld(w, x + 2);
     const uint32_t ja = ld(w, y), jb = ld(w, y + 1), jc = ld(w, y + 2);
     const F3 a = ld3(w, L.positions + (size_t)ia * 3), b = ld3(w, L.positions + (size_t)ib * 3),
@@ -353,44 +405,34 @@ RT_DEV bool gi_leaf(const uint32_t* __restrict__ w, GiLane<AM>& L, uint32_t chil
              c2 = ld3(w, L.positions + (size_t)jc * 3);
     float t, u, v;
     if (gi_triangle(L.o, L.d, a, b, c, L.ray.tmin, gi_limit(L.best, i), t, u, v)) {
-      L.best.hit = true, L.best.t = t, L.best.inst = i, L.best.u = u, L.best.v = v;
+      L.best = GiNear{t, u, v, i, x};
       if (any_of<AM>(L)) return true;
-      L.best.n = normal_of(a, b, c);
-      if (L.prim_base != 0) L.best.tri[0] = ld(w, L.prim_base + (first + k) / 3), L.best.tri[1] = 0, L.best.tri[2] = 0;
-      else L.best.tri[0] = ia, L.best.tri[1] = ib, L.best.tri[2] = ic;
     }
     if (two && gi_triangle(L.o, L.d, a2, b2, c2, L.ray.tmin, gi_limit(L.best, i), t, u, v)) {
-      L.best.hit = true, L.best.t = t, L.best.inst = i, L.best.u = u, L.best.v = v;
+      L.best = GiNear{t, u, v, i, y};
       if (any_of<AM>(L)) return true;
-      L.best.n = normal_of(a2, b2, c2);
-      if (L.prim_base != 0) L.best.tri[0] = ld(w, L.prim_base + (first + k) / 3 + 1), L.best.tri[1] = 0, L.best.tri[2] = 0;
-      else L.best.tri[0] = ja, L.best.tri[1] = jb, L.best.tri[2] = jc;
     }
   }
   return false;
 }
 
-// One GI BLAS node (gi_rays_software.wgsl:171-204): every surviving child pushed far to near.
+// One GI BLAS node (gi_rays_software.wgsl:171-204): every surviving child pushed far to near; the
+// nearest of them is returned instead (it would be popped next), EMPTY when none survives.
 template <int AM>
-RT_DEV void gi_node(const uint32_t* __restrict__ w, GiLane<AM>& L, uint32_t child, uint32_t* stack, DevStatus* st) {
+RT_DEV uint32_t gi_node(const uint32_t* __restrict__ w, GiLane<AM>& L, uint32_t child, uint32_t* stack, DevStatus* st) {
   const size_t n = L.nodes + (size_t)child * 16;
-  const uint4 n0 = ld4u(w, n), n1 = ld4u(w, n + 4), n2 = ld4u(w, n + 8), n3 = ld4u(w, n + 12);
-  const F3 oq = {__uint_as_float(n0.x), __uint_as_float(n0.y), __uint_as_float(n0.z)};
-  const F3 step = {__uint_as_float(n0.w), __uint_as_float(n1.x), __uint_as_float(n1.y)};
+  uint4 nn[4];
+  ld16(w, n, nn);
+  const uint4 &n0 = nn[0], &n1 = nn[1], &n2 = nn[2], &n3 = nn[3];
   uint32_t c[4] = {n1.z, n1.w, n2.x, n2.y};
   const float lim = gi_limit(L.best, L.inst);
+  float dist[4];
+  child_slabs({__uint_as_float(n0.x), __uint_as_float(n0.y), __uint_as_float(n0.z)},
+              {__uint_as_float(n0.w), __uint_as_float(n1.x), __uint_as_float(n1.y)}, n2.z, n2.w, n3.x, n3.y, n3.z, n3.w, L.o,
+              L.inv, L.ray.tmin, lim, dist);
   uint32_t tb[4];
 #pragma unroll
-  for (int s = 0; s < 4; ++s) {
-    tb[s] = __float_as_uint(BIG);
-    if (c[s] == EMPTY) continue;
-    const uint32_t sh = 8 * s;
-    const F3 lo = {add(oq.x, mul(step.x, byte_f(n2.z, sh))), add(oq.y, mul(step.y, byte_f(n2.w, sh))),
-                   add(oq.z, mul(step.z, byte_f(n3.x, sh)))};
-    const F3 hi = {add(oq.x, mul(step.x, byte_f(n3.y, sh))), add(oq.y, mul(step.y, byte_f(n3.z, sh))),
-                   add(oq.z, mul(step.z, byte_f(n3.w, sh)))};
-    tb[s] = __float_as_uint(slab_near(L.o, L.inv, lo, hi, L.ray.tmin, lim));
-  }
+  for (int s = 0; s < 4; ++s) tb[s] = __float_as_uint(c[s] == EMPTY ? BIG : dist[s]);
 #define RT_SW(a, b)                          \
   if (tb[a] < tb[b]) {                       \
     uint32_t x = tb[a]; tb[a] = tb[b]; tb[b] = x; \
@@ -398,19 +440,21 @@ RT_DEV void gi_node(const uint32_t* __restrict__ w, GiLane<AM>& L, uint32_t chil
   }
   RT_SW(0, 1) RT_SW(2, 3) RT_SW(0, 2) RT_SW(1, 3) RT_SW(1, 2)
 #undef RT_SW
+  uint32_t next = EMPTY;
 #pragma unroll
   for (int s = 0; s < 4; ++s) {
     if (__uint_as_float(tb[s]) <= lim && c[s] != EMPTY) {
-      if (L.sp < STACK) stack[L.sp++] = c[s];
-      else atomicAdd(&st->stack_drops, 1ull);
+      if (next != EMPTY) stack[L.sp++] = next;
+      next = c[s];
+      if (L.sp >= STACK) next = EMPTY, atomicAdd(&st->stack_drops, 1ull);
     }
   }
-  L.cur = EMPTY;
+  return next;
 }
 
 template <int AM, int BLOCK, class Src>
-__global__ void __launch_bounds__(BLOCK) k_gi_fast(const uint32_t* __restrict__ w, const Src src, RayQueue queue,
-                                                   DevStatus* st) {
+__global__ void __launch_bounds__(BLOCK, FAST_MIN_BLOCKS)
+    k_gi_fast(const uint32_t* __restrict__ w, const Src src, RayQueue queue, DevStatus* st) {
   uint32_t stack[STACK];
   uint32_t top_stack[STACK];
   GiLane<AM> L;
@@ -419,62 +463,40 @@ __global__ void __launch_bounds__(BLOCK) k_gi_fast(const uint32_t* __restrict__ 
   bool drained = false;
   for (;;) {
     __syncwarp();
-    const uint32_t id = take_ray(queue, L.phase == PH_IDLE, drained);
-    if (L.phase == PH_IDLE && id != EMPTY) {
+    const uint32_t id = take_ray(queue, L.phase == PH_IDLE || L.phase == PH_DONE, drained);
+    if (id != EMPTY) {
+      if (L.phase == PH_DONE) gi_finish<AM>(w, L, src);
       L.ray = fetch(src, id, L);
       L.world_inv = safe_inverse(L.ray.d);
-      L.best.hit = false, L.best.t = L.ray.tmax, L.best.n = {0.0f, 0.0f, 0.0f}, L.best.inst = EMPTY;
-      L.best.tri[0] = L.best.tri[1] = L.best.tri[2] = 0, L.best.u = L.best.v = 0.0f;
-      L.phase = PH_TOP;
-      L.flat_i = 0;
-      L.tsp = 1;
+      L.best = GiNear{L.ray.tmax, 0.0f, 0.0f, EMPTY, 0u};
+      L.top_at = top == 0 ? 0 : 1;
       top_stack[0] = root;
+      next_top(L, top_stack, top == 0, instances);
     }
-    if (!__any_sync(0xffffffffu, L.phase != PH_IDLE)) {
+    const uint32_t run = vote_phase(L.phase);
+    if (run == PH_IDLE) {
       if (drained) break;
       continue;
     }
-    if (L.phase == PH_BLAS) {
-      if (L.cur == EMPTY) {
-        if (L.sp == 0) L.phase = PH_TOP;
-        else L.cur = stack[--L.sp];
-      }
-      if (L.phase == PH_BLAS) {
-        const uint32_t child = L.cur;
-        if (child & LEAF) {
-          if (gi_leaf<AM>(w, L, child)) {
-            gi_finish<AM>(L, src);
-            continue;
-          }
-          L.cur = EMPTY;
-        } else {
-          gi_node<AM>(w, L, child, stack, st);
-        }
-        continue;
-      }
-    }
-    if (L.phase == PH_TOP) {
-      if (top == 0) {
-        if (L.flat_i >= instances) {
-          gi_finish<AM>(L, src);
-          continue;
-        }
-        gi_enter<AM>(w, L, L.flat_i++);
-        continue;
-      }
-      if (L.tsp == 0) {
-        gi_finish<AM>(L, src);
-        continue;
-      }
-      const uint32_t item = top_stack[--L.tsp];
-      if (item & LEAF) {
-        gi_enter<AM>(w, L, item & ~LEAF);
-        continue;
-      }
-      const float bound = L.best.hit ? next_up(L.best.t) : L.best.t;
-      top_step(w, top + (size_t)item * 32, L.ray, L.world_inv, bound, top_stack, L.tsp, st);
+    if (L.phase != run) continue;
+    if (run == PH_NODE) {
+      const uint32_t c = gi_node<AM>(w, L, L.cur, stack, st);
+      if (c != EMPTY) set_child(L, c);
+      else if (L.sp) set_child(L, stack[--L.sp]);
+      else next_top(L, top_stack, top == 0, instances);
+    } else if (run == PH_LEAF) {
+      if (gi_leaf<AM>(w, L, L.cur)) L.phase = PH_DONE;
+      else if (L.sp) set_child(L, stack[--L.sp]);
+      else next_top(L, top_stack, top == 0, instances);
+    } else if (run == PH_ENTER) {
+      if (!gi_enter<AM>(w, L, L.cur)) next_top(L, top_stack, top == 0, instances);
+    } else {
+      const float bound = L.best.inst != EMPTY ? next_up(L.best.t) : L.best.t;
+      top_step(w, top + (size_t)L.cur * 32, L.ray, L.world_inv, bound, top_stack, L.top_at, st);
+      next_top(L, top_stack, false, 0);
     }
   }
+  if (L.phase == PH_DONE) gi_finish<AM>(w, L, src);
 }
 
 }  // namespace rtk

@@ -156,19 +156,24 @@ RT_DEV void top_step(const uint32_t* __restrict__ w, size_t n, const Ray& ray, F
   // the node's seven 16-byte rows: lo x, lo y, lo z, hi x, hi y, hi z (four children each), ids
   const uint4 lx = ld4u(w, n), ly = ld4u(w, n + 4), lz = ld4u(w, n + 8);
   const uint4 hx = ld4u(w, n + 12), hy = ld4u(w, n + 16), hz = ld4u(w, n + 20), id4 = ld4u(w, n + 24);
-  auto at = [](const uint4& q, int c) { return c == 0 ? q.x : (c == 1 ? q.y : (c == 2 ? q.z : q.w)); };
+  // two children to an instruction, each lane's difference and product rounded on its own
+  auto plane = [](uint32_t a, uint32_t b, float o, float inv) {
+    return mul2(add2(pack2(__uint_as_float(a), __uint_as_float(b)), both(-o)), both(inv));
+  };
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const float ax = mul(sub(__uint_as_float(at(lx, c)), ray.o.x), world_inv.x),
-                bx = mul(sub(__uint_as_float(at(hx, c)), ray.o.x), world_inv.x);
-    const float ay = mul(sub(__uint_as_float(at(ly, c)), ray.o.y), world_inv.y),
-                by = mul(sub(__uint_as_float(at(hy, c)), ray.o.y), world_inv.y);
-    const float az = mul(sub(__uint_as_float(at(lz, c)), ray.o.z), world_inv.z),
-                bz = mul(sub(__uint_as_float(at(hz, c)), ray.o.z), world_inv.z);
-    const float near = fmaxf(fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fminf(az, bz)), ray.tmin);
-    const float far = fminf(fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fmaxf(az, bz)), bound);
-    ids[c] = at(id4, c);
-    dist[c] = (near <= far && ids[c] != EMPTY) ? near : BIG;
+  for (int c = 0; c < 4; c += 2) {
+    auto pair = [&](const uint4& q, float o, float inv) { return c == 0 ? plane(q.x, q.y, o, inv) : plane(q.z, q.w, o, inv); };
+    const P2 ax = pair(lx, ray.o.x, world_inv.x), bx = pair(hx, ray.o.x, world_inv.x);
+    const P2 ay = pair(ly, ray.o.y, world_inv.y), by = pair(hy, ray.o.y, world_inv.y);
+    const P2 az = pair(lz, ray.o.z, world_inv.z), bz = pair(hz, ray.o.z, world_inv.z);
+    auto entry = [&](float x0, float x1, float y0, float y1, float z0, float z1, uint32_t id) {
+      const float near = fmaxf(fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fminf(z0, z1)), ray.tmin);
+      const float far = fminf(fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fmaxf(z0, z1)), bound);
+      return near <= far && id != EMPTY ? near : BIG;
+    };
+    ids[c] = c == 0 ? id4.x : id4.z, ids[c + 1] = c == 0 ? id4.y : id4.w;
+    dist[c] = entry(first(ax), first(bx), first(ay), first(by), first(az), first(bz), ids[c]);
+    dist[c + 1] = entry(second(ax), second(bx), second(ay), second(by), second(az), second(bz), ids[c + 1]);
   }
 #define RT_SW(a, b)                                      \
   if (dist[b] < dist[a]) {                               \

@@ -40,12 +40,20 @@ cudaError_t resident_blocks(K kernel, uint32_t& out) {
   return cudaSuccess;
 }
 
+// The launch's grid and the lanes of each warp that take rays. A launch that does not fill the GPU
+// is bound by its longest rays' chains of loads, and a warp's lanes delay one another where they
+// part; so its rays are spread over half of the resident warps, in as few lanes each as hold them.
+// 4,096 GI rays over a 250k-triangle scene: 159 us against 196 with all 32 lanes; 10,000 (GI
+// layout): 151 against 162; from about 65,000 rays on both are the same.
 template <class K>
-cudaError_t grid_for(K kernel, uint32_t n, dim3& grid) {
+cudaError_t grid_for(K kernel, uint32_t n, dim3& grid, uint32_t& width) {
   uint32_t full = 0;
   cudaError_t e = resident_blocks(kernel, full);
   if (e != cudaSuccess) return e;
-  const uint32_t need = (n + FAST_BLOCK - 1) / FAST_BLOCK;
+  constexpr uint32_t warps = FAST_BLOCK / 32;
+  width = 1;
+  while (width < 32 && (uint64_t)full * warps * width < 2 * (uint64_t)n) width *= 2;
+  const uint32_t need = (uint32_t)(((uint64_t)n + warps * width - 1) / (warps * width));
   grid = dim3(need < full ? need : full);
   return cudaSuccess;
 }
@@ -54,10 +62,11 @@ template <class K, class Src>
 cudaError_t run(K kernel, const SceneView& s, const Src& src, uint32_t n, unsigned int* counter, rtk::DevStatus* st,
                 cudaStream_t stream, uint32_t refill) {
   dim3 grid;
-  cudaError_t e = grid_for(kernel, n, grid);
+  uint32_t width = 32;
+  cudaError_t e = grid_for(kernel, n, grid, width);
   if (e != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), stream)) != cudaSuccess) return e;
-  kernel<<<grid, FAST_BLOCK, 0, stream>>>(s.words, src, rtk::RayQueue{counter, n, refill}, st);
+  kernel<<<grid, FAST_BLOCK, 0, stream>>>(s.words, src, rtk::RayQueue{counter, n, refill < width ? refill : width, width}, st);
   return cudaGetLastError();
 }
 }  // namespace
