@@ -367,6 +367,9 @@ struct W8Lane {
   uint32_t sp;
 };
 
+// The widening of a node's planes along one axis (derived in w8_box_hits).
+RT_DEV float w8_margin(float a, float b) { return 2.0f * W8_U * fmaf(4.2f, fabsf(a), 7.1f * fabsf(b)); }
+
 // The eight child-box tests of one node for one ray: bit s is set when slot s's box meets
 // [tmin, lim] (conservatively: no box the ray meets is missed).
 RT_DEV uint32_t w8_box_hits(const W8Ray& R, const uint4& a0, const uint4& a2, const uint4& a3, const uint4& a4, float tmin,
@@ -386,9 +389,7 @@ RT_DEV uint32_t w8_box_hits(const W8Ray& R, const uint4& a0, const uint4& a2, co
   // So each plane is within u (4.02 |A'| + 6.01 |B|) of exact; doubled (8.4 |A'| + 14.2 |B| with
   // margin for E's own rounding) it moves the near planes down and the far planes up. The max /
   // min of the planes adds no rounding, so the entry and exit need no further widening.
-  const float Ex = 2.0f * W8_U * fmaf(4.2f, fabsf(Ax), 7.1f * fabsf(Bx));
-  const float Ey = 2.0f * W8_U * fmaf(4.2f, fabsf(Ay), 7.1f * fabsf(By));
-  const float Ez = 2.0f * W8_U * fmaf(4.2f, fabsf(Az), 7.1f * fabsf(Bz));
+  const float Ex = w8_margin(Ax, Bx), Ey = w8_margin(Ay, By), Ez = w8_margin(Az, Bz);
   const float Cx = __fsub_rn(Bx, Ax), Cy = __fsub_rn(By, Ay), Cz = __fsub_rn(Bz, Az);
   const float Bnx = Cx - Ex, Bfx = Cx + Ex, Bny = Cy - Ey, Bfy = Cy + Ey, Bnz = Cz - Ez, Bfz = Cz + Ez;
   // near / far planes per axis by the direction's sign
@@ -861,6 +862,64 @@ struct WarpGroupStack {  // W8_STACK (32) node-group entries: (first child, pend
 };
 static_assert(W8_STACK == 32, "WarpGroupStack holds one entry a lane");
 
+// The packet walk's current node, decoded once for the warp (each lane decoding all 48 planes for
+// itself, on the pipe that also takes the minima and maxima, was what bound the walk: 3.30 ms for
+// 4.19M camera rays over 1M triangles against 2.89): the child planes as 1 + q 2^-15 (lower
+// x, y, z, then upper x, y, z, eight slots each), the node's eight header words and 2^(e+15) per axis.
+struct W8Decoded {
+  float planes[48];
+  uint4 head[2];
+  float4 scale;
+};
+
+// Reads and decodes one node, a word a lane. Called by all 32 lanes; they may read `D` on return,
+// and must have done so before the next call.
+RT_DEV void w8_decode(const W8View& V, uint32_t node, W8Decoded& D) {
+  const uint32_t lane = threadIdx.x & 31;
+  __syncwarp();
+  if (lane < 23) {  // lanes 20-22: one axis' exponent each
+    const uint32_t* np = reinterpret_cast<const uint32_t*>(V.nodes + 5 * (size_t)node);
+    const uint32_t x = __ldg(np + (lane < 20 ? lane : 3u));
+    if (lane >= 20) reinterpret_cast<uint32_t*>(&D.scale)[lane - 20] = (((x >> (8 * (lane - 20))) & 0xffu) + 15u) << 23;
+    else if (lane >= 8) reinterpret_cast<float4*>(D.planes)[lane - 8] = make_float4(q15(x, 0), q15(x, 1), q15(x, 2), q15(x, 3));
+    else reinterpret_cast<uint32_t*>(D.head)[lane] = x;
+  }
+  __syncwarp();
+}
+
+// w8_box_hits from the decoded node: the same planes, products and margins, two slots to an
+// instruction.
+RT_DEV uint32_t w8_box_hits(const W8Ray& R, const W8Decoded& D, const uint4& a0, float tmin, float lim) {
+  const float4 sc = D.scale;
+  const float Ax = __fmul_rn(sc.x, R.inv.x), Ay = __fmul_rn(sc.y, R.inv.y), Az = __fmul_rn(sc.z, R.inv.z);
+  const float Bx = __fmul_rn(__fsub_rn(__uint_as_float(a0.x), R.o.x), R.inv.x),
+              By = __fmul_rn(__fsub_rn(__uint_as_float(a0.y), R.o.y), R.inv.y),
+              Bz = __fmul_rn(__fsub_rn(__uint_as_float(a0.z), R.o.z), R.inv.z);
+  const float Ex = w8_margin(Ax, Bx), Ey = w8_margin(Ay, By), Ez = w8_margin(Az, Bz);
+  const float Cx = __fsub_rn(Bx, Ax), Cy = __fsub_rn(By, Ay), Cz = __fsub_rn(Bz, Az);
+  const float Bnx = Cx - Ex, Bfx = Cx + Ex, Bny = Cy - Ey, Bfy = Cy + Ey, Bnz = Cz - Ez, Bfz = Cz + Ez;
+  const uint32_t ox = R.oct & 1u ? 24u : 0u, oy = R.oct & 2u ? 24u : 0u, oz = R.oct & 4u ? 24u : 0u;
+  uint32_t miss = 0;
+#pragma unroll
+  for (int h = 1; h >= 0; --h) {
+    auto four = [&](uint32_t at) { return *reinterpret_cast<const ulonglong2*>(D.planes + at + 4 * h); };
+    const ulonglong2 nx = four(ox), fx = four(24u - ox), ny = four(8u + oy), fy = four(32u - oy), nz = four(16u + oz), fz = four(40u - oz);
+#pragma unroll
+    for (int k = 1; k >= 0; --k) {
+      auto plane = [&](const ulonglong2& q, float a, float b) { return fma2(P2{k ? q.y : q.x}, both(a), both(b)); };
+      const P2 tnx = plane(nx, Ax, Bnx), tfx = plane(fx, Ax, Bfx), tny = plane(ny, Ay, Bny), tfy = plane(fy, Ay, Bfy);
+      const P2 tnz = plane(nz, Az, Bnz), tfz = plane(fz, Az, Bfz);
+      const float n1 = fmaxf(fmaxf(second(tnx), second(tny)), fmaxf(second(tnz), tmin));
+      const float f1 = fminf(fminf(second(tfx), second(tfy)), fminf(second(tfz), lim));
+      const float n0 = fmaxf(fmaxf(first(tnx), first(tny)), fmaxf(first(tnz), tmin));
+      const float f0 = fminf(fminf(first(tfx), first(tfy)), fminf(first(tfz), lim));
+      miss = __funnelshift_l(__float_as_uint(__fsub_rn(f1, n1)), miss, 1);
+      miss = __funnelshift_l(__float_as_uint(__fsub_rn(f0, n0)), miss, 1);
+    }
+  }
+  return ~miss & 0xffu;
+}
+
 // One top-level node of the packet walk: each live lane computes its four slab entries against its
 // own bound (the per-ray walk's, from its best hit); a child is visited when any lane meets it,
 // nearest (over the lanes' entries) first, pushed onto the warp's top stack. Every lane returns
@@ -927,6 +986,8 @@ RT_DEV uint32_t w8_packet_top(const uint32_t* __restrict__ w, size_t n, const W8
 template <uint32_t LAYOUT, int AM, int BLOCK, class Src>
 __global__ void __launch_bounds__(BLOCK, RT_W8P_MIN_BLOCKS) k_wide8_packet(const uint32_t* __restrict__ w, W8View V, const Src src,
                                                            unsigned int* __restrict__ counter, uint32_t n, DevStatus* st) {
+  __shared__ W8Decoded decoded[BLOCK / 32];
+  W8Decoded& D = decoded[threadIdx.x / 32];
   WarpGroupStack stack;
   WarpStack<STACK> tstack;
   const int lane = threadIdx.x & 31;
@@ -985,14 +1046,14 @@ __global__ void __launch_bounds__(BLOCK, RT_W8P_MIN_BLOCKS) k_wide8_packet(const
           g_bits &= g_bits - 1;
           node = g_base + __popc(g_imask & ((1u << slot) - 1u));
         }
-        const uint4* np = V.nodes + 5 * (size_t)node;
-        const uint4 a0 = __ldg(np), a1 = __ldg(np + 1), a2 = __ldg(np + 2), a3 = __ldg(np + 3), a4 = __ldg(np + 4);
+        w8_decode(V, node, D);
+        const uint4 a0 = D.head[0], a1 = D.head[1];
         const uint32_t imask = a0.w >> 24, child_base = a1.x, tri_base = a1.y, meta_lo = a1.z, meta_hi = a1.w;
         uint32_t hits = 0;
         if (in) {
           const W8Best& best = L.best;
           const float lim = best.hit ? best.t + 2.0f * best.band + W8_TIE * best.t : L.ray.tmax;
-          hits = w8_box_hits(L.R, a0, a2, a3, a4, L.ray.tmin, lim);
+          hits = w8_box_hits(L.R, D, a0, L.ray.tmin, lim);
         }
         // leaves: every lane whose ray meets one tests its triangles
         for (uint32_t lh = __reduce_or_sync(0xffffffffu, hits & ~imask); lh; lh &= lh - 1) {
