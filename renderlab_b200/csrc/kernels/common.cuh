@@ -148,6 +148,23 @@ RT_DEV void to_object(uint4 q0, uint4 q1, uint4 q2, const Ray& ray, F3& o, F3& d
   d = {dot3(r0, ray.d), dot3(r1, ray.d), dot3(r2, ray.d)};
 }
 
+// What a lane does next. PH_DONE: its ray has ended and its result is not stored yet.
+enum : uint32_t { PH_IDLE = 0, PH_TOP = 1, PH_ENTER = 2, PH_NODE = 3, PH_LEAF = 4, PH_DONE = 5 };
+
+// The step that the warp runs next: the one that most of its lanes wait for (PH_IDLE: none does).
+// Called by all 32 lanes; the same answer in each.
+RT_DEV uint32_t vote_phase(uint32_t phase) {
+  const bool waits = phase - PH_TOP <= PH_LEAF - PH_TOP;
+  const uint32_t votes = __reduce_add_sync(0xffffffffu, waits ? 1u << (8 * (phase - PH_TOP)) : 0u);
+  uint32_t best = PH_IDLE, most = 0;
+#pragma unroll
+  for (uint32_t p = PH_TOP; p <= PH_LEAF; ++p) {
+    const uint32_t c = (votes >> (8 * (p - PH_TOP))) & 0xffu;
+    if (c > most) most = c, best = p;
+  }
+  return best;
+}
+
 // One ray batch of a many-batch launch, as the device reads it (32 bytes).
 struct BatchEntry {
   const float4* rays;

@@ -52,23 +52,6 @@ RT_DEV uint32_t take_ray(const RayQueue& q, bool need, bool& drained) {
 
 // ---------------------------------------------------------------- the walk's schedule
 
-// What a lane does next. PH_DONE: its ray has ended and its result is not stored yet.
-enum : uint32_t { PH_IDLE = 0, PH_TOP = 1, PH_ENTER = 2, PH_NODE = 3, PH_LEAF = 4, PH_DONE = 5 };
-
-// The step that the warp runs next: the one that most of its lanes wait for (PH_IDLE: none does).
-// Called by all 32 lanes; the same answer in each.
-RT_DEV uint32_t vote_phase(uint32_t phase) {
-  const bool waits = phase - PH_TOP <= PH_LEAF - PH_TOP;
-  const uint32_t votes = __reduce_add_sync(0xffffffffu, waits ? 1u << (8 * (phase - PH_TOP)) : 0u);
-  uint32_t best = PH_IDLE, most = 0;
-#pragma unroll
-  for (uint32_t p = PH_TOP; p <= PH_LEAF; ++p) {
-    const uint32_t c = (votes >> (8 * (p - PH_TOP))) & 0xffu;
-    if (c > most) most = c, best = p;
-  }
-  return best;
-}
-
 // Byte c of `word` as a float, exactly: as_float(0x4B000000 | q) - 2^23.
 RT_DEV float byte_f(uint32_t word, uint32_t c) {
   return __fsub_rn(__uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540u | c)), 8388608.0f);

@@ -34,18 +34,15 @@ constexpr uint32_t W8_STACK = 32;
 // Entries of the shared-memory group stack (a scene whose 8-wide trees are at most this many
 // levels deep stacks at most W8_SSTACK - 1 groups).
 constexpr uint32_t W8_SSTACK = 16;
-// Resident 128-thread blocks per SM the register allocation is sized for: the per-ray walk
-// (RT_W8_MIN_BLOCKS: 7, 72 registers) and the packet walk (RT_W8P_MIN_BLOCKS: 7, 72 registers).
-// The f64 resolution of uncertain candidates is out of line, so the per-ray loop fits its budget
-// with a few bytes of spills (the packet walk with about 150). Measured on clusters-1M and
-// clusters-4M rays against 4 to 8 blocks, with neither walk holding shared memory: 7 is the
-// fastest for both.
-#ifndef RT_W8_MIN_BLOCKS
-#define RT_W8_MIN_BLOCKS 7
-#endif
-#ifndef RT_W8P_MIN_BLOCKS
-#define RT_W8P_MIN_BLOCKS 7
-#endif
+// Resident 128-thread blocks per SM the register allocation is sized for.
+// Flat scenes (W8_FLAT_BLOCKS, 96 registers): the lane's ray and best hit stay in registers, which
+// takes more than 72; 4.19M GI rays over 1M triangles: 4.92, 4.66 and 5.13 ms at 4, 5 and 6 blocks
+// (with both in local memory 5.45 ms at 7, the fastest then). Scenes with a top level
+// (W8_TOP_BLOCKS, 72 registers, both in local memory): 7.48 ms a plan over 1,000 instances, and 12.6
+// against 11.9 ms with both in registers before the walk voted. The packet walk (W8P_MIN_BLOCKS, 72
+// registers, both in local memory, about 140 bytes of spills): 3.01, 2.93, 2.88 and 3.12 ms for
+// 4.19M camera rays at 5, 6, 7 and 8 blocks, and 3.2 ms at 5 to 7 with both in registers.
+constexpr int W8_FLAT_BLOCKS = 5, W8_TOP_BLOCKS = 7, W8P_MIN_BLOCKS = 7;
 
 // Opt-in device counters of the WIDE8 walk (diagnostics and the bytes-per-ray roofline).
 enum W8Count { W8C_RAYS, W8C_TOP_NODES, W8C_INSTANCE_TESTS, W8C_NODES, W8C_LEAVES, W8C_TRIS, W8C_RETESTS, W8C_FINAL64, W8C_N };
@@ -158,13 +155,15 @@ __device__ __noinline__ bool mt64(const uint32_t* __restrict__ w, uint32_t inst,
 // set when the instance is entered; the triangle test's part (the shear, oerr, tscale) when the
 // instance's first leaf triangle is tested (w8_shear): in scenes of many overlapping instances
 // most entered instances end at their root node's boxes, and never need it.
-struct W8Ray {
-  F3 o, d, inv;
-  uint32_t oct;
+struct W8Shear {
   // watertight shear rows: (Ax, Ay, Az) = M (v - o)
   F3 mx, my, mz;
   float oerr;   // |o - o64|_inf: the f32 object-space origin against the f64 reference's
   float tscale; // 8 u |1 / d_kz|: absolute error of t per unit of |v - o|
+};
+struct W8Ray : W8Shear {
+  F3 o, d, inv;
+  uint32_t oct;
   bool valid;
   bool sheared; // the triangle test's part is set
 };
@@ -180,11 +179,12 @@ RT_DEV void w8_setup(W8Ray& R) {
 // The triangle test's part for instance `inst` of the packed words (record rows at `r`): the
 // shear of Woop, Benthin and Wald (2013) for the object-space direction, and the error of the
 // f32 object-space origin against the f64 reference's (ray64's arithmetic over the same rows).
-__device__ __forceinline__ void w8_shear(const uint32_t* __restrict__ w, size_t r, const F3& world_o, W8Ray& R) {
-  const float ax = fabsf(R.d.x), ay = fabsf(R.d.y), az = fabsf(R.d.z);
+RT_DEV W8Shear w8_shear(const uint32_t* __restrict__ w, size_t r, F3 world_o, F3 o, F3 d) {
+  W8Shear R;
+  const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
   const int kz = (ax >= ay && ax >= az) ? 0 : (ay >= az ? 1 : 2);
   int kx = kz == 2 ? 0 : kz + 1, ky = kx == 2 ? 0 : kx + 1;
-  auto comp = [&](int k) { return k == 0 ? R.d.x : (k == 1 ? R.d.y : R.d.z); };
+  auto comp = [&](int k) { return k == 0 ? d.x : (k == 1 ? d.y : d.z); };
   const float dz = comp(kz);
   if (dz < 0.0f) {
     const int t = kx;
@@ -209,15 +209,16 @@ __device__ __forceinline__ void w8_shear(const uint32_t* __restrict__ w, size_t 
                                __dmul_rn((double)ldf(w, k + 2), oz)),
                      (double)ldf(w, k + 3));
   };
-  const double e = fmax(fmax(fabs(o64(r) - (double)R.o.x), fabs(o64(r + 4) - (double)R.o.y)),
-                        fabs(o64(r + 8) - (double)R.o.z));
+  const double e = fmax(fmax(fabs(o64(r) - (double)o.x), fabs(o64(r + 4) - (double)o.y)),
+                        fabs(o64(r + 8) - (double)o.z));
   R.oerr = e > 0.0 ? __double2float_ru(e) : 0.0f;
-  R.sheared = true;
+  return R;
 }
-// The same, out of line: a lazy setup at an instance's first triangle (see W8Ray), which most
-// entries of an instance-heavy scene never reach, so its code stays out of the walk's registers.
-__device__ __noinline__ void w8_shear_late(const uint32_t* __restrict__ w, size_t r, const F3& world_o, W8Ray& R) {
-  w8_shear(w, r, world_o, R);
+// The same, out of line (by value, so that the walk's state needs no address): a lazy setup at an
+// instance's first triangle (see W8Ray), which most entries of an instance-heavy scene never reach,
+// so its code stays out of the walk's registers.
+__device__ __noinline__ W8Shear w8_shear_late(const uint32_t* __restrict__ w, size_t r, F3 world_o, F3 o, F3 d) {
+  return w8_shear(w, r, world_o, o, d);
 }
 
 // Projected vertex (Ax, Ay, Az): one fixed chain of operations per vertex. `m` keeps the
@@ -302,12 +303,15 @@ __device__ __noinline__ bool w8_resolve64(const uint32_t* __restrict__ w, const 
   return true;
 }
 
-// Considers one candidate triangle; returns true when an any-hit query is satisfied.
-template <uint32_t LAYOUT, int AM, bool COUNT, bool LAZY = false>
+// Considers one candidate triangle; returns true when an any-hit query is satisfied. COPY: the ray
+// and the best hit go to the f64 resolution as copies, so that the walk can hold its own in
+// registers (else they live in local memory and every use of them is a load).
+template <uint32_t LAYOUT, int AM, bool COUNT, bool LAZY = false, bool COPY = false>
 RT_DEV bool w8_candidate(const uint32_t* __restrict__ w, const W8View& V, W8Ray& R, const Ray& ray, uint32_t inst,
                          uint32_t tri, W8Best& best, unsigned long long* cnt, bool lane_any) {
   w8_count<COUNT>(cnt, W8C_TRIS);
-  if (LAZY && !R.sheared) w8_shear_late(w, (LAYOUT == 0 ? 16 : 8) + (size_t)(LAYOUT == 0 ? 32 : 24) * inst, ray.o, R);
+  if (LAZY && !R.sheared)
+    static_cast<W8Shear&>(R) = w8_shear_late(w, (LAYOUT == 0 ? 16 : 8) + (size_t)(LAYOUT == 0 ? 32 : 24) * inst, ray.o, R.o, R.d), R.sheared = true;
   const uint4 q0 = __ldg(V.tris + 3 * (size_t)tri), q1 = __ldg(V.tris + 3 * (size_t)tri + 1),
               q2 = __ldg(V.tris + 3 * (size_t)tri + 2);
   const F3 v0 = {__uint_as_float(q0.x), __uint_as_float(q0.y), __uint_as_float(q0.z)};
@@ -331,7 +335,15 @@ RT_DEV bool w8_candidate(const uint32_t* __restrict__ w, const W8View& V, W8Ray&
                          (best.hit && t >= best.t - band - best.band);
   if (uncertain) {
     w8_count<COUNT>(cnt, W8C_RETESTS);
-    if (!w8_resolve64<LAYOUT>(w, V, ray, inst, tri, ident, ref, best)) return false;
+    if (COPY) {  // what the call takes by reference has to have an address: a copy's, not the walk's own
+      const Ray r = ray;
+      W8Best b = best;
+      const bool better = w8_resolve64<LAYOUT>(w, V, r, inst, tri, ident, ref, b);
+      best = b;
+      if (!better) return false;
+    } else if (!w8_resolve64<LAYOUT>(w, V, ray, inst, tri, ident, ref, best)) {
+      return false;
+    }
   } else {
     best.hit = true, best.has64 = false, best.t = t, best.band = band;
     best.inst = inst, best.tri = tri, best.ident = ident;
@@ -364,11 +376,19 @@ struct W8Lane {
   W8Ray R;
   uint32_t node;                     // next node to process, EMPTY: take one from the group
   uint32_t g_base, g_bits, g_imask;  // current node group
+  uint32_t leaves, tri_base, meta_lo, meta_hi;  // leaf slots still to test, and where their triangles are
+  uint32_t at;  // BLAS node to enter at
   uint32_t sp;
 };
 
 // The widening of a node's planes along one axis (derived in w8_box_hits).
 RT_DEV float w8_margin(float a, float b) { return 2.0f * W8_U * fmaf(4.2f, fabsf(a), 7.1f * fabsf(b)); }
+
+// How far along the lane's ray a node can hold a better hit.
+RT_DEV float w8_limit(const W8Lane& L) {
+  const W8Best& b = L.best;
+  return b.hit ? b.t + 2.0f * b.band + W8_TIE * b.t : L.ray.tmax;
+}
 
 // The eight child-box tests of one node for one ray: bit s is set when slot s's box meets
 // [tmin, lim] (conservatively: no box the ray meets is missed).
@@ -399,21 +419,20 @@ RT_DEV uint32_t w8_box_hits(const W8Ray& R, const uint4& a0, const uint4& a2, co
   const uint32_t fy0 = R.oct & 2u ? a2.z : a4.x, fy1 = R.oct & 2u ? a2.w : a4.y;
   const uint32_t nz0 = R.oct & 4u ? a4.z : a3.x, nz1 = R.oct & 4u ? a4.w : a3.y;
   const uint32_t fz0 = R.oct & 4u ? a3.x : a4.z, fz1 = R.oct & 4u ? a3.y : a4.w;
-  uint32_t hits = 0;
+  uint32_t miss = 0;  // the sign of far - near, slot 7 first
 #pragma unroll
-  for (int s = 0; s < 8; ++s) {
+  for (int s = 7; s >= 0; --s) {
     const uint32_t b = s & 3;
-    const float tnx = fmaf(q15(s < 4 ? nx0 : nx1, b), Ax, Bnx), tfx = fmaf(q15(s < 4 ? fx0 : fx1, b), Ax, Bfx);
-    const float tny = fmaf(q15(s < 4 ? ny0 : ny1, b), Ay, Bny), tfy = fmaf(q15(s < 4 ? fy0 : fy1, b), Ay, Bfy);
-    const float tnz = fmaf(q15(s < 4 ? nz0 : nz1, b), Az, Bnz), tfz = fmaf(q15(s < 4 ? fz0 : fz1, b), Az, Bfz);
+    const P2 tx = fma2(pack2(q15(s < 4 ? nx0 : nx1, b), q15(s < 4 ? fx0 : fx1, b)), both(Ax), pack2(Bnx, Bfx));
+    const P2 ty = fma2(pack2(q15(s < 4 ? ny0 : ny1, b), q15(s < 4 ? fy0 : fy1, b)), both(Ay), pack2(Bny, Bfy));
+    const P2 tz = fma2(pack2(q15(s < 4 ? nz0 : nz1, b), q15(s < 4 ? fz0 : fz1, b)), both(Az), pack2(Bnz, Bfz));
+    const float tnx = first(tx), tny = first(ty), tnz = first(tz), tfx = second(tx), tfy = second(ty), tfz = second(tz);
     const float tn = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, tmin)), tf = fminf(fminf(tfx, tfy), fminf(tfz, lim));
-    if (tn <= tf) hits |= 1u << s;
+    miss = __funnelshift_l(__float_as_uint(__fsub_rn(tf, tn)), miss, 1);
   }
-  return hits;
+  return ~miss & 0xffu;
 }
 
-// One 8-wide node: its leaf triangles are tested now, its inner hits become the group.
-// Returns true when an any-hit query is satisfied.
 // A lane's node-group stack: W8_STACK entries in local memory (cached by L1), or SS entries in a
 // shared-memory column of the block (entry i of thread t at i * BLOCK + t: the lanes of a warp
 // touch 32 consecutive words, so no bank conflict).
@@ -432,39 +451,39 @@ struct W8GroupStack<0, BLOCK> {
   RT_DEV uint2 pop(uint32_t& sp) { return e[--sp]; }
 };
 
-template <uint32_t LAYOUT, int AM, bool COUNT, bool LAZY, class Stack>
-RT_DEV bool w8_node(const uint32_t* __restrict__ w, const W8View& V, W8Lane& L, Stack& stack, DevStatus* st,
-                    unsigned long long* cnt) {
+// One 8-wide node: the leaf children met become the lane's pending leaves, the inner ones its group.
+template <bool COUNT, class Stack>
+RT_DEV void w8_node(const W8View& V, W8Lane& L, Stack& stack, DevStatus* st, unsigned long long* cnt) {
   w8_count<COUNT>(cnt, W8C_NODES);
   W8Ray& R = L.R;
   const uint4* np = V.nodes + 5 * (size_t)L.node;
   const uint4 a0 = __ldg(np), a1 = __ldg(np + 1), a2 = __ldg(np + 2), a3 = __ldg(np + 3), a4 = __ldg(np + 4);
   const uint32_t imask = a0.w >> 24;
-  const uint32_t child_base = a1.x, tri_base = a1.y, meta_lo = a1.z, meta_hi = a1.w;
-  const W8Best& best = L.best;
-  const float lim = best.hit ? best.t + 2.0f * best.band + W8_TIE * best.t : L.ray.tmax;
-  const uint32_t hits = w8_box_hits(R, a0, a2, a3, a4, L.ray.tmin, lim);
+  const uint32_t hits = w8_box_hits(R, a0, a2, a3, a4, L.ray.tmin, w8_limit(L));
   // Empty slots hold inverted boxes, which no ray meets; one that is met all the same (a node
   // tiny beside its distance, where the widening exceeds 255 steps) has a zero count.
-  uint32_t leaf_hits = hits & ~imask;
-  while (leaf_hits) {
-    const uint32_t s = __ffs(leaf_hits) - 1;
-    leaf_hits &= leaf_hits - 1;
-    const uint32_t m = ((s < 4 ? meta_lo : meta_hi) >> (8 * (s & 3))) & 0xffu;
-    const uint32_t first = tri_base + (m & 31u), count = m >> 5;
-    w8_count<COUNT>(cnt, W8C_LEAVES);
-    for (uint32_t k = 0; k < count; ++k)
-      if (w8_candidate<LAYOUT, AM, COUNT, LAZY>(w, V, R, L.ray, L.inst, first + k, L.best, cnt, L.any)) return true;
-  }
+  L.leaves = hits & ~imask;
+  L.tri_base = a1.y, L.meta_lo = a1.z, L.meta_hi = a1.w;
   const uint32_t inner = oct_permute(hits & imask, R.oct);
   if (inner) {
     if (L.g_bits) {
       if (L.sp < Stack::cap) stack.push(L.sp, make_uint2(L.g_base, L.g_bits | L.g_imask << 8));
       else atomicAdd(&st->stack_drops, 1ull);
     }
-    L.g_base = child_base, L.g_bits = inner, L.g_imask = imask;
+    L.g_base = a1.x, L.g_bits = inner, L.g_imask = imask;
   }
-  L.node = EMPTY;
+}
+
+// The first of a lane's pending leaves. Returns true when an any-hit query is satisfied.
+template <uint32_t LAYOUT, int AM, bool COUNT, bool LAZY>
+RT_DEV bool w8_leaf(const uint32_t* __restrict__ w, const W8View& V, W8Lane& L, unsigned long long* cnt) {
+  const uint32_t s = __ffs(L.leaves) - 1;
+  L.leaves &= L.leaves - 1;
+  const uint32_t m = ((s < 4 ? L.meta_lo : L.meta_hi) >> (8 * (s & 3))) & 0xffu;
+  const uint32_t first = L.tri_base + (m & 31u), count = m >> 5;
+  w8_count<COUNT>(cnt, W8C_LEAVES);
+  for (uint32_t k = 0; k < count; ++k)
+    if (w8_candidate<LAYOUT, AM, COUNT, LAZY, !LAZY>(w, V, L.R, L.ray, L.inst, first + k, L.best, cnt, L.any)) return true;
   return false;
 }
 
@@ -484,7 +503,7 @@ RT_DEV bool w8_next(W8Lane& L, Stack& stack) {
 }
 
 // Enters instance i when its world box survives; sets up the object-space ray.
-template <uint32_t LAYOUT, int AM, bool COUNT, bool LAZY = false>
+template <uint32_t LAYOUT, int AM, bool COUNT, bool LAZY = false, bool KEEP_INV = true>
 // `from_top`: the instance comes from a leaf of the 8-wide top level, whose box the walk has just
 // tested: a box around the world positions of the subtree of BLAS node `at` (relative to the root),
 // where this entry starts the walk. The instance's world box would not cull anything more that
@@ -499,7 +518,8 @@ RT_DEV void w8_enter(const uint32_t* __restrict__ w, const W8View& V, W8Lane& L,
   if (!from_top) {
     const W8Best& best = L.best;
     const float bound = best.hit ? best.t + 2.0f * best.band + 2.0f * W8_TIE * best.t : L.ray.tmax;
-    if (!(slab_near(L.ray.o, L.world_inv, ld3(w, r + 12), ld3(w, r + 15), L.ray.tmin, bound) <= bound)) return;
+    const F3 inv = KEEP_INV ? L.world_inv : safe_inverse(L.ray.d);
+    if (!(slab_near(L.ray.o, inv, ld3(w, r + 12), ld3(w, r + 15), L.ray.tmin, bound) <= bound)) return;
   }
   const uint32_t root = __ldg(V.inst + 2 * (size_t)i);
   if (root == EMPTY) return;
@@ -511,12 +531,12 @@ RT_DEV void w8_enter(const uint32_t* __restrict__ w, const W8View& V, W8Lane& L,
   L.R.d = {dot3({r00, r01, r02}, L.ray.d), dot3({r10, r11, r12}, L.ray.d), dot3({r20, r21, r22}, L.ray.d)};
   w8_setup(L.R);
   if (!L.R.valid) return;
-  if (!LAZY) w8_shear(w, r, L.ray.o, L.R);
+  if (!LAZY) static_cast<W8Shear&>(L.R) = w8_shear(w, r, L.ray.o, L.R.o, L.R.d), L.R.sheared = true;
   L.inst = i;
   L.node = root + at;
   L.g_bits = 0;
   L.sp = 0;
-  L.phase = 2;
+  L.phase = PH_NODE;
 }
 
 // Ends a lane's ray. Any hit: the flag. Closest hit: the winner as the walk knows it -- the f32 t
@@ -529,7 +549,6 @@ RT_DEV void w8_finish(const uint32_t* __restrict__ w, const W8View& V, W8Lane& L
   w8_count<COUNT>(cnt, W8C_RAYS);
   W8Best& b = L.best;
   const uint32_t id = L.ray_id;
-  L.phase = 0;
   if (any_of<AM>(L)) {
     put_flag(src, L.entry, id, L.ray, b.hit);
     return;
@@ -714,11 +733,19 @@ RT_DEV void w8_top_node(const W8View& V, const uint4* cache, uint32_t cached, ui
   }
 }
 
-// Persistent warps, one ray per lane, refilled as rays end; every iteration a lane takes one
-// step (a top-level node, an instance entry, or one 8-wide node with its leaves) and the warp
-// re-converges at the top of the loop.
+// Persistent warps, one ray per lane, refilled as rays end; a ray's result is stored when its lane
+// is refilled or the warp leaves. LAZY: the launches over scenes with a top level; the others walk
+// the instances as a flat list (whatever the words hold: a plan outlives a change of its records).
+//
+// Over a top level the lanes of a warp wait for different kinds of step (top-level node, instance
+// entry, BLAS node, leaf), and instruction issue bounds the walk; the warp runs the one that most of
+// them wait for (vote_phase), one leaf a step. 1.2M rays in 32 batches over 1,000 overlapping
+// instances: 7.47 ms, 11.9 with every kind run each time around. In a flat scene nearly all lanes
+// wait for a node, and loads bound the walk, so all run: nodes, each with its leaves at once, and
+// entries. 4.19M GI rays over 1M triangles: 4.66 ms, 4.90 with a vote and 5.11 with leaves as steps of
+// their own (which also drops the top level's stack: 5.45 ms before all of this).
 template <uint32_t LAYOUT, int AM, int BLOCK, bool COUNT, class Src, int SS = 0, bool LAZY = false>
-__global__ void __launch_bounds__(BLOCK, RT_W8_MIN_BLOCKS) k_wide8(const uint32_t* __restrict__ w, W8View V, const Src src,
+__global__ void __launch_bounds__(BLOCK, LAZY ? W8_TOP_BLOCKS : W8_FLAT_BLOCKS) k_wide8(const uint32_t* __restrict__ w, W8View V, const Src src,
                                                  unsigned int* __restrict__ counter, uint32_t n, DevStatus* st,
                                                  unsigned long long* cnt, uint32_t refill) {
   W8GroupStack<SS, BLOCK> stack;
@@ -729,8 +756,8 @@ __global__ void __launch_bounds__(BLOCK, RT_W8_MIN_BLOCKS) k_wide8(const uint32_
   // the packed BVH4 top level's stack (STACK items), or the 8-wide top level's (word pairs)
   uint32_t tstack[STACK > 2 * W8_TOP_STACK ? STACK : 2 * W8_TOP_STACK];
   W8Lane L;
-  L.phase = 0;
-  const uint32_t count = ld(w, 0), top = ld(w, 1), root = ld(w, 2);
+  L.phase = PH_IDLE;
+  const uint32_t count = ld(w, 0), top = LAZY ? ld(w, 1) : 0u, root = LAZY ? ld(w, 2) : 0u;
   const size_t top_base = LAYOUT == 0 ? top : (top & ~3u);
   // the 8-wide top level's first nodes, staged once per block (LAZY: the launches over scenes
   // with a top level; a flat scene's launch keeps no shared memory, which leaves L1 more room)
@@ -744,12 +771,43 @@ __global__ void __launch_bounds__(BLOCK, RT_W8_MIN_BLOCKS) k_wide8(const uint32_
     __syncthreads();
     top_cache = staged;
   }
+  // what the lane takes next from the top level (or the flat instance list)
+  auto next_top = [&]() {
+    L.phase = PH_DONE;
+    if (top == 0) {
+      if (L.flat >= count) return;
+      L.node = L.flat++, L.at = 0, L.phase = PH_ENTER;
+      return;
+    }
+    if (L.tsp == 0) return;
+    if (top8) {
+      L.tsp -= 2;
+      const uint32_t ex = tstack[L.tsp], ey = tstack[L.tsp + 1];
+      if (ey & W8_ENTRY) {  // a leaf's entry: an instance, at a node of its BLAS
+        L.node = ex, L.at = ey & ~W8_ENTRY, L.phase = PH_ENTER;
+        return;
+      }
+      uint32_t bits = ey & 0xffu;  // a group: its first pending child now, the rest back on the stack
+      const uint32_t imask = ey >> 8, k = __ffs(bits) - 1;
+      bits &= bits - 1;
+      if (bits) tstack[L.tsp] = ex, tstack[L.tsp + 1] = bits | imask << 8, L.tsp += 2;
+      const uint32_t slot = k ^ octant_of(L.ray.d);
+      L.node = ex + __popc(imask & ((1u << slot) - 1u)), L.phase = PH_TOP;
+      return;
+    }
+    const uint32_t item = tstack[--L.tsp];
+    L.node = item & ~LEAF, L.at = 0, L.phase = (item & LEAF) ? PH_ENTER : PH_TOP;
+  };
+  auto next_node = [&]() {
+    if (w8_next(L, stack)) L.phase = PH_NODE;
+    else next_top();
+  };
   bool drained = false;
   for (;;) {
     __syncwarp();
     // ray refill (warp-aggregated) once `refill` lanes are idle: 1 keeps every lane busy,
     // 32 hands out whole runs of 32 consecutive rays (keeps a coherent batch's tiles together)
-    const unsigned idle = __ballot_sync(0xffffffffu, L.phase == 0);
+    const unsigned idle = __ballot_sync(0xffffffffu, L.phase == PH_IDLE || L.phase == PH_DONE);
     const unsigned want = (!drained && (uint32_t)__popc(idle) >= refill) ? idle : 0u;
     uint32_t id = EMPTY;
     if (want) {
@@ -762,12 +820,12 @@ __global__ void __launch_bounds__(BLOCK, RT_W8_MIN_BLOCKS) k_wide8(const uint32_
       if ((want >> lane & 1u) && idx < n) id = idx;
     }
     if (id != EMPTY) {
+      if (L.phase == PH_DONE) w8_finish<LAYOUT, AM, COUNT>(w, V, L, src, cnt);
       L.ray = fetch<true>(src, id, L);
-      L.world_inv = safe_inverse(L.ray.d);
+      if (LAZY) L.world_inv = safe_inverse(L.ray.d);
       W8Best& b = L.best;
       b.hit = false, b.has64 = false, b.t = L.ray.tmax, b.band = 0.0f, b.t64 = 0.0;
       b.inst = EMPTY, b.tri = 0, b.ident = 0;
-      L.phase = 1;
       L.flat = 0;
       L.tsp = 0;
       if (top8) {  // the root as a group of one: slot 0 of an all-inner group at node 0
@@ -775,58 +833,49 @@ __global__ void __launch_bounds__(BLOCK, RT_W8_MIN_BLOCKS) k_wide8(const uint32_
       } else if (top != 0 && count != 0) {
         tstack[L.tsp++] = root;
       }
+      next_top();
     }
-    if (!__any_sync(0xffffffffu, L.phase != 0)) {
+    const uint32_t run = LAZY ? vote_phase(L.phase) : L.phase;
+    const bool none = LAZY ? run == PH_IDLE : !__any_sync(0xffffffffu, L.phase == PH_NODE || L.phase == PH_ENTER);
+    if (none) {
       if (drained) break;
       continue;
     }
-    if (L.phase == 2) {
-      if (L.node == EMPTY && !w8_next(L, stack)) {
-        L.phase = 1;
-      } else {
-        if (w8_node<LAYOUT, AM, COUNT, LAZY>(w, V, L, stack, st, cnt)) w8_finish<LAYOUT, AM, COUNT>(w, V, L, src, cnt);
+    if (L.phase != run) continue;
+    if (run == PH_NODE) {
+      w8_node<COUNT>(V, L, stack, st, cnt);
+      if (LAZY && L.leaves) {
+        L.phase = PH_LEAF;
         continue;
       }
-    }
-    if (L.phase == 1) {
-      if (top == 0) {
-        if (L.flat >= count) {
-          w8_finish<LAYOUT, AM, COUNT>(w, V, L, src, cnt);
-          continue;
-        }
-        w8_enter<LAYOUT, AM, COUNT, LAZY>(w, V, L, L.flat++, cnt, false);
-        continue;
+      bool blocked = false;
+      if (!LAZY)
+        while (L.leaves && !blocked) blocked = w8_leaf<LAYOUT, AM, COUNT, LAZY>(w, V, L, cnt);
+      if (blocked) L.phase = PH_DONE;
+      else next_node();
+    } else if (!LAZY) {
+      if (run == PH_ENTER) {
+        w8_enter<LAYOUT, AM, COUNT, LAZY, false>(w, V, L, L.node, cnt, false, 0);
+        if (L.phase == PH_ENTER) next_top();
       }
-      if (L.tsp == 0) {
-        w8_finish<LAYOUT, AM, COUNT>(w, V, L, src, cnt);
-        continue;
-      }
-      if (top8) {
-        L.tsp -= 2;
-        const uint32_t ex = tstack[L.tsp], ey = tstack[L.tsp + 1];
-        if (ey & W8_ENTRY) {  // a leaf's entry: an instance, at a node of its BLAS
-          w8_enter<LAYOUT, AM, COUNT, LAZY>(w, V, L, ex, cnt, true, ey & ~W8_ENTRY);
-          continue;
-        }
-        uint32_t bits = ey & 0xffu;  // a group: its first pending child now, the rest back on the stack
-        const uint32_t imask = ey >> 8, k = __ffs(bits) - 1;
-        bits &= bits - 1;
-        if (bits) tstack[L.tsp] = ex, tstack[L.tsp + 1] = bits | imask << 8, L.tsp += 2;
-        const uint32_t slot = k ^ octant_of(L.ray.d);
-        w8_top_node<COUNT>(V, top_cache, cached, ex + __popc(imask & ((1u << slot) - 1u)), L, tstack, L.tsp, st, cnt);
-        continue;
-      }
-      const uint32_t item = tstack[--L.tsp];
-      if (item & LEAF) {
-        w8_enter<LAYOUT, AM, COUNT, LAZY>(w, V, L, item & ~LEAF, cnt, true);
-        continue;
-      }
+    } else if (run == PH_LEAF) {
+      if (w8_leaf<LAYOUT, AM, COUNT, LAZY>(w, V, L, cnt)) L.phase = PH_DONE;
+      else if (L.leaves == 0) next_node();
+    } else if (run == PH_ENTER) {
+      w8_enter<LAYOUT, AM, COUNT, LAZY>(w, V, L, L.node, cnt, top != 0, L.at);
+      if (L.phase == PH_ENTER) next_top();
+    } else if (top8) {
+      w8_top_node<COUNT>(V, top_cache, cached, L.node, L, tstack, L.tsp, st, cnt);
+      next_top();
+    } else {
       const W8Best& b = L.best;
       const float bound = b.hit ? b.t + 2.0f * b.band + 2.0f * W8_TIE * b.t : b.t;
       w8_count<COUNT>(cnt, W8C_TOP_NODES);
-      top_step(w, top_base + (size_t)item * 32, L.ray, L.world_inv, bound, tstack, L.tsp, st);
+      top_step(w, top_base + (size_t)L.node * 32, L.ray, L.world_inv, bound, tstack, L.tsp, st);
+      next_top();
     }
   }
+  if (L.phase == PH_DONE) w8_finish<LAYOUT, AM, COUNT>(w, V, L, src, cnt);
 }
 
 // The packet walk's stacks, held in registers across the warp: entry i lives in lane i % 32, in
@@ -984,7 +1033,7 @@ RT_DEV uint32_t w8_packet_top(const uint32_t* __restrict__ w, size_t n, const W8
 // the visit order (conservative boxes, ties resolved in f64 on (t, instance, triangle)), so each
 // ray gets the hit the per-ray walk finds.
 template <uint32_t LAYOUT, int AM, int BLOCK, class Src>
-__global__ void __launch_bounds__(BLOCK, RT_W8P_MIN_BLOCKS) k_wide8_packet(const uint32_t* __restrict__ w, W8View V, const Src src,
+__global__ void __launch_bounds__(BLOCK, W8P_MIN_BLOCKS) k_wide8_packet(const uint32_t* __restrict__ w, W8View V, const Src src,
                                                            unsigned int* __restrict__ counter, uint32_t n, DevStatus* st) {
   __shared__ W8Decoded decoded[BLOCK / 32];
   W8Decoded& D = decoded[threadIdx.x / 32];
@@ -1030,7 +1079,7 @@ __global__ void __launch_bounds__(BLOCK, RT_W8P_MIN_BLOCKS) k_wide8_packet(const
       }
       L.phase = 0;
       if (live) w8_enter<LAYOUT, AM, false>(w, V, L, i, nullptr, false);
-      bool in = L.phase == 2;
+      bool in = L.phase == PH_NODE;
       const unsigned entering = __ballot_sync(0xffffffffu, in);
       if (!entering) continue;
       const uint32_t oct = __shfl_sync(0xffffffffu, L.R.oct, __ffs(entering) - 1);
@@ -1050,11 +1099,7 @@ __global__ void __launch_bounds__(BLOCK, RT_W8P_MIN_BLOCKS) k_wide8_packet(const
         const uint4 a0 = D.head[0], a1 = D.head[1];
         const uint32_t imask = a0.w >> 24, child_base = a1.x, tri_base = a1.y, meta_lo = a1.z, meta_hi = a1.w;
         uint32_t hits = 0;
-        if (in) {
-          const W8Best& best = L.best;
-          const float lim = best.hit ? best.t + 2.0f * best.band + W8_TIE * best.t : L.ray.tmax;
-          hits = w8_box_hits(L.R, D, a0, L.ray.tmin, lim);
-        }
+        if (in) hits = w8_box_hits(L.R, D, a0, L.ray.tmin, w8_limit(L));
         // leaves: every lane whose ray meets one tests its triangles
         for (uint32_t lh = __reduce_or_sync(0xffffffffu, hits & ~imask); lh; lh &= lh - 1) {
           const uint32_t s = __ffs(lh) - 1;
@@ -1062,7 +1107,7 @@ __global__ void __launch_bounds__(BLOCK, RT_W8P_MIN_BLOCKS) k_wide8_packet(const
           const uint32_t m = ((s < 4 ? meta_lo : meta_hi) >> (8 * (s & 3))) & 0xffu;
           const uint32_t first = tri_base + (m & 31u), cnt = m >> 5;
           for (uint32_t k = 0; k < cnt; ++k)
-            if (w8_candidate<LAYOUT, AM, false>(w, V, L.R, L.ray, L.inst, first + k, L.best, nullptr, L.any)) {
+            if (w8_candidate<LAYOUT, AM, false, false, false>(w, V, L.R, L.ray, L.inst, first + k, L.best, nullptr, L.any)) {
               in = false, live = false;  // an any-hit ray is blocked
               break;
             }
