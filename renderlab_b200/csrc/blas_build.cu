@@ -14,7 +14,7 @@
 // A split of a range is a node group when its binary depth is even: its halves, and the halves of
 // those halves, are the node's children (near_field.rs:286-306). The node ids follow postorder,
 // which is the order of (range end, range length). A child's slot is its order by range start.
-// Nodes are quantised bottom-up, one launch per node level, with the refit's device quantiser.
+// Nodes are quantised bottom-up by the refit's kernel.
 // An SAH tree deeper than 15 node levels is built again by median splits (near_field.rs:184-190).
 // The deepest node group then sits at binary depth 30 or more, which the level loop sees as it
 // gets there.
@@ -546,9 +546,10 @@ __global__ void k_link(const Seg* __restrict__ segs, uint32_t n, const uint32_t*
   kid_id[4 * (size_t)o + q] = id[s];
 }
 
-// A node's child slots in range order.
+// A node's child slots in range order, its inner children's parent and their count.
 __global__ void k_node_children(uint32_t n, const uint32_t* __restrict__ kid_n, const uint32_t* __restrict__ kid_b,
-                                const uint32_t* __restrict__ kid_id, uint32_t* __restrict__ nodes) {
+                                const uint32_t* __restrict__ kid_id, uint32_t* __restrict__ nodes,
+                                uint32_t* __restrict__ parent, uint8_t* __restrict__ inner) {
   const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
   const uint32_t m = min(kid_n[r], 4u);
@@ -560,28 +561,13 @@ __global__ void k_node_children(uint32_t n, const uint32_t* __restrict__ kid_n, 
       b[p] = b[p - 1], c[p] = c[p - 1];
       b[p - 1] = tb, c[p - 1] = tc;
     }
-  for (uint32_t q = 0; q < 4; ++q) nodes[16 * (size_t)r + 6 + q] = q < m ? c[q] : EMPTY;
-}
-
-// Quantises the node groups of one level (their node children are a level pair deeper, done).
-__global__ void k_quantize_level(const Seg* __restrict__ segs, uint32_t lv0, uint32_t width, const uint32_t* __restrict__ id,
-                                 View v) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= width) return;
-  const Seg g = segs[lv0 + i];
-  if (g.e - g.b <= LEAF_TRIS || (g.depth & 1u)) return;
-  uint32_t* w = v.w + v.nodes + 16 * (size_t)id[lv0 + i];
-  uint32_t kids[4];
-  Box boxes[4];
-  int m = 0;
-  for (int s = 0; s < 4; ++s) {
-    const uint32_t c = w[6 + s];
-    if (c == EMPTY) continue;
-    kids[m] = c;
-    boxes[m] = child_box(v, c);
-    ++m;
+  uint32_t kids = 0;
+  for (uint32_t q = 0; q < 4; ++q) {
+    nodes[16 * (size_t)r + 6 + q] = q < m ? c[q] : EMPTY;
+    if (q < m && !(c[q] & LEAF)) parent[c[q]] = r, ++kids;
   }
-  quantize(w, kids, boxes, m);
+  inner[r] = (uint8_t)kids;
+  if (r == n - 1) parent[r] = EMPTY;  // postorder: the root
 }
 
 // Device memory for one build, carved out of one allocation; freed once the build's stream has
@@ -735,18 +721,15 @@ rt_status rt_blas_build_device(rt_ctx* ctx, const float* positions, uint32_t n_p
   RT_CUDA(ctx, cudaGetLastError());
 
   // The level loop; an SAH tree past 15 node levels starts over with median splits.
-  std::vector<std::pair<uint32_t, uint32_t>> levels;  // (first range, ranges) of each binary depth
   std::vector<LargeSeg> large;
   std::vector<Chunk> chunks;
   uint32_t total = 0;
   for (;;) {
-    levels.clear();
     const Seg root{0, nt, 0, EMPTY};
     RT_CUDA(ctx, cudaMemcpyAsync(d_segs, &root, sizeof root, cudaMemcpyHostToDevice, st));
     uint32_t lv0 = 0, width = 1, depth = 0;
     bool too_deep = false;
     for (;;) {
-      levels.emplace_back(lv0, width);
       k_level_flags<<<blocks(width + 1, 256), 256, 0, st>>>(d_segs + lv0, width, d_flags);
       size_t nb = 0;
       RT_CUDA(ctx, cub::DeviceScan::ExclusiveSum(nullptr, nb, d_flags, d_rank, (int)width + 1, st));
@@ -848,6 +831,9 @@ rt_status rt_blas_build_device(rt_ctx* ctx, const float* positions, uint32_t n_p
   rec.plan<uint32_t>(nn);  // node ranges, sorted
   rec.plan<uint32_t>(nn);
   rec.plan<uint32_t>(nn);  // children per node
+  rec.plan<uint32_t>(nn);  // parents
+  rec.plan<uint32_t>(nn);  // inner children done
+  rec.plan<uint8_t>(nn);   // inner children
   rec.plan<uint32_t>(4 * nn);
   rec.plan<uint32_t>(4 * nn);
   rec.plan<char>(sort_bytes);
@@ -862,6 +848,9 @@ rt_status rt_blas_build_device(rt_ctx* ctx, const float* positions, uint32_t n_p
   uint32_t* d_node_seg = rec.take<uint32_t>(nn);
   uint32_t* d_node_seg_sorted = rec.take<uint32_t>(nn);
   uint32_t* d_kid_n = rec.take<uint32_t>(nn);
+  uint32_t* d_parent = rec.take<uint32_t>(nn);
+  uint32_t* d_done = rec.take<uint32_t>(nn);
+  uint8_t* d_inner = rec.take<uint8_t>(nn);
   uint32_t* d_kid_b = rec.take<uint32_t>(4 * nn);
   uint32_t* d_kid_id = rec.take<uint32_t>(4 * nn);
   void* d_sort = rec.take<char>(sort_bytes);
@@ -880,15 +869,12 @@ rt_status rt_blas_build_device(rt_ctx* ctx, const float* positions, uint32_t n_p
   if (n_nodes) {
     RT_CUDA(ctx, cudaMemsetAsync(d_kid_n, 0, 4 * (size_t)n_nodes, st));
     k_link<<<blocks(total, 256), 256, 0, st>>>(d_segs, total, d_id, d_kid_n, d_kid_b, d_kid_id);
-    k_node_children<<<blocks(n_nodes, 256), 256, 0, st>>>(n_nodes, d_kid_n, d_kid_b, d_kid_id, d_nodes);
+    k_node_children<<<blocks(n_nodes, 256), 256, 0, st>>>(n_nodes, d_kid_n, d_kid_b, d_kid_id, d_nodes, d_parent, d_inner);
+    RT_CUDA(ctx, cudaMemsetAsync(d_done, 0, 4 * (size_t)n_nodes, st));
     View v{};
     v.w = d_out, v.layout = 0, v.nodes = out_nodes, v.leaves = out_leaves, v.indices = out_indices,
     v.positions = out_positions;
-    for (size_t d = levels.size(); d-- > 0;) {
-      if (d & 1) continue;
-      const uint32_t lv0 = levels[d].first, width = levels[d].second;
-      k_quantize_level<<<blocks(width, 128), 128, 0, st>>>(d_segs, lv0, width, d_id, v);
-    }
+    k_refit_up<REFIT_BLOCK><<<blocks(4 * (size_t)n_nodes, REFIT_BLOCK), REFIT_BLOCK, 0, st>>>(v, n_nodes, d_parent, d_inner, d_done);
   }
   RT_CUDA(ctx, cudaGetLastError());
 

@@ -16,14 +16,12 @@
 #include "host/wide8.hpp"
 #include "launch.hpp"
 
-// Per BLAS of a scene, what rt_scene_refit needs about its (fixed) topology: its nodes ordered
-// by height above the leaves, and where each height starts.
+// Per BLAS of a scene, what rt_scene_refit needs about its (fixed) topology.
 struct RefitLevels {
   uint32_t node_count = 0;
-  uint32_t tri_count = 0;           // reflection layout: packed triangles of the BLAS
-  uint32_t position_count = 0;      // GI layout: position records of the BLAS
-  std::vector<uint32_t> level_start;  // level h: d_order[level_start[h], level_start[h + 1])
-  uint32_t* d_order = nullptr;
+  uint32_t tri_count = 0;       // reflection layout: packed triangles of the BLAS
+  uint32_t position_count = 0;  // GI layout: position records of the BLAS
+  uint32_t* d_tree = nullptr;   // per node: its parent, a counter, and (bytes) its inner children
 };
 
 struct rt_scene {
@@ -31,6 +29,7 @@ struct rt_scene {
   uint32_t* d_words = nullptr;
   size_t n_words = 0;
   rtb::SceneInfo info;
+  std::vector<uint32_t> blas_words;  // words 18-23 of each instance record: its BLAS (rt_scene_refit reads them here)
   size_t device_bytes = 0;
   void* d_wide8 = nullptr;
   size_t wide8_bytes = 0;

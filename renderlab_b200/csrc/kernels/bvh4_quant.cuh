@@ -76,7 +76,12 @@ inline __device__ Box child_box(const View& v, uint32_t c) {
     }
     return b;
   }
-  const uint32_t* n = v.w + v.nodes + 16 * (size_t)c;
+  // another thread block may have written the child in this launch: past L1
+  const uint32_t* p = v.w + v.nodes + 16 * (size_t)c;
+  uint32_t n[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) n[k] = __ldcg(p + k);
+#pragma unroll
   for (int t = 0; t < 4; ++t) {
     if (n[6 + t] == EMPTY) continue;
     for (int fused = 0; fused < 2; ++fused)
@@ -89,32 +94,87 @@ inline __device__ Box child_box(const View& v, uint32_t c) {
   return b;
 }
 
-// quantize_node: the node's origin and step per axis, then the outward 8-bit planes of each child.
-inline __device__ void quantize(uint32_t* w, const uint32_t* kids, const Box* boxes, int n) {
-  Box all = empty_box();
-  for (int k = 0; k < n; ++k)
-    for (int a = 0; a < 3; ++a) all.lo[a] = lo_of(all.lo[a], boxes[k].lo[a]), all.hi[a] = hi_of(all.hi[a], boxes[k].hi[a]);
-  float step[3];
-  for (int a = 0; a < 3; ++a) {
-    const float lo = all.lo[a], hi = all.hi[a];
-    float s = hi_of(__fdiv_rn(__fsub_rn(hi, lo), 255.0f), hi_of(FLT_MIN, __fmul_rn(fabsf(lo), 1e-7f)));
-    while (__fadd_rn(lo, __fmul_rn(s, 255.0f)) < hi || __fmaf_rn(s, 255.0f, lo) < hi) s = __fmul_rn(s, 1.0f + 1.0f / 1048576.0f);
-    step[a] = s;
-  }
-  uint32_t lower[3] = {0, 0, 0}, upper[3] = {0, 0, 0};
-  for (int k = 0; k < n; ++k)
+// One node by four lanes (`quad`: their mask, `c`: this lane's 0-3), a child each: the children's
+// boxes, quantize_node's origin and step per axis, and each child's outward 8-bit planes. Minima and
+// maxima prefer the earlier child of two equal values, as the host's sequential pass does.
+inline __device__ void refit_node(const View& v, uint32_t node, unsigned quad, int c) {
+  uint32_t* w = v.w + v.nodes + 16 * (size_t)node;
+  const uint32_t id = w[6 + c];
+  const bool here = id != EMPTY;
+  const unsigned present = (__ballot_sync(quad, here) >> (__ffs(quad) - 1)) & 0xfu;
+  const int n = __popc(present), k = __popc(present & ((1u << c) - 1u));  // k: the child's place among those present
+  const Box box = here ? child_box(v, id) : empty_box();
+  Box all = box;
+  for (int step = 1; step < 4; step *= 2)
     for (int a = 0; a < 3; ++a) {
-      const float o = all.lo[a], s = step[a], x = boxes[k].lo[a], y = boxes[k].hi[a];
-      uint32_t ql = to_u8(floorf(__fdiv_rn(__fsub_rn(x, o), s)));
-      while (ql > 0 && (plane(o, s, ql, false) > x || plane(o, s, ql, true) > x)) --ql;
-      uint32_t qh = to_u8(ceilf(__fdiv_rn(__fsub_rn(y, o), s)));
-      while (qh < 255 && (plane(o, s, qh, false) < y || plane(o, s, qh, true) < y)) ++qh;
-      lower[a] |= ql << (8 * k);
-      upper[a] |= qh << (8 * k);
+      const float lo = __shfl_xor_sync(quad, all.lo[a], step), hi = __shfl_xor_sync(quad, all.hi[a], step);
+      all.lo[a] = (c & step) ? lo_of(lo, all.lo[a]) : lo_of(all.lo[a], lo);
+      all.hi[a] = (c & step) ? hi_of(hi, all.hi[a]) : hi_of(all.hi[a], hi);
     }
-  for (int a = 0; a < 3; ++a) w[a] = __float_as_uint(all.lo[a]), w[3 + a] = __float_as_uint(step[a]);
-  for (int s = 0; s < 4; ++s) w[6 + s] = s < n ? kids[s] : EMPTY;
-  for (int a = 0; a < 3; ++a) w[10 + a] = lower[a], w[13 + a] = upper[a];
+  float mine = 0.0f;  // lanes 0-2: the step of one axis
+  if (c < 3) {
+    const float lo = c == 0 ? all.lo[0] : (c == 1 ? all.lo[1] : all.lo[2]), hi = c == 0 ? all.hi[0] : (c == 1 ? all.hi[1] : all.hi[2]);
+    mine = hi_of(__fdiv_rn(__fsub_rn(hi, lo), 255.0f), hi_of(FLT_MIN, __fmul_rn(fabsf(lo), 1e-7f)));
+    while (__fadd_rn(lo, __fmul_rn(mine, 255.0f)) < hi || __fmaf_rn(mine, 255.0f, lo) < hi)
+      mine = __fmul_rn(mine, 1.0f + 1.0f / 1048576.0f);
+  }
+  const int first = __ffs(quad) - 1;
+  uint32_t planes[6];  // lower x, y, z, upper x, y, z
+  float steps[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float o = all.lo[a], s = __shfl_sync(quad, mine, first + a), x = box.lo[a], y = box.hi[a];
+    steps[a] = s;
+    uint32_t ql = 0, qh = 0;
+    if (here) {
+      ql = to_u8(floorf(__fdiv_rn(__fsub_rn(x, o), s)));
+      while (ql > 0 && (plane(o, s, ql, false) > x || plane(o, s, ql, true) > x)) --ql;
+      qh = to_u8(ceilf(__fdiv_rn(__fsub_rn(y, o), s)));
+      while (qh < 255 && (plane(o, s, qh, false) < y || plane(o, s, qh, true) < y)) ++qh;
+    }
+    planes[a] = ql << (8 * k), planes[3 + a] = qh << (8 * k);
+  }
+  if (!here)  // places past the children present
+    for (int a = 0; a < 6; ++a) planes[a] = 0;
+  for (int step = 1; step < 4; step *= 2)
+    for (int a = 0; a < 6; ++a) planes[a] |= __shfl_xor_sync(quad, planes[a], step);
+  w[6 + (here ? k : n + c - k)] = here ? id : EMPTY;
+  if (c < 3) {
+    w[c] = __float_as_uint(c == 0 ? all.lo[0] : (c == 1 ? all.lo[1] : all.lo[2]));
+    w[3 + c] = __float_as_uint(c == 0 ? steps[0] : (c == 1 ? steps[1] : steps[2]));
+    w[10 + c] = c == 0 ? planes[0] : (c == 1 ? planes[1] : planes[2]);
+    w[13 + c] = c == 0 ? planes[3] : (c == 1 ? planes[4] : planes[5]);
+  }
+}
+
+constexpr uint8_t NEVER = 0xff;  // inner children of a node that is not refit
+
+// Every node of a BLAS, children before parents, in one launch: four lanes start at each node without
+// inner children (inner[node] == 0) and climb; of a node's inner children, the last one done takes
+// the node (done[], zeroed before the launch). A launch per height had the upper heights wait on a
+// few lone warps each: 250k triangles, 10 heights, 218 us against 60. Nothing waits.
+constexpr int REFIT_BLOCK = 128;
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK) k_refit_up(View v, uint32_t n, const uint32_t* __restrict__ parent,
+                                                    const uint8_t* __restrict__ inner, uint32_t* __restrict__ done) {
+  const uint32_t i = (blockIdx.x * BLOCK + threadIdx.x) / 4;
+  if (i >= n || inner[i] != 0) return;
+  const int c = threadIdx.x & 3;
+  const unsigned quad = 0xfu << (threadIdx.x & 28);
+  for (uint32_t node = i;;) {
+    refit_node(v, node, quad, c);
+    const uint32_t up = parent[node];
+    if (up == EMPTY) return;
+    __syncwarp(quad);  // the four lanes' words are written
+    uint32_t last = 0;
+    if (c == 0) {
+      __threadfence();
+      last = atomicAdd(&done[up], 1u) + 1u == inner[up] ? 1u : 0u;
+      __threadfence();
+    }
+    if (!__shfl_sync(quad, last, 0, 4)) return;
+    node = up;
+  }
 }
 
 }  // namespace rtq

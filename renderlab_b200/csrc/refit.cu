@@ -1,10 +1,10 @@
 // GPU refit of one BLAS of an uploaded scene (near_field::refit_bvh, near_field.rs:445-478, on the
 // device): new positions for the same vertices, the BVH4-Q8 node boxes recomputed bottom-up and
 // quantised with the host quantiser's exact arithmetic (quantize_node, near_field.rs:481-525), so
-// the words equal those of rt_blas_refit followed by packing, bit for bit. Nodes of one height
-// above the leaves are independent: one launch per height.
+// the words equal those of rt_blas_refit followed by packing, bit for bit.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <vector>
@@ -18,23 +18,6 @@ using namespace rtc;
 namespace {
 
 using namespace rtq;
-
-__global__ void k_refit_nodes(View v, const uint32_t* __restrict__ order, uint32_t count) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  uint32_t* w = v.w + v.nodes + 16 * (size_t)order[i];
-  uint32_t kids[4];
-  Box boxes[4];
-  int m = 0;
-  for (int s = 0; s < 4; ++s) {
-    const uint32_t c = w[6 + s];
-    if (c == EMPTY) continue;
-    kids[m] = c;
-    boxes[m] = child_box(v, c);
-    ++m;
-  }
-  quantize(w, kids, boxes, m);
-}
 
 // GI: the new positions into the BLAS's position words.
 __global__ void k_refit_positions(uint32_t* __restrict__ dst, const float* __restrict__ pos, uint32_t n_floats) {
@@ -68,46 +51,49 @@ rt_status levels_of(rt_ctx* ctx, rt_scene* scene, const uint32_t* rec, RefitLeve
   const uint32_t n = root + 1;    // postorder: the root is the last node
   std::vector<uint32_t> w(16 * (size_t)n);
   RT_CUDA(ctx, cudaMemcpy(w.data(), scene->d_words + nodes, w.size() * 4, cudaMemcpyDeviceToHost));
-  std::vector<uint32_t> height(n, 0);
-  uint32_t top = 0, tris = 0, leaves_max = 0;
+  uint32_t tris = 0;
   for (uint32_t k = 0; k < n; ++k) {
-    uint32_t h = 0;
     for (int s = 0; s < 4; ++s) {
       const uint32_t c = w[16 * (size_t)k + 6 + s];
       if (c == EMPTY) continue;
       if (c & LEAF) {
-        if (gi) leaves_max = std::max(leaves_max, (c & ~LEAF) + 1);
-        else tris = std::max(tris, ((c & ~LEAF) >> 4) + (c & 15u));
-      } else if (c < k) {
-        h = std::max(h, height[c]);
-      } else {
+        if (!gi) tris = std::max(tris, ((c & ~LEAF) >> 4) + (c & 15u));
+      } else if (c >= k) {
         return fail(ctx, RT_ERR_LAYOUT, "refit: BLAS children must precede their parent");
       }
     }
-    height[k] = h + 1;
-    top = std::max(top, h + 1);
   }
-  std::vector<uint32_t> order;
-  order.reserve(n);
-  out.level_start.assign(top + 1, 0);
-  for (uint32_t h = 1; h <= top; ++h) {
-    out.level_start[h - 1] = (uint32_t)order.size();
-    for (uint32_t k = 0; k < n; ++k)
-      if (height[k] == h) order.push_back(k);
+  // the tree from the root: each node's parent and inner children (a node it does not reach is left)
+  std::vector<uint32_t> parent(n, EMPTY);
+  std::vector<uint8_t> inner(n, rtq::NEVER);
+  inner[root] = 0;
+  for (uint32_t k = n; k-- > 0;) {
+    if (inner[k] == rtq::NEVER) continue;
+    for (int s = 0; s < 4; ++s) {
+      const uint32_t c = w[16 * (size_t)k + 6 + s];
+      if (c == EMPTY || (c & LEAF)) continue;
+      parent[c] = k, inner[c] = 0, ++inner[k];
+    }
   }
-  out.level_start[top] = (uint32_t)order.size();
   out.node_count = n;
   out.tri_count = tris;
-  (void)leaves_max;
   if (gi) {  // the packer lays a mesh's positions (3 words each) right before its indices
     if (rec[21] < rec[20] || (rec[21] - rec[20]) % 3 != 0) return fail(ctx, RT_ERR_LAYOUT, "refit: GI position words");
     out.position_count = (rec[21] - rec[20]) / 3;
   }
-  if (cudaMalloc(&out.d_order, std::max<size_t>(order.size(), 1) * 4) != cudaSuccess) {
+  // one allocation: parents, counters of a launch, inner child counts
+  if (cudaMalloc(&out.d_tree, 9 * (size_t)n) != cudaSuccess) {
     cudaGetLastError();
-    return fail(ctx, RT_ERR_OOM, "refit node order");
+    out.d_tree = nullptr;
+    return fail(ctx, RT_ERR_OOM, "refit tree");
   }
-  RT_CUDA(ctx, cudaMemcpy(out.d_order, order.data(), order.size() * 4, cudaMemcpyHostToDevice));
+  cudaError_t e = cudaMemcpy(out.d_tree, parent.data(), 4 * (size_t)n, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(out.d_tree + 2 * (size_t)n, inner.data(), n, cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    cudaFree(out.d_tree);
+    out.d_tree = nullptr;
+    return fail(ctx, RT_ERR_CUDA, "refit tree: %s", cudaGetErrorString(e));
+  }
   return RT_OK;
 }
 
@@ -123,9 +109,8 @@ rt_status rt_scene_refit(rt_ctx* ctx, rt_scene* scene, uint32_t instance, const 
   if (!gi && !d_indices) return fail(ctx, RT_ERR_INVALID_ARG, "the reflection layout refits from the triangle list");
   std::lock_guard<std::mutex> lock(ctx->mu);
   RT_CUDA(ctx, cudaSetDevice(ctx->device));
-  uint32_t rec[24];
-  const size_t r = gi ? 16 + 32 * (size_t)instance : 8 + 24 * (size_t)instance;
-  RT_CUDA(ctx, cudaMemcpy(rec, scene->d_words + r, 24 * 4, cudaMemcpyDeviceToHost));
+  uint32_t rec[24] = {};
+  std::copy_n(scene->blas_words.begin() + 6 * (size_t)instance, 6, rec + 18);
   const uint32_t base = gi ? rec[18] : (rec[18] & ~3u);
   auto it = scene->refit.find(base);
   if (it == scene->refit.end()) {
@@ -160,9 +145,11 @@ rt_status rt_scene_refit(rt_ctx* ctx, rt_scene* scene, uint32_t instance, const 
     if (lv.tri_count) k_refit_triangles<<<(lv.tri_count + 255) / 256, 256, 0, s>>>(v, lv.tri_count);
   }
   RT_CUDA(ctx, cudaGetLastError());
-  for (size_t h = 0; h + 1 < lv.level_start.size(); ++h) {
-    const uint32_t a = lv.level_start[h], n = lv.level_start[h + 1] - a;
-    if (n) k_refit_nodes<<<(n + 127) / 128, 128, 0, s>>>(v, lv.d_order + a, n);
+  if (lv.node_count) {
+    const uint32_t n = lv.node_count;
+    RT_CUDA(ctx, cudaMemsetAsync(lv.d_tree + n, 0, 4 * (size_t)n, s));
+    k_refit_up<REFIT_BLOCK><<<(uint32_t)((4 * (uint64_t)n + REFIT_BLOCK - 1) / REFIT_BLOCK), REFIT_BLOCK, 0, s>>>(
+        v, n, lv.d_tree, reinterpret_cast<const uint8_t*>(lv.d_tree + 2 * (size_t)n), lv.d_tree + n);
   }
   RT_CUDA(ctx, cudaGetLastError());
   return RT_OK;

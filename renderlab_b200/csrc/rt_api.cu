@@ -171,6 +171,14 @@ bool same_instances(uint32_t layout, const uint32_t* a, const uint32_t* b) {
   return true;
 }
 
+// The host's copy of the records' BLAS words, after an upload or a rewrite of the records.
+void keep_blas_words(rt_scene* s, const uint32_t* words) {
+  const size_t header = s->layout == 0 ? 16 : 8, stride = s->layout == 0 ? 32 : 24;
+  s->blas_words.resize(6 * (size_t)s->info.instances);
+  for (uint32_t i = 0; i < s->info.instances; ++i)
+    std::copy_n(words + header + stride * (size_t)i + 18, 6, s->blas_words.begin() + 6 * (size_t)i);
+}
+
 }  // namespace
 
 extern "C" {
@@ -279,6 +287,7 @@ rt_status rt_scene_upload(rt_ctx* ctx, rt_layout layout, const uint32_t* words, 
     cudaFree(s->d_words);
     return fail(ctx, RT_ERR_CUDA, "scene copy: %s", cudaGetErrorString(e));
   }
+  keep_blas_words(s.get(), words);
   ctx->scene_bytes += s->device_bytes;
   *out = s.release();
   return RT_OK;
@@ -319,6 +328,7 @@ rt_status rt_scene_update_records(rt_ctx* ctx, rt_scene* scene, const uint32_t* 
   if (scene->d_wide8 && !same_instances(scene->layout, before.data(), all.data())) drop_wide8(ctx, scene);
   RT_CUDA(ctx, cudaMemcpy(scene->d_words, words, n_words * 4, cudaMemcpyHostToDevice));
   scene->info = info;
+  keep_blas_words(scene, all.data());
   scene->w8_top_valid = false;  // the instances' boxes may have moved: the packed top level until re-prepared
   return RT_OK;
 }
@@ -515,7 +525,7 @@ rt_status rt_scene_release(rt_ctx* ctx, rt_scene* scene) {
   cudaFree(scene->d_w8_top);
   cudaFree(scene->d_move);
   cudaFree(scene->d_top_order);
-  for (auto& kv : scene->refit) cudaFree(kv.second.d_order);
+  for (auto& kv : scene->refit) cudaFree(kv.second.d_tree);
   ctx->scene_bytes -= scene->device_bytes;
   delete scene;
   return RT_OK;
