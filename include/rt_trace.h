@@ -461,11 +461,11 @@ rt_status rt_object_box(rt_layout layout, const rt_blas* blas, const float* posi
  * rt_scene_move_instances does the same on the device. */
 rt_status rt_move_instances_host(rt_layout layout, uint32_t* words, size_t n_words, const rt_instance* instances,
                                  uint32_t n, const float* mesh_boxes, uint32_t n_meshes);
-/* The same on an uploaded scene, on the device (records, top-level refit one launch per level,
+/* The same on an uploaded scene, on the device (records, top-level refit in one launch,
  * the rebuild after 64 refits, scene bounds), with rt_move_instances_host's words bit for bit:
  * the per-frame instance update of the reference (instance_words + instance_bvh::place,
- * src/instance_bvh.rs:162-275) without a host round trip. Host arrays; it reads the scene's
- * header and, on the first call, the top level's topology, synchronously. */
+ * src/instance_bvh.rs:162-275) without a host round trip. Host arrays; it reads, on the first
+ * call, the top level's topology synchronously. */
 rt_status rt_scene_move_instances(rt_ctx* ctx, rt_scene* scene, const rt_instance* instances, uint32_t n,
                                   const float* mesh_boxes, uint32_t n_meshes, void* stream);
 

@@ -29,6 +29,7 @@ struct rt_scene {
   uint32_t* d_words = nullptr;
   size_t n_words = 0;
   rtb::SceneInfo info;
+  uint32_t head[8] = {};  // the header's first words, as they are on the device
   std::vector<uint32_t> blas_words;  // words 18-23 of each instance record: its BLAS (rt_scene_refit reads them here)
   size_t device_bytes = 0;
   void* d_wide8 = nullptr;
@@ -47,11 +48,12 @@ struct rt_scene {
 
   std::map<uint32_t, RefitLevels> refit;  // by the BLAS's node base word
   // rt_scene_move_instances: staging for the moved instances and mesh boxes, and the top level's
-  // nodes grouped by height (deepest last), kept until a rebuild changes the tree.
+  // links (see k_refit_top), made by the first move and by each rebuild.
+  std::vector<char> move_stage;
   void* d_move = nullptr;
   size_t move_bytes = 0;
-  std::vector<uint32_t> top_order, top_level_start;
-  uint32_t* d_top_order = nullptr;
+  uint32_t* d_top_tree = nullptr;
+  uint32_t top_nodes = 0;  // nodes the links cover; 0: not made yet
 };
 
 struct rt_blas {
@@ -102,11 +104,10 @@ namespace rtc {
 
 // The instance top level built on the device (tlas_build.cu), word for word rtb::tlas_build's:
 // instance i's box is lo xyz at d_box_words[i * stride], hi xyz right after (float bits). The
-// nodes go to d_out (cap_words available, the rest zeroed); with d_order, the node ids grouped
-// by level, deepest first (a bottom-up refit order), level starts in *level_start. Synchronous
+// nodes go to d_out (cap_words available, the rest zeroed). Synchronous
 // on `st`; the caller holds the context's lock.
 rt_status tlas_build_device(rt_ctx* ctx, const uint32_t* d_box_words, size_t stride, uint32_t n, bool sah, uint32_t* d_out,
-                            size_t cap_words, uint32_t* d_order, std::vector<uint32_t>* level_start, uint32_t* n_nodes,
+                            size_t cap_words, uint32_t* n_nodes,
                             cudaStream_t st);
 
 constexpr size_t GI_HIT_BYTES = 40, RS_HIT_BYTES = 20, ANY_HIT_BYTES = 4, RAY_BYTES = 32;

@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "ctx.hpp"
@@ -22,11 +23,6 @@ using rtk::EMPTY;
 using rtk::LEAF;
 
 constexpr size_t TOP_WORDS = 32;  // a top-level node: 24 box words, 4 child ids, 4 unused
-
-struct Moved {  // one instance's new placement, as staged on the device
-  float model[12], rows[12];
-  uint32_t mesh, pad[3];
-};
 
 struct Box {
   float lo[3], hi[3];
@@ -70,51 +66,91 @@ __device__ Box instance_box(uint32_t layout, const float* m, const float* obj) {
   return out;
 }
 
-__global__ void k_move_records(uint32_t* __restrict__ w, uint32_t layout, const Moved* __restrict__ moved, uint32_t n,
-                               const float* __restrict__ mesh_boxes) {
+__global__ void k_move_records(uint32_t* __restrict__ w, uint32_t layout, const rt_instance* __restrict__ moved, uint32_t n,
+                               const float* __restrict__ mesh_boxes, uint32_t refits) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) w[3] = refits;
   if (i >= n) return;
-  const Moved& g = moved[i];
+  const rt_instance& g = moved[i];
   uint32_t* r = w + (layout == 0 ? 16 + 32 * (size_t)i : 8 + 24 * (size_t)i);
   for (int k = 0; k < 12; ++k) r[k] = __float_as_uint(g.rows[k]);
   const Box b = instance_box(layout, g.model, mesh_boxes + 6 * (size_t)g.mesh);
   for (int a = 0; a < 3; ++a) r[12 + a] = __float_as_uint(b.lo[a]), r[15 + a] = __float_as_uint(b.hi[a]);
 }
 
-// One height of the top level: each node's child boxes from its instances' records or from its
-// inner children's (already refit) boxes, grown in slot order as instance_bvh::refit_wide does.
-__global__ void k_refit_top(uint32_t* __restrict__ w, uint32_t layout, size_t base, const uint32_t* __restrict__ order,
-                            uint32_t first, uint32_t count) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  uint32_t* node = w + base + TOP_WORDS * (size_t)order[first + k];
-  for (int c = 0; c < 4; ++c) {
+constexpr uint8_t NEVER = 0xff;  // inner children of a node that is not refit
+
+// The top level refit over the records' boxes in one launch: four lanes a node, a child each, climb
+// from the nodes without inner children; of a node's inner children the last one done takes the
+// node (done[], zeroed before the launch; nothing waits). An inner child's box is grown in slot order
+// as instance_bvh::refit_wide does. 2,500 instances, 6 heights: 40 us as a launch per height with a
+// thread a node, 16 so (the whole call, its copies included: 144 -> 62 us).
+constexpr int TOP_BLOCK = 128;
+__global__ void __launch_bounds__(TOP_BLOCK) k_refit_top(uint32_t* __restrict__ w, uint32_t layout, size_t base, uint32_t n,
+                                                         const uint32_t* __restrict__ parent,
+                                                         const uint8_t* __restrict__ inner, uint32_t* __restrict__ done) {
+  const uint32_t i = (blockIdx.x * TOP_BLOCK + threadIdx.x) / 4;
+  if (i >= n || inner[i] != 0) return;
+  const int c = threadIdx.x & 3;
+  const unsigned quad = 0xfu << (threadIdx.x & 28);
+  for (uint32_t at = i;;) {
+    uint32_t* node = w + base + TOP_WORDS * (size_t)at;
     const uint32_t id = node[24 + c];
-    if (id == EMPTY) continue;
-    Box b;
-    if (id & LEAF) {
-      const uint32_t* r = w + (layout == 0 ? 16 + 32 * (size_t)(id & ~LEAF) : 8 + 24 * (size_t)(id & ~LEAF));
-      for (int a = 0; a < 3; ++a) b.lo[a] = __uint_as_float(r[12 + a]), b.hi[a] = __uint_as_float(r[15 + a]);
-    } else {
-      const uint32_t* child = w + base + TOP_WORDS * (size_t)id;
-      b = empty_box();
-      for (int cc = 0; cc < 4; ++cc) {
-        if (child[24 + cc] == EMPTY) continue;
-        float l[3], h[3];
-        for (int a = 0; a < 3; ++a) l[a] = __uint_as_float(child[4 * a + cc]), h[a] = __uint_as_float(child[12 + 4 * a + cc]);
-        grow(b, l, h);
+    if (id != EMPTY) {
+      Box b;
+      if (id & LEAF) {
+        const uint32_t* r = w + (layout == 0 ? 16 + 32 * (size_t)(id & ~LEAF) : 8 + 24 * (size_t)(id & ~LEAF));
+        for (int a = 0; a < 3; ++a) b.lo[a] = __uint_as_float(r[12 + a]), b.hi[a] = __uint_as_float(r[15 + a]);
+      } else {  // another thread block may have written it in this launch: past L1
+        const uint32_t* child = w + base + TOP_WORDS * (size_t)id;
+        uint32_t x[28];
+#pragma unroll
+        for (int k = 0; k < 28; ++k) x[k] = __ldcg(child + k);
+        b = empty_box();
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) {
+          if (x[24 + cc] == EMPTY) continue;
+          float l[3], h[3];
+          for (int a = 0; a < 3; ++a) l[a] = __uint_as_float(x[4 * a + cc]), h[a] = __uint_as_float(x[12 + 4 * a + cc]);
+          grow(b, l, h);
+        }
       }
+      for (int a = 0; a < 3; ++a) node[4 * a + c] = __float_as_uint(b.lo[a]), node[12 + 4 * a + c] = __float_as_uint(b.hi[a]);
     }
-    for (int a = 0; a < 3; ++a) node[4 * a + c] = __float_as_uint(b.lo[a]), node[12 + 4 * a + c] = __float_as_uint(b.hi[a]);
+    const uint32_t up = parent[at];
+    if (up == EMPTY) return;
+    __syncwarp(quad);  // the four lanes' words are written
+    uint32_t last = 0;
+    if (c == 0) {
+      __threadfence();
+      last = atomicAdd(&done[up], 1u) + 1u == inner[up] ? 1u : 0u;
+      __threadfence();
+    }
+    if (!__shfl_sync(quad, last, 0, 4)) return;
+    at = up;
   }
 }
 
+// Parents and inner child counts of a tree built on the device (nodes 0 to n - 1, the root first).
+__global__ void k_top_links(const uint32_t* __restrict__ nodes, uint32_t n, uint32_t* __restrict__ parent,
+                            uint8_t* __restrict__ inner) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  uint32_t kids = 0;
+  for (int c = 0; c < 4; ++c) {
+    const uint32_t id = nodes[TOP_WORDS * (size_t)i + 24 + c];
+    if (id != EMPTY && !(id & LEAF)) parent[id] = i, ++kids;
+  }
+  inner[i] = (uint8_t)kids;
+  if (i == 0) parent[0] = EMPTY;
+}
+
 // The reflection scene bounds: the instances' boxes grown in record order. Each thread grows a
-// contiguous run, then thread 0 grows the runs in order; a strict comparison keeps the earlier of
-// two equal values (+0 and -0), as one sequential pass does.
-constexpr int BOUNDS_THREADS = 256;
-__global__ void k_scene_bounds(uint32_t* __restrict__ w, uint32_t n) {
-  __shared__ Box part[BOUNDS_THREADS];
+// contiguous run, then the runs are combined in order, neighbours first; a strict comparison keeps
+// the earlier of two equal values (+0 and -0), as one sequential pass does.
+constexpr int BOUNDS_THREADS = 512;
+__global__ void __launch_bounds__(BOUNDS_THREADS) k_scene_bounds(uint32_t* __restrict__ w, uint32_t n) {
+  __shared__ Box part[BOUNDS_THREADS / 32];
   const uint32_t t = threadIdx.x, per = (n + BOUNDS_THREADS - 1) / BOUNDS_THREADS;
   Box b = empty_box();
   for (uint32_t i = t * per; i < n && i < (t + 1) * per; ++i) {
@@ -123,48 +159,44 @@ __global__ void k_scene_bounds(uint32_t* __restrict__ w, uint32_t n) {
     for (int a = 0; a < 3; ++a) l[a] = __uint_as_float(r[12 + a]), h[a] = __uint_as_float(r[15 + a]);
     grow(b, l, h);
   }
-  part[t] = b;
+  auto combine = [](Box& x, int lanes) {
+    for (int off = 1; off < lanes; off *= 2) {
+      float l[3], h[3];
+      for (int a = 0; a < 3; ++a)
+        l[a] = __shfl_down_sync(0xffffffffu, x.lo[a], off), h[a] = __shfl_down_sync(0xffffffffu, x.hi[a], off);
+      grow(x, l, h);
+    }
+  };
+  combine(b, 32);
+  if ((t & 31) == 0) part[t / 32] = b;
   __syncthreads();
+  if (t >= 32) return;
+  constexpr int WARPS = BOUNDS_THREADS / 32;
+  Box all = t < WARPS ? part[t] : empty_box();
+  combine(all, WARPS);
   if (t != 0) return;
-  Box all = empty_box();
-  for (int k = 0; k < BOUNDS_THREADS; ++k) grow(all, part[k].lo, part[k].hi);
   const size_t at = w[4];
   for (int a = 0; a < 3; ++a) w[at + a] = __float_as_uint(all.lo[a]), w[at + 4 + a] = __float_as_uint(all.hi[a]);
 }
 
-// The top level's nodes grouped by height above the instances (height 1 first).
-void top_levels(const std::vector<uint32_t>& nodes, std::vector<uint32_t>& order, std::vector<uint32_t>& start) {
+// Parents and inner child counts of the top level's nodes reachable from the root (the reserve may
+// hold unused space: NEVER); false when a node names a child outside it.
+bool top_links(const std::vector<uint32_t>& nodes, std::vector<uint32_t>& parent, std::vector<uint8_t>& inner) {
   const size_t nn = nodes.size() / TOP_WORDS;
-  std::vector<uint32_t> height(nn, 0);
-  for (size_t i = nn; i-- > 0;) {  // children follow their parents
-    uint32_t h = 1;
+  parent.assign(nn, EMPTY);
+  inner.assign(nn, NEVER);
+  if (nn == 0) return true;
+  inner[0] = 0;
+  for (size_t i = 0; i < nn; ++i) {  // children follow their parents
+    if (inner[i] == NEVER) continue;
     for (int c = 0; c < 4; ++c) {
       const uint32_t id = nodes[i * TOP_WORDS + 24 + c];
-      if (id != EMPTY && !(id & LEAF) && id < nn) h = std::max(h, height[id] + 1);
-    }
-    height[i] = h;
-  }
-  // only the nodes reachable from the root (the reserve may hold unused space)
-  std::vector<uint8_t> live(nn, 0);
-  std::vector<uint32_t> stack{0};
-  while (!stack.empty()) {
-    const uint32_t i = stack.back();
-    stack.pop_back();
-    if (i >= nn || live[i]) continue;
-    live[i] = 1;
-    for (int c = 0; c < 4; ++c) {
-      const uint32_t id = nodes[(size_t)i * TOP_WORDS + 24 + c];
-      if (id != EMPTY && !(id & LEAF)) stack.push_back(id);
+      if (id == EMPTY || (id & LEAF)) continue;
+      if (id >= nn || id <= i) return false;
+      parent[id] = (uint32_t)i, inner[id] = 0, ++inner[i];
     }
   }
-  const uint32_t top = nn ? height[0] : 0;
-  order.clear();
-  start.assign(1, 0);
-  for (uint32_t h = 1; h <= top; ++h) {
-    for (size_t i = 0; i < nn; ++i)
-      if (live[i] && height[i] == h) order.push_back((uint32_t)i);
-    start.push_back((uint32_t)order.size());
-  }
+  return true;
 }
 
 }  // namespace
@@ -176,27 +208,21 @@ extern "C" rt_status rt_scene_move_instances(rt_ctx* ctx, rt_scene* scene, const
   const uint32_t layout = scene->layout;
   std::lock_guard<std::mutex> lock(ctx->mu);
   RT_CUDA(ctx, cudaSetDevice(ctx->device));
-  uint32_t head[8];
-  RT_CUDA(ctx, cudaMemcpy(head, scene->d_words, sizeof head, cudaMemcpyDeviceToHost));
+  const uint32_t* head = scene->head;
   const uint32_t count = head[0];
   if (n != count || (layout == 0 && head[4] > count))  // GI word 4: a see-through tail
     return fail(ctx, RT_ERR_INVALID_ARG, "moved instances must be the scene's %u instances, in record order", count);
-  std::vector<Moved> moved(n);
-  std::vector<rtb::Placement> placed(n);
   for (uint32_t i = 0; i < n; ++i) {
     const rt_instance& s = instances[i];
-    std::copy(s.model, s.model + 12, moved[i].model);
-    std::copy(s.rows, s.rows + 12, moved[i].rows);
-    moved[i].mesh = s.mesh;
-    std::copy(s.model, s.model + 12, placed[i].model);
-    std::copy(s.rows, s.rows + 12, placed[i].rows);
-    placed[i].mesh = s.mesh;
+    rtb::Placement p;
+    std::copy(s.model, s.model + 12, p.model);
+    std::copy(s.rows, s.rows + 12, p.rows);
     if (s.mesh >= n_meshes) return fail(ctx, RT_ERR_INVALID_ARG, "instance %u: mesh %u of %u", i, s.mesh, n_meshes);
-    if (rtb::is_singular(placed[i])) return fail(ctx, RT_ERR_LAYOUT, "instance %u: singular placement", i);
+    if (rtb::is_singular(p)) return fail(ctx, RT_ERR_LAYOUT, "instance %u: singular placement", i);
   }
   if (n == 0) return RT_OK;
   scene->w8_top_valid = false;  // the instances move: the packed top level until re-prepared
-  const size_t need = sizeof(Moved) * n + 24 * (size_t)n_meshes;
+  const size_t need = sizeof(rt_instance) * n + 24 * (size_t)n_meshes;
   if (need > scene->move_bytes) {
     RT_CUDA(ctx, cudaFree(scene->d_move));
     scene->d_move = nullptr;
@@ -212,68 +238,62 @@ extern "C" rt_status rt_scene_move_instances(rt_ctx* ctx, rt_scene* scene, const
     ctx->scene_bytes += need;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  Moved* d_moved = static_cast<Moved*>(scene->d_move);
+  rt_instance* d_moved = static_cast<rt_instance*>(scene->d_move);
   float* d_boxes = reinterpret_cast<float*>(d_moved + n);
-  RT_CUDA(ctx, cudaMemcpyAsync(d_moved, moved.data(), sizeof(Moved) * n, cudaMemcpyHostToDevice, s));
-  RT_CUDA(ctx, cudaMemcpyAsync(d_boxes, mesh_boxes, 24 * (size_t)n_meshes, cudaMemcpyHostToDevice, s));
-  k_move_records<<<(n + 127) / 128, 128, 0, s>>>(scene->d_words, layout, d_moved, n, d_boxes);
-  RT_CUDA(ctx, cudaGetLastError());
   const size_t base = layout == 0 ? head[1] : (head[1] & ~3u);
-  if (head[1] != 0 && count >= 2) {
-    const size_t span = rtb::tlas_reserve(count);
-    if (base + span > scene->n_words) return fail(ctx, RT_ERR_LAYOUT, "top level exceeds the scene's words");
-    uint32_t refits = head[3];
-    std::vector<uint32_t> nodes;
-    if (refits >= rtb::TLAS_REFITS) {
-      // Rebuilt on the device from the records' new boxes (instance_bvh::place for a moved set),
-      // with the new tree's refit order.
-      RT_CUDA(ctx, cudaFree(scene->d_top_order));
-      scene->d_top_order = nullptr;
-      scene->top_order.clear();
-      if (cudaMalloc(&scene->d_top_order, 4 * (size_t)n) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(ctx, RT_ERR_OOM, "top-level order");
-      }
+  const bool top = head[1] != 0 && count >= 2, rebuild = top && head[3] >= rtb::TLAS_REFITS;
+  const size_t span = top ? rtb::tlas_reserve(count) : 0;
+  if (top && base + span > scene->n_words) return fail(ctx, RT_ERR_LAYOUT, "top level exceeds the scene's words");
+  if (layout == 1 && (size_t)head[4] + 8 > scene->n_words) return fail(ctx, RT_ERR_LAYOUT, "scene bounds exceed the words");
+  const uint32_t refits = !top ? head[3] : (rebuild ? 0u : head[3] + 1);
+  // one copy, from pageable memory of the scene's own: it is staged before the call returns, whatever
+  // memory the caller's arrays are in
+  scene->move_stage.resize(need);
+  std::memcpy(scene->move_stage.data(), instances, sizeof(rt_instance) * n);
+  if (n_meshes) std::memcpy(scene->move_stage.data() + sizeof(rt_instance) * n, mesh_boxes, 24 * (size_t)n_meshes);
+  RT_CUDA(ctx, cudaMemcpyAsync(d_moved, scene->move_stage.data(), need, cudaMemcpyHostToDevice, s));
+  k_move_records<<<(n + 127) / 128, 128, 0, s>>>(scene->d_words, layout, d_moved, n, d_boxes, refits);
+  RT_CUDA(ctx, cudaGetLastError());
+  scene->head[3] = refits;
+  if (top) {
+    // per node: its parent, a counter, and (bytes) its inner children; span / TOP_WORDS nodes at most
+    const size_t cap = span / TOP_WORDS;
+    if (!scene->d_top_tree && cudaMalloc(&scene->d_top_tree, 9 * cap) != cudaSuccess) {
+      cudaGetLastError();
+      scene->d_top_tree = nullptr;
+      return fail(ctx, RT_ERR_OOM, "top-level links");
+    }
+    uint32_t *parent = scene->d_top_tree, *done = parent + cap;
+    uint8_t* inner = reinterpret_cast<uint8_t*>(done + cap);
+    if (rebuild) {
+      // Rebuilt on the device from the records' new boxes (instance_bvh::place for a moved set).
       const size_t header = layout == 0 ? 16 : 8, stride = layout == 0 ? 32 : 24;
       uint32_t n_nodes = 0;
-      std::vector<uint32_t> starts;
+      scene->top_nodes = 0;
       const rt_status st = tlas_build_device(ctx, scene->d_words + header + 12, stride, n, true, scene->d_words + base, span,
-                                             scene->d_top_order, &starts, &n_nodes, s);
+                                             &n_nodes, s);
       if (st != RT_OK) return st;
-      scene->top_order.resize(n_nodes);
-      RT_CUDA(ctx, cudaMemcpy(scene->top_order.data(), scene->d_top_order, 4 * (size_t)n_nodes, cudaMemcpyDeviceToHost));
-      scene->top_level_start = starts;
-      refits = 0;
+      k_top_links<<<(n_nodes + 127) / 128, 128, 0, s>>>(scene->d_words + base, n_nodes, parent, inner);
+      RT_CUDA(ctx, cudaGetLastError());
+      scene->top_nodes = n_nodes;
     } else {
-      if (scene->top_order.empty()) {  // the tree's topology, once (and after every rebuild)
-        nodes.resize(span);
+      if (scene->top_nodes == 0) {  // the tree's topology, once (a rebuild keeps its own)
+        std::vector<uint32_t> nodes(span), up;
+        std::vector<uint8_t> kids;
         RT_CUDA(ctx, cudaMemcpyAsync(nodes.data(), scene->d_words + base, 4 * span, cudaMemcpyDeviceToHost, s));
         RT_CUDA(ctx, cudaStreamSynchronize(s));
-        top_levels(nodes, scene->top_order, scene->top_level_start);
-        RT_CUDA(ctx, cudaFree(scene->d_top_order));
-        scene->d_top_order = nullptr;
-        if (cudaMalloc(&scene->d_top_order, 4 * std::max<size_t>(1, scene->top_order.size())) != cudaSuccess) {
-          cudaGetLastError();
-          scene->top_order.clear();
-          return fail(ctx, RT_ERR_OOM, "top-level order");
-        }
-        RT_CUDA(ctx, cudaMemcpy(scene->d_top_order, scene->top_order.data(), 4 * scene->top_order.size(),
-                                cudaMemcpyHostToDevice));
+        if (!top_links(nodes, up, kids)) return fail(ctx, RT_ERR_LAYOUT, "move: top-level children out of order");
+        RT_CUDA(ctx, cudaMemcpy(parent, up.data(), 4 * up.size(), cudaMemcpyHostToDevice));
+        RT_CUDA(ctx, cudaMemcpy(inner, kids.data(), kids.size(), cudaMemcpyHostToDevice));
+        scene->top_nodes = (uint32_t)up.size();
       }
-      const std::vector<uint32_t>& st = scene->top_level_start;
-      for (size_t h = 0; h + 1 < st.size(); ++h) {
-        const uint32_t first = st[h], cnt = st[h + 1] - st[h];
-        if (!cnt) continue;
-        k_refit_top<<<(cnt + 127) / 128, 128, 0, s>>>(scene->d_words, layout, base, scene->d_top_order, first, cnt);
-        RT_CUDA(ctx, cudaGetLastError());
-      }
-      refits += 1;
+      RT_CUDA(ctx, cudaMemsetAsync(done, 0, 4 * cap, s));
+      k_refit_top<<<(4 * scene->top_nodes + TOP_BLOCK - 1) / TOP_BLOCK, TOP_BLOCK, 0, s>>>(
+          scene->d_words, layout, base, scene->top_nodes, parent, inner, done);
+      RT_CUDA(ctx, cudaGetLastError());
     }
-    RT_CUDA(ctx, cudaMemcpyAsync(scene->d_words + 3, &refits, 4, cudaMemcpyHostToDevice, s));
-    RT_CUDA(ctx, cudaStreamSynchronize(s));  // `refits` is a local
   }
   if (layout == 1) {
-    if ((size_t)head[4] + 8 > scene->n_words) return fail(ctx, RT_ERR_LAYOUT, "scene bounds exceed the words");
     k_scene_bounds<<<1, BOUNDS_THREADS, 0, s>>>(scene->d_words, n);
     RT_CUDA(ctx, cudaGetLastError());
   }

@@ -171,8 +171,10 @@ bool same_instances(uint32_t layout, const uint32_t* a, const uint32_t* b) {
   return true;
 }
 
-// The host's copy of the records' BLAS words, after an upload or a rewrite of the records.
-void keep_blas_words(rt_scene* s, const uint32_t* words) {
+// The host's copies of the header and of the records' BLAS words, after an upload or a rewrite of
+// the records.
+void keep_records(rt_scene* s, const uint32_t* words, size_t n_words) {
+  std::copy_n(words, std::min<size_t>(n_words, 8), s->head);
   const size_t header = s->layout == 0 ? 16 : 8, stride = s->layout == 0 ? 32 : 24;
   s->blas_words.resize(6 * (size_t)s->info.instances);
   for (uint32_t i = 0; i < s->info.instances; ++i)
@@ -287,7 +289,7 @@ rt_status rt_scene_upload(rt_ctx* ctx, rt_layout layout, const uint32_t* words, 
     cudaFree(s->d_words);
     return fail(ctx, RT_ERR_CUDA, "scene copy: %s", cudaGetErrorString(e));
   }
-  keep_blas_words(s.get(), words);
+  keep_records(s.get(), words, n_words);
   ctx->scene_bytes += s->device_bytes;
   *out = s.release();
   return RT_OK;
@@ -319,6 +321,13 @@ rt_status rt_scene_update_records(rt_ctx* ctx, rt_scene* scene, const uint32_t* 
   const size_t header = scene->layout == 0 ? 16 : 8, stride = scene->layout == 0 ? 32 : 24;
   const uint32_t most = std::max(all.empty() ? 0u : all[0], n_words ? words[0] : 0u);
   const std::vector<uint32_t> before(all.begin(), all.begin() + std::min(all.size(), header + stride * (size_t)most));
+  // another top level voids the links that rt_scene_move_instances keeps
+  bool same_top = scene->top_nodes != 0 && std::equal(words, words + std::min<size_t>(n_words, 3), all.begin());
+  if (same_top) {
+    const size_t base = scene->layout == 0 ? all[1] : (all[1] & ~3u);
+    for (size_t i = 0; i < scene->top_nodes && same_top; ++i)
+      for (size_t k = base + 32 * i + 24; k < base + 32 * i + 28 && k < n_words; ++k) same_top &= words[k] == all[k];
+  }
   std::copy(words, words + n_words, all.begin());
   rtb::SceneInfo info;
   std::string err;
@@ -327,8 +336,12 @@ rt_status rt_scene_update_records(rt_ctx* ctx, rt_scene* scene, const uint32_t* 
   // records that name other BLASes, or another instance count, void the 8-wide instance table
   if (scene->d_wide8 && !same_instances(scene->layout, before.data(), all.data())) drop_wide8(ctx, scene);
   RT_CUDA(ctx, cudaMemcpy(scene->d_words, words, n_words * 4, cudaMemcpyHostToDevice));
+  if (!same_top) {
+    cudaFree(scene->d_top_tree);
+    scene->d_top_tree = nullptr, scene->top_nodes = 0;
+  }
   scene->info = info;
-  keep_blas_words(scene, all.data());
+  keep_records(scene, all.data(), all.size());
   scene->w8_top_valid = false;  // the instances' boxes may have moved: the packed top level until re-prepared
   return RT_OK;
 }
@@ -524,7 +537,7 @@ rt_status rt_scene_release(rt_ctx* ctx, rt_scene* scene) {
   cudaFree(scene->d_wide8);
   cudaFree(scene->d_w8_top);
   cudaFree(scene->d_move);
-  cudaFree(scene->d_top_order);
+  cudaFree(scene->d_top_tree);
   for (auto& kv : scene->refit) cudaFree(kv.second.d_tree);
   ctx->scene_bytes -= scene->device_bytes;
   delete scene;

@@ -360,7 +360,7 @@ __global__ void k_ids(const Seg* __restrict__ segs, const uint32_t* __restrict__
 // or a node id), EMPTY for an unused slot, whose box words stay 0.
 __global__ void k_words(const Seg* __restrict__ segs, const uint32_t* __restrict__ list, uint32_t first, uint32_t count,
                         const uint32_t* __restrict__ kids, const uint32_t* __restrict__ id, const uint32_t* __restrict__ ids,
-                        const float* __restrict__ sbox, uint32_t* __restrict__ out, uint32_t* __restrict__ order_at) {
+                        const float* __restrict__ sbox, uint32_t* __restrict__ out) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const uint32_t x = list[first + i];
@@ -375,7 +375,6 @@ __global__ void k_words(const Seg* __restrict__ segs, const uint32_t* __restrict
     for (int a = 0; a < 3; ++a) w[4 * a + c] = __float_as_uint(bx[a]), w[12 + 4 * a + c] = __float_as_uint(bx[3 + a]);
     w[24 + c] = inner(segs, k) ? id[k] : (LEAF | ids[segs[k].b]);
   }
-  if (order_at) order_at[i] = id[x];
 }
 
 class Scratch {
@@ -410,7 +409,7 @@ inline uint32_t grid(size_t n, uint32_t t) { return (uint32_t)((n + t - 1) / t);
 namespace rtc {
 
 rt_status tlas_build_device(rt_ctx* ctx, const uint32_t* d_box_words, size_t stride, uint32_t n, bool sah, uint32_t* d_out,
-                            size_t cap_words, uint32_t* d_order, std::vector<uint32_t>* level_start, uint32_t* n_nodes,
+                            size_t cap_words, uint32_t* n_nodes,
                             cudaStream_t st) {
   if (n < 2) return fail(ctx, RT_ERR_INVALID_ARG, "a top level needs two instances");
   if ((size_t)n - 1 > cap_words / NODE_WORDS) return fail(ctx, RT_ERR_INVALID_ARG, "top-level words too small");
@@ -547,18 +546,12 @@ rt_status tlas_build_device(rt_ctx* ctx, const uint32_t* d_box_words, size_t str
   for (size_t l = 0; l < levels4; ++l)
     k_ids<<<grid(wide[l + 1] - wide[l], 128), 128, 0, st>>>(d_segs, d_list, wide[l], wide[l + 1] - wide[l], d_kids, d_size, d_id);
   RT_CUDA(ctx, cudaMemsetAsync(d_out, 0, 4 * cap_words, st));
-  // The node ids a level, deepest level first in `d_order` (a bottom-up refit order).
-  std::vector<uint32_t> starts(1, 0);
-  for (size_t l = levels4; l-- > 0;) starts.push_back(starts.back() + (wide[l + 1] - wide[l]));
   for (size_t l = 0; l < levels4; ++l) {
     const uint32_t first = wide[l], count = wide[l + 1] - wide[l];
-    const size_t at = starts[levels4 - 1 - l];
-    k_words<<<grid(count, 128), 128, 0, st>>>(d_segs, d_list, first, count, d_kids, d_id, d_ids, d_sbox, d_out,
-                                               d_order ? d_order + at : nullptr);
+    k_words<<<grid(count, 128), 128, 0, st>>>(d_segs, d_list, first, count, d_kids, d_id, d_ids, d_sbox, d_out);
   }
   RT_CUDA(ctx, cudaGetLastError());
   RT_CUDA(ctx, cudaStreamSynchronize(st));
-  if (level_start) *level_start = starts;
   if (n_nodes) *n_nodes = nodes;
   return RT_OK;
 }
@@ -593,7 +586,7 @@ rt_status rt_tlas_build_device(rt_ctx* ctx, const float* boxes, uint32_t n, int 
   uint32_t* d_out = d + 6 * (size_t)n;
   RT_CUDA(ctx, cudaMemcpyAsync(d_boxes, boxes, 24 * (size_t)n, cudaMemcpyHostToDevice, st));
   uint32_t nodes = 0;
-  rt_status s = rtc::tlas_build_device(ctx, d_boxes, 6, n, sah != 0, d_out, cap, nullptr, nullptr, &nodes, st);
+  rt_status s = rtc::tlas_build_device(ctx, d_boxes, 6, n, sah != 0, d_out, cap, &nodes, st);
   if (s != RT_OK) return s;
   const size_t words = (size_t)nodes * NODE_WORDS;
   if (!out) {
