@@ -291,30 +291,42 @@ class Blas:
         self.positions = p
 
 
+# rt_instance as a numpy record: the whole array is filled a field at a time
+_INSTANCE_DTYPE = np.dtype([("model", np.float32, 12), ("rows", np.float32, 12), ("mesh", np.uint32), ("slot", np.uint32),
+                            ("casts_shadow", np.uint32), ("near_base", np.uint32), ("extra", np.uint32, 8)])
+
+
+def _words32(values, n: int) -> np.ndarray:
+    """The first n values (of any numeric type, truncated) as 32-bit words, as ctypes stores them."""
+    v = np.asarray(values)[:n]
+    if len(v) < n:
+        raise IndexError(f"{len(v)} values for {n} instances")
+    if v.dtype.kind == "f" and not np.isfinite(v).all():
+        raise ValueError("an instance field is not finite")
+    return v if v.dtype == np.uint32 else (v.astype(np.int64) & 0xFFFFFFFF).astype(np.uint32)
+
+
 def _instance_array(layout: int, instances):
     """rt_instance records for an Instances-like object (see pack_scene)."""
     n = len(instances.mesh)
-    arr = (RtInstance * max(n, 1))()
-    model = np.ascontiguousarray(instances.model, np.float32).reshape(n, 12)
-    rows = np.ascontiguousarray(instances.rows, np.float32).reshape(n, 12)
+    rec = np.zeros(max(n, 1), _INSTANCE_DTYPE)
+    rec["model"][:n] = np.ascontiguousarray(instances.model, np.float32).reshape(n, 12)
+    rec["rows"][:n] = np.ascontiguousarray(instances.rows, np.float32).reshape(n, 12)
     casts = getattr(instances, "casts", None)
     slot = getattr(instances, "slot", None)
     near = getattr(instances, "near_base", None)
     extra = getattr(instances, "extra", None)
-    for i in range(n):
-        rec = arr[i]
-        ctypes.memmove(rec.model, model[i].ctypes.data, 48)
-        ctypes.memmove(rec.rows, rows[i].ctypes.data, 48)
-        rec.mesh = int(instances.mesh[i])
-        rec.slot = int(slot[i]) if slot is not None else i
-        rec.casts_shadow = int(bool(casts[i])) if casts is not None else 1
-        rec.near_base = int(near[i]) if near is not None else 0
-        if extra is not None:
-            for k in range(8):
-                rec.extra[k] = int(extra[i][k])
-        elif casts is not None and layout == LAYOUT_GI:
-            rec.extra[3] = 0 if casts[i] else 1
-    return arr, n
+    rec["mesh"][:n] = _words32(instances.mesh, n)
+    rec["slot"][:n] = np.arange(n) if slot is None else _words32(slot, n)
+    rec["casts_shadow"][:n] = 1 if casts is None else _words32(np.asarray(casts).astype(bool), n)
+    if near is not None:
+        rec["near_base"][:n] = _words32(near, n)
+    if extra is not None:
+        if n:
+            rec["extra"][:n] = np.stack([_words32(extra, n)[:, k] for k in range(8)], axis=1)
+    elif casts is not None and layout == LAYOUT_GI:
+        rec["extra"][:n, 3] = 1 - rec["casts_shadow"][:n]
+    return (RtInstance * len(rec)).from_buffer(rec), n
 
 
 def pack_scene(layout: int, meshes, instances, tlas_mode: int = -1, primitives=None) -> np.ndarray:
