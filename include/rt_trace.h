@@ -189,6 +189,21 @@ rt_status rt_trace(rt_ctx* ctx, const rt_scene* scene, rt_mode mode, const rt_ra
 rt_status rt_trace_ex(rt_ctx* ctx, const rt_scene* scene, rt_mode mode, rt_kernel kernel,
                       const rt_ray* d_rays, const uint32_t* d_order, void* d_hits, uint32_t n,
                       void* stream);
+/* The seam's own argument form: origins, directions and ranges in arrays of their own (gi_closest,
+ * gi_visible and rs_trace take them so, gi_rays_software.wgsl:280-291), traced by RT_KERNEL_PLAIN
+ * without a ray buffer in between. d_out receives rt_trace's hit records (closest) or one byte a ray
+ * (any hit): 1 when something blocks it, or with `clear` nonzero 1 when nothing does. GI and
+ * reflection layouts. Asynchronous on `stream`; allocates nothing. */
+typedef struct rt_split_rays {
+  const float* d_o;    /* origin of ray i at d_o[i * o_stride] */
+  const float* d_d;    /* direction of ray i at d_d[i * d_stride] */
+  const float* d_tmin; /* one a ray, or NULL: `tmin` for all */
+  const float* d_tmax; /* one a ray, or NULL: `tmax` for all */
+  float tmin, tmax;
+  uint32_t o_stride, d_stride; /* in floats */
+} rt_split_rays;
+rt_status rt_trace_split(rt_ctx* ctx, const rt_scene* scene, rt_mode mode, const rt_split_rays* rays, uint32_t n,
+                         void* d_out, int clear, void* stream);
 /* Ray order keys for rt_order_rays. */
 typedef enum rt_ray_order {
   RT_ORDER_NONE = 0,

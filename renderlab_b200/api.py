@@ -57,6 +57,12 @@ class RtInstance(ctypes.Structure):
                 ("extra", ctypes.c_uint32 * 8)]
 
 
+class RtSplitRays(ctypes.Structure):
+    _fields_ = [("d_o", ctypes.c_void_p), ("d_d", ctypes.c_void_p), ("d_tmin", ctypes.c_void_p), ("d_tmax", ctypes.c_void_p),
+                ("tmin", ctypes.c_float), ("tmax", ctypes.c_float), ("o_stride", ctypes.c_uint32),
+                ("d_stride", ctypes.c_uint32)]
+
+
 class RtBatch(ctypes.Structure):
     _fields_ = [("d_rays", ctypes.c_void_p), ("d_hits", ctypes.c_void_p), ("n", ctypes.c_uint32), ("mode", ctypes.c_int)]
 
@@ -100,7 +106,7 @@ class RtTuning(ctypes.Structure):
 EXPORTS = ("rt_abi_version", "rt_ctx_create", "rt_ctx_destroy", "rt_get_last_error", "rt_get_stats",
            "rt_ctx_set_tuning", "rt_ctx_get_tuning",
            "rt_selftest", "rt_scene_upload", "rt_scene_update_records", "rt_scene_release",
-           "rt_scene_device_bytes", "rt_scene_validate", "rt_scene_prepare", "rt_trace", "rt_trace_ex", "rt_trace_host", "rt_trace_host_batches", "rt_ctx_reserve", "rt_trace_counted", "rt_order_rays",
+           "rt_scene_device_bytes", "rt_scene_validate", "rt_scene_prepare", "rt_trace", "rt_trace_ex", "rt_trace_split", "rt_trace_host", "rt_trace_host_batches", "rt_ctx_reserve", "rt_trace_counted", "rt_order_rays",
            "rt_trace_batches", "rt_plan_create", "rt_plan_launch", "rt_plan_info", "rt_plan_destroy",
            "rt_scene_refit", "rt_scene_read_words", "rt_scene_tune_top", "rt_gi_cell_rays", "rt_trace_gi_cells", "rt_trace_gi_lights", "rt_server_create", "rt_server_add_scene", "rt_server_remove_scene", "rt_server_submit",
            "rt_server_wait", "rt_server_get_stats", "rt_server_fail_next", "rt_server_destroy",
@@ -149,6 +155,7 @@ def lib() -> ctypes.CDLL:
     L.rt_scene_device_bytes.restype = ctypes.c_size_t
     L.rt_trace.argtypes = [_vp, _vp, ctypes.c_int, _vp, _vp, ctypes.c_uint32, _vp]
     L.rt_trace_ex.argtypes = [_vp, _vp, ctypes.c_int, ctypes.c_int, _vp, _vp, _vp, ctypes.c_uint32, _vp]
+    L.rt_trace_split.argtypes = [_vp, _vp, ctypes.c_int, ctypes.POINTER(RtSplitRays), ctypes.c_uint32, _vp, ctypes.c_int, _vp]
     L.rt_trace_host.argtypes = [_vp, _vp, ctypes.c_int, ctypes.c_int, _vp, _vp, ctypes.c_uint32]
     L.rt_trace_host_batches.argtypes = [_vp, _vp, ctypes.POINTER(RtHostBatch), ctypes.c_uint32]
     L.rt_ctx_reserve.argtypes = [_vp, ctypes.c_uint32]
@@ -879,6 +886,53 @@ def _rays(origin, direction, tmin, tmax):
     return r
 
 
+def _seam(engine: Engine, scene: Scene, origin, direction, tmin, tmax, mode: int, clear: bool):
+    """The call as one launch over the caller's own arrays (rt_trace_split): hit words, or for an
+    any-hit mode a bool tensor of blocked (clear: unblocked) rays. None unless the scene has a BVH4
+    layout and the arrays are rows of float32 on one CUDA device, the ranges one value or one a ray."""
+    import torch
+    if scene.layout not in (LAYOUT_GI, LAYOUT_REFLECTION):
+        return None
+    for x in (origin, direction):
+        if type(x) is not torch.Tensor or not x.is_cuda or x.dtype != torch.float32 or x.dim() != 2 or x.shape[1] != 3:
+            return None
+    n, device = origin.shape[0], origin.device
+    strides = origin.stride(), direction.stride()
+    if n == 0 or direction.shape[0] != n or direction.device != device:
+        return None
+    if any(inner != 1 or not 3 <= row < 1 << 32 for row, inner in strides):
+        return None
+    ranges = []
+    for x in (tmin, tmax):
+        if type(x) is float or type(x) is int:
+            if not abs(x) <= 3.0e38:
+                return None
+            ranges.append((None, x))
+        elif (type(x) is torch.Tensor and x.is_cuda and x.dtype == torch.float32 and x.dim() == 1 and x.shape[0] == n
+              and x.device == device and x.is_contiguous()):
+            ranges.append((x.data_ptr(), 0.0))
+        else:
+            return None
+    words = hit_words(scene.layout, mode)
+    hits = (torch.empty((n, words), dtype=torch.int32, device=device) if mode == CLOSEST
+            else torch.empty(n, dtype=torch.bool, device=device))
+    rays = RtSplitRays(origin.data_ptr(), direction.data_ptr(), ranges[0][0], ranges[1][0], ranges[0][1], ranges[1][1],
+                       strides[0][0], strides[1][0])
+    engine._check(lib().rt_trace_split(engine.ctx, scene.handle, mode, ctypes.byref(rays), n, hits.data_ptr(), int(clear),
+                                       torch.cuda.current_stream(device).cuda_stream))
+    return hits
+
+
+def _trace_seam(engine: Engine, scene: Scene, origin, direction, tmin, tmax, mode: int, kernel: str, clear: bool = False):
+    """A seam call: as one launch where it can be, else through a ray buffer."""
+    hits = _seam(engine, scene, origin, direction, tmin, tmax, mode, clear) if kernel == "plain" else None
+    if hits is None:
+        hits = engine.trace(scene, _rays(origin, direction, tmin, tmax), mode, kernel)
+        if mode != CLOSEST:
+            hits = hits == 0 if clear else hits != 0
+    return hits
+
+
 def decode_gi(hits) -> dict:
     """Split (n, 10) GI hit words into named fields (torch int32 tensor or numpy)."""
     h = hits
@@ -888,25 +942,25 @@ def decode_gi(hits) -> dict:
 
 def gi_closest(engine: Engine, scene: Scene, origin, direction, tmin, tmax, kernel="plain") -> dict:
     """gi_closest (gi_rays_software.wgsl:280-282) for a batch of rays on the device."""
-    return decode_gi(engine.trace(scene, _rays(origin, direction, tmin, tmax), CLOSEST, kernel))
+    return decode_gi(_trace_seam(engine, scene, origin, direction, tmin, tmax, CLOSEST, kernel))
 
 
 def gi_visible(engine: Engine, scene: Scene, origin, direction, kernel="plain"):
     """gi_visible (gi_rays_software.wgsl:285-287): sky visibility along [0, 1e20)."""
-    return engine.trace(scene, _rays(origin, direction, 0.0, 1e20), ANY_SKY, kernel) == 0
+    return _trace_seam(engine, scene, origin, direction, 0.0, 1e20, ANY_SKY, kernel, clear=True)
 
 
 def gi_visible_within(engine: Engine, scene: Scene, origin, direction, tmax, kernel="plain"):
     """gi_visible_within (gi_rays_software.wgsl:289-291): opaque casters within tmax."""
-    return engine.trace(scene, _rays(origin, direction, 0.0, tmax), ANY_CASTERS, kernel) == 0
+    return _trace_seam(engine, scene, origin, direction, 0.0, tmax, ANY_CASTERS, kernel, clear=True)
 
 
 def rs_trace(engine: Engine, scene: Scene, origin, direction, tmin, tmax, any_hit=False, kernel="plain"):
     """rs_trace (reflections_software_bvh4.wgsl:140): (t, record) or the blocked flags."""
     import torch
-    h = engine.trace(scene, _rays(origin, direction, tmin, tmax), ANY_CASTERS if any_hit else CLOSEST, kernel)
+    h = _trace_seam(engine, scene, origin, direction, tmin, tmax, ANY_CASTERS if any_hit else CLOSEST, kernel)
     if any_hit:
-        return h != 0
+        return h
     return h[:, 0].view(torch.float32), h[:, 1:5]
 
 

@@ -229,6 +229,32 @@ RT_DEV void put_flag(const Src& s, uint32_t entry, uint32_t id, const Ray&, bool
   reinterpret_cast<uint32_t*>(out_of(s, entry))[id] = blocked ? 1u : 0u;
 }
 
+// Rays whose parts lie in arrays of their own, as a caller of the seam's functions holds them: origin
+// and direction in rows of `o_stride` and `d_stride` floats, tmin and tmax an array or one value. Any
+// hit: a byte a ray, 1 when it is blocked, or with `clear` 1 when it is not.
+struct SplitRays {
+  const float* o;
+  const float* d;
+  const float* tmin;  // null: tmin_all
+  const float* tmax;  // null: tmax_all
+  float tmin_all, tmax_all;
+  uint32_t o_stride, d_stride;
+  void* out;
+  uint32_t clear;
+};
+template <bool CS = false, class Lane>
+RT_DEV Ray fetch(const SplitRays& s, uint32_t id, Lane& L) {
+  L.ray_id = id;
+  L.entry = 0;
+  const float *o = s.o + (size_t)s.o_stride * id, *d = s.d + (size_t)s.d_stride * id;
+  return Ray{{__ldg(o), __ldg(o + 1), __ldg(o + 2)}, s.tmin ? __ldg(s.tmin + id) : s.tmin_all,
+             {__ldg(d), __ldg(d + 1), __ldg(d + 2)}, s.tmax ? __ldg(s.tmax + id) : s.tmax_all};
+}
+RT_DEV void* out_of(const SplitRays& s, uint32_t) { return s.out; }
+RT_DEV void put_flag(const SplitRays& s, uint32_t, uint32_t id, const Ray&, bool blocked) {
+  reinterpret_cast<uint8_t*>(s.out)[id] = blocked != (s.clear != 0) ? 1 : 0;
+}
+
 // Device-side counters every traversal kernel may bump (rare events only).
 struct DevStatus {
   unsigned long long stack_drops;

@@ -31,6 +31,9 @@ struct SceneView {
 // PLAIN: mode 0 closest, 1/2 any-hit. Hits as documented in rt_trace.h.
 cudaError_t launch_plain(const SceneView& s, uint32_t mode, const float4* rays, void* hits, uint32_t n,
                          rtk::DevStatus* st, cudaStream_t stream);
+// PLAIN over rays in separate arrays (layouts 0 and 1).
+cudaError_t launch_plain_split(const SceneView& s, uint32_t mode, const rtk::SplitRays& src, uint32_t n, rtk::DevStatus* st,
+                               cudaStream_t stream);
 // FAST: bit-exact with PLAIN; `order` (optional) permutes which ray each thread traces.
 // `counter` is a device word the launch owns until it completes (zeroed on `stream`).
 cudaError_t launch_fast(const SceneView& s, uint32_t mode, const float4* rays, const uint32_t* order, void* hits,

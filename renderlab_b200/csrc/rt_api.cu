@@ -562,6 +562,27 @@ rt_status rt_trace_ex(rt_ctx* ctx, const rt_scene* scene, rt_mode mode, rt_kerne
   return dispatch(ctx, scene, mode, kernel, d_rays, d_order, d_hits, n, static_cast<cudaStream_t>(stream));
 }
 
+rt_status rt_trace_split(rt_ctx* ctx, const rt_scene* scene, rt_mode mode, const rt_split_rays* rays, uint32_t n,
+                         void* d_out, int clear, void* stream) {
+  rt_status s = check_trace_args(ctx, scene, mode, RT_KERNEL_PLAIN);
+  if (s != RT_OK) return s;
+  if (scene->layout == RT_LAYOUT_REFLECTION_BVH2)
+    return fail(ctx, RT_ERR_UNSUPPORTED, "separate ray arrays are traced over the BVH4 layouts");
+  if (n == 0) return RT_OK;
+  if (!rays || !rays->d_o || !rays->d_d || !d_out) return fail(ctx, RT_ERR_INVALID_ARG, "null ray or hit buffer");
+  for (const void* p : {(const void*)rays->d_o, (const void*)rays->d_d, (const void*)rays->d_tmin, (const void*)rays->d_tmax})
+    if (reinterpret_cast<uintptr_t>(p) % 4 != 0) return fail(ctx, RT_ERR_INVALID_ARG, "ray arrays must be 4-byte aligned");
+  if (mode == RT_CLOSEST && reinterpret_cast<uintptr_t>(d_out) % 4 != 0)
+    return fail(ctx, RT_ERR_INVALID_ARG, "hits must be 4-byte aligned");
+  const rtk::SplitRays src{rays->d_o, rays->d_d, rays->d_tmin, rays->d_tmax, rays->tmin, rays->tmax, rays->o_stride,
+                           rays->d_stride, d_out, clear ? 1u : 0u};
+  const cudaError_t e = rtl::launch_plain_split(view_of(scene), (uint32_t)mode, src, n, ctx->d_status, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return fail(ctx, RT_ERR_CUDA, "traversal launch: %s", cudaGetErrorString(e));
+  ctx->rays += n;
+  ctx->launches += 1;
+  return RT_OK;
+}
+
 rt_status rt_trace_counted(rt_ctx* ctx, const rt_scene* scene, rt_mode mode, rt_kernel kernel, const rt_ray* d_rays,
                            void* d_hits, uint32_t n, uint64_t counts[8]) {
   rt_status s = check_trace_args(ctx, scene, mode, kernel);
