@@ -119,6 +119,7 @@ constexpr size_t GI_HIT_BYTES = 40, RS_HIT_BYTES = 20, ANY_HIT_BYTES = 4, RAY_BY
 // against 752 for 2^19 (more launches, each with its tail of idle lanes and its final pass) and
 // 773 for 2^21 (eight stages of 2^20: 776).
 constexpr uint32_t HOST_CHUNK = 1u << RT_HOST_CHUNK_LOG2;
+constexpr uint32_t HOST_CHUNK_LEAST = 1u << 18;  // rays of a chunk of a smaller call
 constexpr uint32_t COUNTER_SLOTS = 4096;
 
 inline rt_status fail(rt_ctx* ctx, rt_status s, const char* fmt, ...) {
