@@ -42,9 +42,9 @@ using namespace rtq;
 constexpr uint32_t LEAF_TRIS = rtb::LEAF_TRIANGLES;     // near_field.rs:23
 constexpr uint32_t BINS = 16;                           // near_field.rs:273
 constexpr uint32_t TOO_DEEP = 2 * rtb::MAX_SAH_DEPTH;   // binary depth of node level 16
-constexpr uint32_t SMALL = 2048;          // a range of at most this many triangles splits in one block
-constexpr uint32_t SMALL_THREADS = 128;
-constexpr uint32_t CHUNK = 4096;          // triangles one block takes of a larger range
+constexpr uint32_t SMALL = 2048;          // a range of at most this many triangles is one block's, to its leaves
+constexpr uint32_t SMALL_WARPS = 8;
+constexpr uint32_t CHUNK = 1024;          // triangles one block takes of a larger range
 constexpr uint32_t CHUNK_THREADS = 256;
 constexpr uint32_t MAX_TRIANGLES = 1u << 29;
 constexpr int KIND_MEDIAN = 0, KIND_SAH = 1;
@@ -85,40 +85,64 @@ __device__ __forceinline__ float half_area(const float* lo, const float* hi) {  
 
 struct Choice {
   int kind, axis, plane;
+  uint32_t left;  // SAH: triangles left of the plane
 };
 
 // The split of one range from its centroid box and bins (near_field.rs:317-379): the cheapest
 // SAH plane, ties to the lower axis and bin, else the median on the axis of largest extent (the
-// last of equal extents). Bin boxes are order keys; an empty bin adds nothing.
+// last of equal extents). Bin boxes are order keys; an empty bin adds nothing. By one warp, a bin to
+// a lane: the boxes and counts on both sides of each plane are prefix and suffix scans, each cost is
+// made by the host's operations, and the cheapest in the host's order is kept (one thread sweeping
+// the 3 x 15 planes took 4 us a range). The same answer in every lane.
 __device__ Choice choose(const float* lo, const float* hi, const uint32_t* cnt, const uint32_t* bl,
                          const uint32_t* bh, uint32_t len, bool sah) {
+  const int lane = threadIdx.x & 31, b = lane & (BINS - 1);
   bool found = false;
   float best = 0.0f;
-  Choice c{KIND_SAH, 0, 0};
+  Choice c{KIND_SAH, 0, 0, 0};
   for (int axis = 0; sah && axis < 3; ++axis) {
     const float extent = __fsub_rn(hi[axis], lo[axis]);
     if (!(extent > 0.0f)) continue;
-    const uint32_t* n = cnt + axis * BINS;
-    const uint32_t* l = bl + axis * BINS * 3;
-    const uint32_t* h = bh + axis * BINS * 3;
-    float right[BINS];
-    float al[3] = {INFINITY, INFINITY, INFINITY}, ah[3] = {-INFINITY, -INFINITY, -INFINITY};
-    uint32_t seen = 0;
-    for (int b = BINS - 1; b >= 1; --b) {
-      if (n[b])
-        for (int a = 0; a < 3; ++a) al[a] = lo_of(al[a], unkey(l[3 * b + a])), ah[a] = hi_of(ah[a], unkey(h[3 * b + a]));
-      seen += n[b];
-      right[b] = __fmul_rn(half_area(al, ah), (float)seen);
+    // lanes 0-15: bins from the left; lanes 16-31: bins from the right
+    const int bin = lane < (int)BINS ? b : (int)BINS - 1 - b;
+    uint32_t seen = cnt[axis * BINS + bin];
+    float al[3], ah[3];
+    for (int a = 0; a < 3; ++a) {
+      al[a] = seen ? unkey(bl[(axis * BINS + bin) * 3 + a]) : INFINITY;
+      ah[a] = seen ? unkey(bh[(axis * BINS + bin) * 3 + a]) : -INFINITY;
     }
-    for (int a = 0; a < 3; ++a) al[a] = INFINITY, ah[a] = -INFINITY;
-    seen = 0;
-    for (int b = 0; b < (int)BINS - 1; ++b) {
-      if (n[b])
-        for (int a = 0; a < 3; ++a) al[a] = lo_of(al[a], unkey(l[3 * b + a])), ah[a] = hi_of(ah[a], unkey(h[3 * b + a]));
-      seen += n[b];
-      if (seen == 0 || seen == len) continue;
-      const float cost = __fadd_rn(__fmul_rn(half_area(al, ah), (float)seen), right[b + 1]);
-      if (!found || cost < best) found = true, best = cost, c.axis = axis, c.plane = b;
+    for (int off = 1; off < (int)BINS; off *= 2) {
+      const uint32_t n = __shfl_up_sync(0xffffffffu, seen, off, BINS);
+      for (int a = 0; a < 3; ++a) {
+        const float l = __shfl_up_sync(0xffffffffu, al[a], off, BINS), h = __shfl_up_sync(0xffffffffu, ah[a], off, BINS);
+        if (b >= off) al[a] = lo_of(l, al[a]), ah[a] = hi_of(h, ah[a]);
+      }
+      if (b >= off) seen += n;
+    }
+    const float side = __fmul_rn(half_area(al, ah), (float)seen);
+    // plane b of lane b: the right side is bins b + 1 to 15, made by the lane that scanned 15 - (b + 1)
+    const float right = __shfl_sync(0xffffffffu, side, (int)BINS + ((int)BINS - 2 - b & (int)BINS - 1));
+    const float cost = __fadd_rn(side, right);
+    const unsigned valid = __ballot_sync(0xffffffffu, lane < (int)BINS - 1 && seen != 0 && seen != len);
+    if (!valid) continue;
+    // In the planes' order a cost replaces a greater one; the first of all has nothing to replace, and
+    // nothing replaces a NaN there.
+    int plane = __ffs(valid) - 1;
+    float at = __shfl_sync(0xffffffffu, cost, plane);
+    if (found || !isnan(at)) {
+      const bool real = (valid >> lane & 1u) && !isnan(cost);
+      float low = real ? cost : INFINITY;
+      for (int off = 16; off; off /= 2) {
+        const float o = __shfl_xor_sync(0xffffffffu, low, off);
+        low = o < low ? o : low;
+      }
+      const unsigned equal = __ballot_sync(0xffffffffu, real && cost == low);
+      if (!equal) continue;
+      plane = __ffs(equal) - 1, at = low;
+    }
+    if (!found || at < best) {
+      found = true, best = at, c.axis = axis, c.plane = plane;
+      c.left = __shfl_sync(0xffffffffu, seen, plane);
     }
   }
   if (found) return c;
@@ -163,8 +187,8 @@ __global__ void k_prepare(const float* __restrict__ pos, const uint32_t* __restr
   perm[t] = t;
 }
 
-// Per range of the level: pending (more than a leaf's triangles) in the low word, split by
-// several blocks in the high word; one extra zero entry so the exclusive sum ends in the totals.
+// Per range of the level, whether several blocks split it, in the low word (its place among the next
+// level's pairs) and the high word; one extra zero entry so the exclusive sum ends in the totals.
 __global__ void k_level_flags(const Seg* __restrict__ segs, uint32_t width, unsigned long long* __restrict__ flags) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i > width) return;
@@ -172,8 +196,7 @@ __global__ void k_level_flags(const Seg* __restrict__ segs, uint32_t width, unsi
     flags[i] = 0;
     return;
   }
-  const uint32_t len = segs[i].e - segs[i].b;
-  flags[i] = (unsigned long long)(len > LEAF_TRIS) | (unsigned long long)(len > SMALL) << 32;
+  flags[i] = segs[i].e - segs[i].b > SMALL ? 1ull << 32 | 1ull : 0ull;
 }
 
 __device__ __forceinline__ void write_children(Seg* segs, uint32_t lv0, uint32_t i, const Seg& g, uint32_t mid,
@@ -184,120 +207,127 @@ __device__ __forceinline__ void write_children(Seg* segs, uint32_t lv0, uint32_t
   segs[next + 2 * r + 1] = Seg{mid, g.e, g.depth + 1, own};
 }
 
-struct LevelArgs {
-  Seg* segs;
-  uint32_t lv0, width, next;  // this level's ranges: segs[lv0, lv0 + width); the next level from `next`
-  const unsigned long long* rank;
-  const float* cen;
-  const uint32_t* tbk;
-  uint32_t* perm;
-  int sah;
+// A range of at most SMALL triangles split down to its leaves by one block, level by level in shared
+// memory, a warp to a range. (A launch per level with a block to a range and one thread sweeping
+// the planes: 20 launches and 975 us of a 250k-triangle build; one launch and 430 us so.)
+struct SmallRange {
+  uint32_t b, e, seg, owner;
 };
-
-// One block splits one range of at most SMALL triangles, all in shared memory.
-__global__ void __launch_bounds__(SMALL_THREADS) k_split_small(LevelArgs a) {
-  const uint32_t i = blockIdx.x;
-  const Seg g = a.segs[a.lv0 + i];
+__global__ void __launch_bounds__(SMALL_WARPS * 32) k_split_small(Seg* __restrict__ segs, const float* __restrict__ cen,
+                                                                  const uint32_t* __restrict__ tbk, uint32_t* __restrict__ perm, int sah,
+                                                                  uint32_t* __restrict__ seg_count, uint32_t* __restrict__ too_deep) {
+  constexpr uint32_t MOST = SMALL / (LEAF_TRIS + 1) + 1;  // ranges of one level that split
+  const Seg g = segs[blockIdx.x];
   const uint32_t len = g.e - g.b;
   if (len <= LEAF_TRIS || len > SMALL) return;
   __shared__ uint32_t sp[SMALL];
-  __shared__ unsigned long long skey[SMALL];
-  __shared__ uint32_t cb[6], cnt[3 * BINS], bl[3 * BINS * 3], bh[3 * BINS * 3], runs[SMALL_THREADS];
-  __shared__ Choice choice;
-  __shared__ uint32_t total;
-  const uint32_t tid = threadIdx.x, nth = blockDim.x;
-  if (tid < 3) cb[tid] = 0xffffffffu, cb[3 + tid] = 0u;
-  for (uint32_t k = tid; k < 3 * BINS; k += nth) cnt[k] = 0;
-  for (uint32_t k = tid; k < 3 * BINS * 3; k += nth) bl[k] = 0xffffffffu, bh[k] = 0u;
+  __shared__ unsigned long long skey[SMALL];  // a median split's keys; an SAH one's scattered triangles
+  __shared__ uint32_t cnt[SMALL_WARPS][3 * BINS], bl[SMALL_WARPS][3 * BINS * 3], bh[SMALL_WARPS][3 * BINS * 3];
+  __shared__ SmallRange list[2][MOST];
+  __shared__ uint32_t count[2];
+  const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid & 31;
+  for (uint32_t k = tid; k < len; k += SMALL_WARPS * 32) sp[k] = perm[g.b + k];
+  if (tid == 0) list[0][0] = SmallRange{0, len, blockIdx.x, g.owner}, count[0] = 1, count[1] = 0;
   __syncthreads();
-  uint32_t l[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, h[3] = {0u, 0u, 0u};
-  for (uint32_t k = tid; k < len; k += nth) {
-    const uint32_t t = a.perm[g.b + k];
-    sp[k] = t;
-    for (int x = 0; x < 3; ++x) {
-      const uint32_t v = okey(a.cen[3 * (size_t)t + x]);
-      l[x] = min(l[x], v), h[x] = max(h[x], v);
+  uint32_t cur = 0;
+  for (uint32_t depth = g.depth; count[cur] != 0; ++depth, cur ^= 1) {
+    if (sah && depth >= TOO_DEEP) {
+      if (tid == 0) *too_deep = 1;
+      return;
     }
-  }
-  for (int x = 0; x < 3; ++x) atomicMin(&cb[x], l[x]), atomicMax(&cb[3 + x], h[x]);
-  __syncthreads();
-  float lo[3], hi[3];
-  for (int x = 0; x < 3; ++x) lo[x] = unkey(cb[x]), hi[x] = unkey(cb[3 + x]);
-  if (a.sah) {
-    for (uint32_t k = tid; k < len; k += nth) {
-      const uint32_t t = sp[k];
-      for (int axis = 0; axis < 3; ++axis) {
-        const float extent = __fsub_rn(hi[axis], lo[axis]);
-        if (!(extent > 0.0f)) continue;
-        const uint32_t b = axis * BINS + bin_of(a.cen[3 * (size_t)t + axis], lo[axis], extent);
-        atomicAdd(&cnt[b], 1u);
-        for (int x = 0; x < 3; ++x)
-          atomicMin(&bl[3 * b + x], a.tbk[6 * (size_t)t + x]), atomicMax(&bh[3 * b + x], a.tbk[6 * (size_t)t + 3 + x]);
-      }
-    }
-    __syncthreads();
-  }
-  if (tid == 0) choice = choose(lo, hi, cnt, bl, bh, len, a.sah != 0);
-  __syncthreads();
-  const Choice c = choice;
-  uint32_t mid;
-  if (c.kind == KIND_SAH) {  // stable partition: thread tid moves the run [r0, r1) of the range
-    const float extent = __fsub_rn(hi[c.axis], lo[c.axis]);
-    const uint32_t per = (len + nth - 1) / nth, r0 = min(len, tid * per), r1 = min(len, r0 + per);
-    uint32_t nl = 0;
-    for (uint32_t k = r0; k < r1; ++k) nl += bin_of(a.cen[3 * (size_t)sp[k] + c.axis], lo[c.axis], extent) <= (uint32_t)c.plane;
-    runs[tid] = nl;
-    __syncthreads();
-    if (tid == 0) {
-      uint32_t s = 0;
-      for (uint32_t j = 0; j < nth; ++j) {
-        const uint32_t v = runs[j];
-        runs[j] = s;
-        s += v;
-      }
-      total = s;
-    }
-    __syncthreads();
-    uint32_t left = runs[tid], right = r0 - runs[tid];
-    const uint32_t n_left = total;
-    for (uint32_t k = r0; k < r1; ++k) {
-      const uint32_t t = sp[k];
-      if (bin_of(a.cen[3 * (size_t)t + c.axis], lo[c.axis], extent) <= (uint32_t)c.plane)
-        a.perm[g.b + left++] = t;
-      else
-        a.perm[g.b + n_left + right++] = t;
-    }
-    mid = g.b + n_left;
-  } else {  // bitonic sort of (centroid key, triangle), padded to a power of two
-    uint32_t n2 = 1;
-    while (n2 < len) n2 <<= 1;
-    for (uint32_t k = tid; k < n2; k += nth) skey[k] = k < len ? median_key(a.cen, sp[k], c.axis) : ~0ull;
-    __syncthreads();
-    for (uint32_t size = 2; size <= n2; size <<= 1)
-      for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-        for (uint32_t k = tid; k < n2; k += nth) {
-          const uint32_t p = k ^ stride;
-          if (p > k) {
-            const unsigned long long x = skey[k], y = skey[p];
-            if ((x > y) == ((k & size) == 0)) skey[k] = y, skey[p] = x;
+    for (uint32_t r = warp; r < count[cur]; r += SMALL_WARPS) {
+      const SmallRange x = list[cur][r];
+      const uint32_t n = x.e - x.b;
+      uint32_t l[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, h[3] = {0u, 0u, 0u};
+      for (uint32_t k = x.b + lane; k < x.e; k += 32)
+        for (int a = 0; a < 3; ++a) {
+          const uint32_t v = okey(cen[3 * (size_t)sp[k] + a]);
+          l[a] = min(l[a], v), h[a] = max(h[a], v);
+        }
+      float lo[3], hi[3];
+      for (int a = 0; a < 3; ++a) lo[a] = unkey(__reduce_min_sync(0xffffffffu, l[a])), hi[a] = unkey(__reduce_max_sync(0xffffffffu, h[a]));
+      if (sah) {
+        for (uint32_t k = lane; k < 3 * BINS * 3; k += 32) {
+          bl[warp][k] = 0xffffffffu, bh[warp][k] = 0u;
+          if (k < 3 * BINS) cnt[warp][k] = 0u;
+        }
+        __syncwarp();
+        for (uint32_t k = x.b + lane; k < x.e; k += 32) {
+          const uint32_t t = sp[k];
+          uint32_t key[6];
+          for (int a = 0; a < 6; ++a) key[a] = tbk[6 * (size_t)t + a];
+          for (int axis = 0; axis < 3; ++axis) {
+            const float extent = __fsub_rn(hi[axis], lo[axis]);
+            if (!(extent > 0.0f)) continue;
+            const uint32_t b = axis * BINS + bin_of(cen[3 * (size_t)t + axis], lo[axis], extent);
+            atomicAdd(&cnt[warp][b], 1u);
+            for (int a = 0; a < 3; ++a) atomicMin(&bl[warp][3 * b + a], key[a]), atomicMax(&bh[warp][3 * b + a], key[3 + a]);
           }
         }
-        __syncthreads();
+        __syncwarp();
       }
-    for (uint32_t k = tid; k < len; k += nth) a.perm[g.b + k] = (uint32_t)skey[k];
-    mid = g.b + len / 2;
+      const Choice c = choose(lo, hi, cnt[warp], bl[warp], bh[warp], n, sah != 0);
+      uint32_t mid;
+      if (c.kind == KIND_SAH) {  // stable partition, 32 triangles at a time
+        uint32_t* tmp = reinterpret_cast<uint32_t*>(skey + x.b);  // in the range's own part
+        const float extent = __fsub_rn(hi[c.axis], lo[c.axis]);
+        uint32_t left = 0, right = c.left;
+        for (uint32_t k = 0; k < n; k += 32) {
+          const bool here = k + lane < n;
+          const uint32_t t = here ? sp[x.b + k + lane] : 0u;
+          const bool to_left = here && bin_of(cen[3 * (size_t)t + c.axis], lo[c.axis], extent) <= (uint32_t)c.plane;
+          const unsigned lefts = __ballot_sync(0xffffffffu, to_left), rights = __ballot_sync(0xffffffffu, here && !to_left);
+          const unsigned below = (1u << lane) - 1u;
+          if (here) tmp[to_left ? left + __popc(lefts & below) : right + __popc(rights & below)] = t;
+          left += __popc(lefts), right += __popc(rights);
+        }
+        __syncwarp();
+        for (uint32_t k = lane; k < n; k += 32) sp[x.b + k] = tmp[k];
+        mid = x.b + c.left;
+      } else {  // bitonic sort of (centroid key, triangle), the places past the range left out
+        unsigned long long* key = skey + x.b;
+        for (uint32_t k = lane; k < n; k += 32) key[k] = median_key(cen, sp[x.b + k], c.axis);
+        __syncwarp();
+        uint32_t n2 = 1;
+        while (n2 < n) n2 <<= 1;
+        for (uint32_t size = 2; size <= n2; size <<= 1)
+          for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+            for (uint32_t k = lane; k < n; k += 32) {
+              const uint32_t p = stride == size >> 1 ? k ^ (size - 1) : k ^ stride;  // each merge starts mirrored
+              if (p > k && p < n) {
+                const unsigned long long u = key[k], v = key[p];
+                if (u > v) key[k] = v, key[p] = u;
+              }
+            }
+            __syncwarp();
+          }
+        for (uint32_t k = lane; k < n; k += 32) sp[x.b + k] = (uint32_t)key[k];
+        mid = x.b + n / 2;
+      }
+      __syncwarp();
+      if (lane == 0) {
+        const uint32_t at = atomicAdd(seg_count, 2u), own = (depth & 1u) ? x.owner : x.seg;
+        segs[at] = Seg{g.b + x.b, g.b + mid, depth + 1, own};
+        segs[at + 1] = Seg{g.b + mid, g.b + x.e, depth + 1, own};
+        if (mid - x.b > LEAF_TRIS) list[cur ^ 1][atomicAdd(&count[cur ^ 1], 1u)] = SmallRange{x.b, mid, at, own};
+        if (x.e - mid > LEAF_TRIS) list[cur ^ 1][atomicAdd(&count[cur ^ 1], 1u)] = SmallRange{mid, x.e, at + 1, own};
+      }
+    }
+    __syncthreads();
+    if (tid == 0) count[cur] = 0;
+    __syncthreads();
   }
-  if (tid == 0) write_children(a.segs, a.lv0, i, g, mid, a.next, a.rank);
+  for (uint32_t k = tid; k < len; k += SMALL_WARPS * 32) perm[g.b + k] = sp[k];
 }
 
 // ---- ranges larger than SMALL: several blocks each, reductions merged through global atomics ----
 
 __global__ void k_large_list(const Seg* __restrict__ segs, uint32_t width, const unsigned long long* __restrict__ rank,
-                             LargeSeg* __restrict__ out) {
+                             LargeSeg* __restrict__ out, uint32_t cap) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= width) return;
   const Seg g = segs[i];
-  if (g.e - g.b > SMALL) out[rank[i] >> 32] = LargeSeg{i, g.b, g.e, 0, 0};
+  if (g.e - g.b > SMALL && (uint32_t)(rank[i] >> 32) < cap) out[rank[i] >> 32] = LargeSeg{i, g.b, g.e, 0, 0};
 }
 
 __global__ void k_large_init(LWork* __restrict__ w, uint32_t n) {
@@ -367,14 +397,12 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_large_bins(const Chunk* __res
   }
 }
 
-__global__ void k_large_choose(const LargeSeg* __restrict__ large, uint32_t n, LWork* __restrict__ work, int sah) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  LWork& w = work[j];
+__global__ void k_large_choose(const LargeSeg* __restrict__ large, LWork* __restrict__ work, int sah) {
+  LWork& w = work[blockIdx.x];
   float lo[3], hi[3];
   bounds_of(w, lo, hi);
-  const Choice c = choose(lo, hi, w.cnt, w.bl, w.bh, large[j].e - large[j].b, sah != 0);
-  w.kind = c.kind, w.axis = c.axis, w.plane = c.plane;
+  const Choice c = choose(lo, hi, w.cnt, w.bl, w.bh, large[blockIdx.x].e - large[blockIdx.x].b, sah != 0);
+  if (threadIdx.x == 0) w.kind = c.kind, w.axis = c.axis, w.plane = c.plane;
 }
 
 __device__ __forceinline__ bool goes_left(const LWork& w, const float* cen, uint32_t t) {
@@ -570,16 +598,17 @@ __global__ void k_node_children(uint32_t n, const uint32_t* __restrict__ kid_n, 
   if (r == n - 1) parent[r] = EMPTY;  // postorder: the root
 }
 
-// Device memory for one build, carved out of one allocation; freed once the build's stream has
-// drained (an early error return may leave work in flight).
+// Device memory for one build, carved out of one allocation: the context's workspace `slot` where it
+// fits (kept between builds, up to BUILD_KEEP bytes; the caller holds the context's lock until the
+// build is done), else memory of its own, freed once the build's stream has drained (an early error
+// return may leave work in flight).
 class Arena {
  public:
-  explicit Arena(cudaStream_t s) : stream_(s) {}
+  Arena(rt_ctx* ctx, int slot, cudaStream_t s) : ctx_(ctx), slot_(slot), stream_(s) {}
   ~Arena() {
-    if (base_) {
-      cudaStreamSynchronize(stream_);
-      cudaFree(base_);
-    }
+    if (!base_) return;
+    cudaStreamSynchronize(stream_);
+    if (own_) cudaFree(base_);
   }
   template <class T>
   T* take(size_t n) {
@@ -589,10 +618,31 @@ class Arena {
   }
   template <class T>
   void plan(size_t n) { size_ += (n * sizeof(T) + 255) & ~(size_t)255; }
-  cudaError_t allocate() { return cudaMalloc(&base_, size_); }
+  cudaError_t allocate() {
+    auto& kept = ctx_->build_space[slot_];
+    if (size_ > BUILD_KEEP) {
+      own_ = true;
+      return cudaMalloc(&base_, size_);
+    }
+    if (size_ > kept.bytes) {
+      cudaFree(kept.p);
+      kept.p = nullptr, kept.bytes = 0;
+      const cudaError_t e = cudaMalloc(&kept.p, size_);
+      if (e != cudaSuccess) {
+        kept.p = nullptr;
+        return e;
+      }
+      kept.bytes = size_;
+    }
+    base_ = kept.p;
+    return cudaSuccess;
+  }
 
  private:
+  rt_ctx* ctx_;
+  int slot_;
   cudaStream_t stream_;
+  bool own_ = false;
   void* base_ = nullptr;
   size_t size_ = 0, used_ = 0;
 };
@@ -657,7 +707,7 @@ rt_status rt_blas_build_device(rt_ctx* ctx, const float* positions, uint32_t n_p
     RT_CUDA(ctx, cub::DeviceSegmentedSort::SortKeys(nullptr, b, u64, u64, (int)nt, (int)large_cap, u32, u32, st));
     cub_bytes = std::max(cub_bytes, b);
   }
-  Arena ar(st);
+  Arena ar(ctx, 0, st);
   ar.plan<float>(3 * (size_t)n_positions);  // positions
   ar.plan<uint32_t>(n_indices);             // indices
   ar.plan<float>(3 * (size_t)nt);           // centroids
@@ -728,67 +778,71 @@ rt_status rt_blas_build_device(rt_ctx* ctx, const float* positions, uint32_t n_p
     const Seg root{0, nt, 0, EMPTY};
     RT_CUDA(ctx, cudaMemcpyAsync(d_segs, &root, sizeof root, cudaMemcpyHostToDevice, st));
     uint32_t lv0 = 0, width = 1, depth = 0;
-    bool too_deep = false;
-    for (;;) {
+    uint32_t over[2] = {0, 0};  // ranges so far, and whether one passed the depth
+    for (uint32_t most = nt > SMALL ? 1 : 0; most != 0;) {  // while a range of this level can be large
       k_level_flags<<<blocks(width + 1, 256), 256, 0, st>>>(d_segs + lv0, width, d_flags);
       size_t nb = 0;
       RT_CUDA(ctx, cub::DeviceScan::ExclusiveSum(nullptr, nb, d_flags, d_rank, (int)width + 1, st));
       if (nb > cub_bytes) return fail(ctx, RT_ERR_OOM, "device build: scan scratch");
       RT_CUDA(ctx, cub::DeviceScan::ExclusiveSum(d_cub, nb, d_flags, d_rank, (int)width + 1, st));
+      most = std::min<uint32_t>(most, (uint32_t)large_cap);
+      k_large_list<<<blocks(width, 256), 256, 0, st>>>(d_segs + lv0, width, d_rank, d_large, (uint32_t)large_cap);
       unsigned long long totals = 0;
+      large.resize(most);
       RT_CUDA(ctx, cudaMemcpyAsync(&totals, d_rank + width, 8, cudaMemcpyDeviceToHost, st));
+      RT_CUDA(ctx, cudaMemcpyAsync(large.data(), d_large, most * sizeof(LargeSeg), cudaMemcpyDeviceToHost, st));
       RT_CUDA(ctx, cudaStreamSynchronize(st));
-      const uint32_t pending = (uint32_t)totals, n_large = (uint32_t)(totals >> 32);
-      if (pending == 0) break;
+      const uint32_t n_large = (uint32_t)(totals >> 32);
+      if (n_large == 0) break;
       if (sah && depth >= TOO_DEEP) {
-        too_deep = true;
+        over[1] = 1;
         break;
       }
       const uint32_t next = lv0 + width;
-      if ((size_t)next + 2 * (size_t)pending > seg_cap || n_large > large_cap)
+      if ((size_t)next + 2 * (size_t)n_large > seg_cap || n_large > most)
         return fail(ctx, RT_ERR_OOM, "device build: range table overflow");
-      if (n_large) {
-        k_large_list<<<blocks(width, 256), 256, 0, st>>>(d_segs + lv0, width, d_rank, d_large);
-        large.resize(n_large);
-        RT_CUDA(ctx, cudaMemcpyAsync(large.data(), d_large, n_large * sizeof(LargeSeg), cudaMemcpyDeviceToHost, st));
-        RT_CUDA(ctx, cudaStreamSynchronize(st));
-        chunks.clear();
-        for (uint32_t j = 0; j < n_large; ++j) {
-          large[j].first = (uint32_t)chunks.size();
-          for (uint32_t s = large[j].b; s < large[j].e; s += std::min(CHUNK, large[j].e - s))
-            chunks.push_back(Chunk{j, s, s + std::min(CHUNK, large[j].e - s)});
-          large[j].n = (uint32_t)chunks.size() - large[j].first;
-        }
-        const uint32_t nc = (uint32_t)chunks.size();
-        if (nc > chunk_cap) return fail(ctx, RT_ERR_OOM, "device build: chunk table overflow");
-        RT_CUDA(ctx, cudaMemcpyAsync(d_large, large.data(), n_large * sizeof(LargeSeg), cudaMemcpyHostToDevice, st));
-        RT_CUDA(ctx, cudaMemcpyAsync(d_chunks, chunks.data(), nc * sizeof(Chunk), cudaMemcpyHostToDevice, st));
-        k_large_init<<<n_large, 128, 0, st>>>(d_work, n_large);
-        k_large_cbox<<<nc, CHUNK_THREADS, 0, st>>>(d_chunks, d_perm, d_cen, d_work);
-        if (sah) k_large_bins<<<nc, CHUNK_THREADS, 0, st>>>(d_chunks, d_perm, d_cen, d_tbk, d_work);
-        k_large_choose<<<blocks(n_large, 64), 64, 0, st>>>(d_large, n_large, d_work, sah);
-        k_large_count<<<nc, CHUNK_THREADS, 0, st>>>(d_chunks, d_perm, d_cen, d_work, d_chunk_left);
-        k_large_scan<<<blocks(n_large, 64), 64, 0, st>>>(d_large, n_large, d_work, d_chunk_left, d_chunk_base, d_sort_begin,
-                                                           d_sort_end, d_segs, lv0, next, d_rank);
-        k_large_scatter<<<nc, CHUNK_THREADS, 0, st>>>(d_chunks, d_large, d_perm, d_cen, d_work, d_chunk_base, d_tmp);
-        k_large_copy<<<nc, CHUNK_THREADS, 0, st>>>(d_chunks, d_work, d_tmp, d_perm);
-        k_large_keys<<<nc, CHUNK_THREADS, 0, st>>>(d_chunks, d_work, d_perm, d_cen, d_keys);
-        nb = 0;
-        RT_CUDA(ctx, cub::DeviceSegmentedSort::SortKeys(nullptr, nb, d_keys, d_keys_out, (int)nt, (int)n_large, d_sort_begin,
-                                                        d_sort_end, st));
-        if (nb > cub_bytes) return fail(ctx, RT_ERR_OOM, "device build: sort scratch");
-        RT_CUDA(ctx, cub::DeviceSegmentedSort::SortKeys(d_cub, nb, d_keys, d_keys_out, (int)nt, (int)n_large, d_sort_begin,
-                                                        d_sort_end, st));
-        k_large_unkey<<<nc, CHUNK_THREADS, 0, st>>>(d_chunks, d_work, d_keys_out, d_perm);
-        RT_CUDA(ctx, cudaGetLastError());
+      large.resize(n_large);
+      chunks.clear();
+      for (uint32_t j = 0; j < n_large; ++j) {
+        large[j].first = (uint32_t)chunks.size();
+        for (uint32_t s = large[j].b; s < large[j].e; s += std::min(CHUNK, large[j].e - s))
+          chunks.push_back(Chunk{j, s, s + std::min(CHUNK, large[j].e - s)});
+        large[j].n = (uint32_t)chunks.size() - large[j].first;
       }
-      LevelArgs a{d_segs, lv0, width, next, d_rank, d_cen, d_tbk, d_perm, sah ? 1 : 0};
-      k_split_small<<<width, SMALL_THREADS, 0, st>>>(a);
+      const uint32_t nc = (uint32_t)chunks.size();
+      if (nc > chunk_cap) return fail(ctx, RT_ERR_OOM, "device build: chunk table overflow");
+      RT_CUDA(ctx, cudaMemcpyAsync(d_large, large.data(), n_large * sizeof(LargeSeg), cudaMemcpyHostToDevice, st));
+      RT_CUDA(ctx, cudaMemcpyAsync(d_chunks, chunks.data(), nc * sizeof(Chunk), cudaMemcpyHostToDevice, st));
+      k_large_init<<<n_large, 128, 0, st>>>(d_work, n_large);
+      k_large_cbox<<<nc, CHUNK_THREADS, 0, st>>>(d_chunks, d_perm, d_cen, d_work);
+      if (sah) k_large_bins<<<nc, CHUNK_THREADS, 0, st>>>(d_chunks, d_perm, d_cen, d_tbk, d_work);
+      k_large_choose<<<n_large, 32, 0, st>>>(d_large, d_work, sah);
+      k_large_count<<<nc, CHUNK_THREADS, 0, st>>>(d_chunks, d_perm, d_cen, d_work, d_chunk_left);
+      k_large_scan<<<blocks(n_large, 64), 64, 0, st>>>(d_large, n_large, d_work, d_chunk_left, d_chunk_base, d_sort_begin,
+                                                         d_sort_end, d_segs, lv0, next, d_rank);
+      k_large_scatter<<<nc, CHUNK_THREADS, 0, st>>>(d_chunks, d_large, d_perm, d_cen, d_work, d_chunk_base, d_tmp);
+      k_large_copy<<<nc, CHUNK_THREADS, 0, st>>>(d_chunks, d_work, d_tmp, d_perm);
+      k_large_keys<<<nc, CHUNK_THREADS, 0, st>>>(d_chunks, d_work, d_perm, d_cen, d_keys);
+      nb = 0;
+      RT_CUDA(ctx, cub::DeviceSegmentedSort::SortKeys(nullptr, nb, d_keys, d_keys_out, (int)nt, (int)n_large, d_sort_begin,
+                                                      d_sort_end, st));
+      if (nb > cub_bytes) return fail(ctx, RT_ERR_OOM, "device build: sort scratch");
+      RT_CUDA(ctx, cub::DeviceSegmentedSort::SortKeys(d_cub, nb, d_keys, d_keys_out, (int)nt, (int)n_large, d_sort_begin,
+                                                      d_sort_end, st));
+      k_large_unkey<<<nc, CHUNK_THREADS, 0, st>>>(d_chunks, d_work, d_keys_out, d_perm);
       RT_CUDA(ctx, cudaGetLastError());
-      lv0 = next, width = 2 * pending, ++depth;
+      lv0 = next, width = most = 2 * n_large, ++depth;
     }
-    if (!too_deep) {
-      total = lv0 + width;
+    if (!over[1]) {
+      over[0] = lv0 + width;
+      RT_CUDA(ctx, cudaMemcpyAsync(d_count + 2, over, 8, cudaMemcpyHostToDevice, st));
+      k_split_small<<<over[0], SMALL_WARPS * 32, 0, st>>>(d_segs, d_cen, d_tbk, d_perm, sah ? 1 : 0, d_count + 2, d_count + 3);
+      RT_CUDA(ctx, cudaGetLastError());
+      RT_CUDA(ctx, cudaMemcpyAsync(over, d_count + 2, 8, cudaMemcpyDeviceToHost, st));
+      RT_CUDA(ctx, cudaStreamSynchronize(st));
+    }
+    if (!over[1]) {
+      total = over[0];
       break;
     }
     sah = false;  // near_field.rs:186-188
@@ -823,7 +877,7 @@ rt_status rt_blas_build_device(rt_ctx* ctx, const float* positions, uint32_t n_p
     RT_CUDA(ctx, cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, u64, u64, u32, u32, (int)std::max(n_nodes, 1u), 0, 64, st));
   }
   const size_t nn = std::max(n_nodes, 1u);
-  Arena rec(st);
+  Arena rec(ctx, 1, st);
   rec.plan<uint32_t>(out_words);
   rec.plan<uint32_t>(n_leaves);  // leaf sources
   rec.plan<unsigned long long>(nn);  // node keys, sorted

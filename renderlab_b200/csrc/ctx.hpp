@@ -71,6 +71,9 @@ struct rt_rnf {
 #define RT_HOST_STAGES 4
 #endif
 
+// Bytes of each BLAS build workspace that a context keeps (meshes of about 300k triangles).
+constexpr size_t BUILD_KEEP = 64u << 20;
+
 struct rt_ctx {
   int device = 0;
   rtk::DevStatus* d_status = nullptr;
@@ -91,6 +94,11 @@ struct rt_ctx {
   // rt_order_rays scratch
   void* d_order_scratch = nullptr;
   size_t order_scratch_bytes = 0;
+  // rt_blas_build_device's two workspaces, kept up to BUILD_KEEP bytes each (under `mu`)
+  struct Space {
+    void* p = nullptr;
+    size_t bytes = 0;
+  } build_space[2];
   // rt_trace_batches: batch tables staged through a ring of pinned / device slots, each reused
   // once the copy that last read it has completed.
   static constexpr uint32_t TABLE_SLOTS = 8;

@@ -216,6 +216,7 @@ void rt_ctx_destroy(rt_ctx* ctx) {
   cudaFree(ctx->d_rays);
   cudaFree(ctx->d_hits);
   cudaFree(ctx->d_order_scratch);
+  for (auto& b : ctx->build_space) cudaFree(b.p);
   cudaFree(ctx->d_tables);
   cudaFreeHost(ctx->h_tables);
   for (cudaEvent_t e : ctx->table_done)
