@@ -743,11 +743,17 @@ RT_DEV void w8_top_node(const W8View& V, const uint4* cache, uint32_t cached, ui
 // instances: 7.47 ms, 11.9 with every kind run each time around. In a flat scene nearly all lanes
 // wait for a node, and loads bound the walk, so all run: nodes, each with its leaves at once, and
 // entries. 4.19M GI rays over 1M triangles: 4.66 ms, 4.90 with a vote and 5.11 with leaves as steps of
-// their own (which also drops the top level's stack: 5.45 ms before all of this).
+// their own (which also drops the top level's stack: 5.45 ms before all of this). An any-hit walk, whose
+// triangle tests end rays instead of shortening them, takes leaves as steps once half as many lanes
+// wait for them as for nodes: 0.84M shadow rays over 250k triangles 645 us, 708 with leaves at once
+// (a third, a half and a fifth as many: 649, 663 and 674; closest hits 1 % slower so).
+//
+// `lanes`: those of a warp that take rays, as in the FAST kernels (RayQueue).
 template <uint32_t LAYOUT, int AM, int BLOCK, bool COUNT, class Src, int SS = 0, bool LAZY = false>
 __global__ void __launch_bounds__(BLOCK, LAZY ? W8_TOP_BLOCKS : W8_FLAT_BLOCKS) k_wide8(const uint32_t* __restrict__ w, W8View V, const Src src,
                                                  unsigned int* __restrict__ counter, uint32_t n, DevStatus* st,
-                                                 unsigned long long* cnt, uint32_t refill) {
+                                                 unsigned long long* cnt, uint32_t refill, uint32_t lanes) {
+  constexpr bool LEAF_STEPS = LAZY || AM == 1;
   W8GroupStack<SS, BLOCK> stack;
   if constexpr (SS > 0) {
     __shared__ uint2 columns[SS * BLOCK];
@@ -807,7 +813,7 @@ __global__ void __launch_bounds__(BLOCK, LAZY ? W8_TOP_BLOCKS : W8_FLAT_BLOCKS) 
     __syncwarp();
     // ray refill (warp-aggregated) once `refill` lanes are idle: 1 keeps every lane busy,
     // 32 hands out whole runs of 32 consecutive rays (keeps a coherent batch's tiles together)
-    const unsigned idle = __ballot_sync(0xffffffffu, L.phase == PH_IDLE || L.phase == PH_DONE);
+    const unsigned idle = __ballot_sync(0xffffffffu, L.phase == PH_IDLE || L.phase == PH_DONE) & lanes;
     const unsigned want = (!drained && (uint32_t)__popc(idle) >= refill) ? idle : 0u;
     uint32_t id = EMPTY;
     if (want) {
@@ -835,8 +841,17 @@ __global__ void __launch_bounds__(BLOCK, LAZY ? W8_TOP_BLOCKS : W8_FLAT_BLOCKS) 
       }
       next_top();
     }
-    const uint32_t run = LAZY ? vote_phase(L.phase) : L.phase;
-    const bool none = LAZY ? run == PH_IDLE : !__any_sync(0xffffffffu, L.phase == PH_NODE || L.phase == PH_ENTER);
+    uint32_t run = LAZY ? vote_phase(L.phase) : L.phase;
+    bool none = run == PH_IDLE;
+    if (!LAZY && LEAF_STEPS) {
+      const unsigned on = __ballot_sync(0xffffffffu, L.phase == PH_NODE || L.phase == PH_ENTER);
+      const unsigned leaf = __ballot_sync(0xffffffffu, L.phase == PH_LEAF);
+      none = (on | leaf) == 0;
+      const bool leaves = leaf != 0 && 2 * __popc(leaf) >= __popc(on);
+      if (leaves != (run == PH_LEAF)) run = PH_IDLE;  // this lane waits
+    } else if (!LAZY) {
+      none = !__any_sync(0xffffffffu, L.phase == PH_NODE || L.phase == PH_ENTER);
+    }
     if (none) {
       if (drained) break;
       continue;
@@ -844,23 +859,23 @@ __global__ void __launch_bounds__(BLOCK, LAZY ? W8_TOP_BLOCKS : W8_FLAT_BLOCKS) 
     if (L.phase != run) continue;
     if (run == PH_NODE) {
       w8_node<COUNT>(V, L, stack, st, cnt);
-      if (LAZY && L.leaves) {
+      if (LEAF_STEPS && L.leaves) {
         L.phase = PH_LEAF;
         continue;
       }
       bool blocked = false;
-      if (!LAZY)
+      if (!LEAF_STEPS)
         while (L.leaves && !blocked) blocked = w8_leaf<LAYOUT, AM, COUNT, LAZY>(w, V, L, cnt);
       if (blocked) L.phase = PH_DONE;
       else next_node();
+    } else if (LEAF_STEPS && run == PH_LEAF) {
+      if (w8_leaf<LAYOUT, AM, COUNT, LAZY>(w, V, L, cnt)) L.phase = PH_DONE;
+      else if (L.leaves == 0) next_node();
     } else if (!LAZY) {
       if (run == PH_ENTER) {
         w8_enter<LAYOUT, AM, COUNT, LAZY, false>(w, V, L, L.node, cnt, false, 0);
         if (L.phase == PH_ENTER) next_top();
       }
-    } else if (run == PH_LEAF) {
-      if (w8_leaf<LAYOUT, AM, COUNT, LAZY>(w, V, L, cnt)) L.phase = PH_DONE;
-      else if (L.leaves == 0) next_node();
     } else if (run == PH_ENTER) {
       w8_enter<LAYOUT, AM, COUNT, LAZY>(w, V, L, L.node, cnt, top != 0, L.at);
       if (L.phase == PH_ENTER) next_top();

@@ -46,9 +46,15 @@ cudaError_t run(K kernel, const uint32_t* words, const rtk::W8View& v, const Src
   uint32_t full = 0;
   cudaError_t e = resident(kernel, full);
   if (e != cudaSuccess) return e;
-  const uint32_t need = (n + W8_BLOCK - 1) / W8_BLOCK;
+  // a launch that does not fill the resident warps spreads its rays over half of them, in as few lanes
+  // each as hold them (3,000 GI rays over 250k triangles: 97 -> 81 us, 20,000: 117 -> 114)
+  constexpr uint32_t warps = W8_BLOCK / 32;
+  uint32_t width = 1;
+  while (width < 32 && (uint64_t)full * warps * width < 2 * (uint64_t)n) width *= 2;
+  const uint32_t need = (uint32_t)(((uint64_t)n + warps * width - 1) / (warps * width));
   if ((e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), stream)) != cudaSuccess) return e;
-  kernel<<<need < full ? need : full, W8_BLOCK, 0, stream>>>(words, v, src, counter, n, st, cnt, refill);
+  kernel<<<need < full ? need : full, W8_BLOCK, 0, stream>>>(words, v, src, counter, n, st, cnt, refill < width ? refill : width,
+                                                               width == 32 ? 0xffffffffu : (1u << width) - 1u);
   return cudaGetLastError();
 }
 
