@@ -304,9 +304,10 @@ RT_DEV void gi_traverse(const uint32_t* __restrict__ w, GiLane<AM>& L, DevStatus
   }
 }
 
-// Resident blocks of 128 threads an SM (72 registers): 6, 7 and 8 give 2.17, 2.10 and 2.15 ms for 1M GI
-// rays over 250k triangles, 559, 538 and 539 us for 1M camera rays there (reflection).
-constexpr int PLAIN_MIN_BLOCKS = 7;
+// Resident blocks of 128 threads an SM. Closest hits (72 registers): 6, 7 and 8 give 2.17, 2.10 and 2.15
+// ms for 1M GI rays over 250k triangles, 559, 538 and 539 us for 1M camera rays there (reflection).
+// Any hit (64 registers): 7, 8, 9 and 10 give 1.87, 1.76, 1.75 and 1.79 ms for 1M shadow rays there.
+constexpr int PLAIN_MIN_BLOCKS = 7, PLAIN_ANY_BLOCKS = 8;
 
 // The ray of this thread: `width` rays to a warp, in its first lanes (n: none).
 RT_DEV uint32_t plain_ray(uint32_t width, uint32_t n) {
@@ -316,7 +317,7 @@ RT_DEV uint32_t plain_ray(uint32_t width, uint32_t n) {
 }
 
 template <int AM, class Src>
-__global__ void __launch_bounds__(128, PLAIN_MIN_BLOCKS) k_gi_plain(const uint32_t* __restrict__ w, const Src src, uint32_t n, uint32_t width,
+__global__ void __launch_bounds__(128, AM ? PLAIN_ANY_BLOCKS : PLAIN_MIN_BLOCKS) k_gi_plain(const uint32_t* __restrict__ w, const Src src, uint32_t n, uint32_t width,
                                                   DevStatus* st) {
   const uint32_t i = plain_ray(width, n);
   if (i == n) return;
@@ -518,7 +519,7 @@ RT_DEV void rs_trace(const uint32_t* __restrict__ w, RsLane<AM>& L, DevStatus* s
 }
 
 template <int AM, class Src>
-__global__ void __launch_bounds__(128, PLAIN_MIN_BLOCKS) k_rs_plain(const uint32_t* __restrict__ w, const Src src, uint32_t n, uint32_t width,
+__global__ void __launch_bounds__(128, AM ? PLAIN_ANY_BLOCKS : PLAIN_MIN_BLOCKS) k_rs_plain(const uint32_t* __restrict__ w, const Src src, uint32_t n, uint32_t width,
                                                   DevStatus* st) {
   const uint32_t i = plain_ray(width, n);
   if (i == n) return;
