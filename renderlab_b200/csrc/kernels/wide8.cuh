@@ -35,14 +35,15 @@ constexpr uint32_t W8_STACK = 32;
 // levels deep stacks at most W8_SSTACK - 1 groups).
 constexpr uint32_t W8_SSTACK = 16;
 // Resident 128-thread blocks per SM the register allocation is sized for.
-// Flat scenes (W8_FLAT_BLOCKS, 96 registers): the lane's ray and best hit stay in registers, which
-// takes more than 72; 4.19M GI rays over 1M triangles: 4.92, 4.66 and 5.13 ms at 4, 5 and 6 blocks
-// (with both in local memory 5.45 ms at 7, the fastest then). Scenes with a top level
-// (W8_TOP_BLOCKS, 72 registers, both in local memory): 7.48 ms a plan over 1,000 instances, and 12.6
-// against 11.9 ms with both in registers before the walk voted. The packet walk (W8P_MIN_BLOCKS, 72
-// registers, both in local memory, about 140 bytes of spills): 3.01, 2.93, 2.88 and 3.12 ms for
-// 4.19M camera rays at 5, 6, 7 and 8 blocks, and 3.2 ms at 5 to 7 with both in registers.
-constexpr int W8_FLAT_BLOCKS = 5, W8_TOP_BLOCKS = 7, W8P_MIN_BLOCKS = 7;
+// The per-ray walk (W8_BLOCKS, 96 registers): the lane's ray and best hit stay in registers, which
+// takes more than 72. Flat scenes, 4.19M GI rays over 1M triangles: 4.92, 4.66 and 5.13 ms at 4, 5 and
+// 6 blocks (with both in local memory 5.45 ms at 7, the fastest then). Top level, 1.2M rays in 32
+// batches over 1,000 instances: 7.74, 7.30 and 7.58 ms at 4, 5 and 6 blocks, 7.47 with both in local
+// memory at 7; smaller batches over 200 and 600 instances 1,198 and 994 us against 1,278 and 1,099.
+// The packet walk (W8P_MIN_BLOCKS, 72 registers, both in local memory, about 140 bytes of spills):
+// 3.01, 2.93, 2.88 and 3.12 ms for 4.19M camera rays at 5, 6, 7 and 8 blocks, and 3.2 ms at 5 to 7 with
+// both in registers.
+constexpr int W8_BLOCKS = 5, W8P_MIN_BLOCKS = 7;
 
 // Opt-in device counters of the WIDE8 walk (diagnostics and the bytes-per-ray roofline).
 enum W8Count { W8C_RAYS, W8C_TOP_NODES, W8C_INSTANCE_TESTS, W8C_NODES, W8C_LEAVES, W8C_TRIS, W8C_RETESTS, W8C_FINAL64, W8C_N };
@@ -483,7 +484,7 @@ RT_DEV bool w8_leaf(const uint32_t* __restrict__ w, const W8View& V, W8Lane& L, 
   const uint32_t first = L.tri_base + (m & 31u), count = m >> 5;
   w8_count<COUNT>(cnt, W8C_LEAVES);
   for (uint32_t k = 0; k < count; ++k)
-    if (w8_candidate<LAYOUT, AM, COUNT, LAZY, !LAZY>(w, V, L.R, L.ray, L.inst, first + k, L.best, cnt, L.any)) return true;
+    if (w8_candidate<LAYOUT, AM, COUNT, LAZY, true>(w, V, L.R, L.ray, L.inst, first + k, L.best, cnt, L.any)) return true;
   return false;
 }
 
@@ -740,7 +741,7 @@ RT_DEV void w8_top_node(const W8View& V, const uint4* cache, uint32_t cached, ui
 // Over a top level the lanes of a warp wait for different kinds of step (top-level node, instance
 // entry, BLAS node, leaf), and instruction issue bounds the walk; the warp runs the one that most of
 // them wait for (vote_phase), one leaf a step. 1.2M rays in 32 batches over 1,000 overlapping
-// instances: 7.47 ms, 11.9 with every kind run each time around. In a flat scene nearly all lanes
+// instances: 7.3 ms, 11.9 with every kind run each time around. In a flat scene nearly all lanes
 // wait for a node, and loads bound the walk, so all run: nodes, each with its leaves at once, and
 // entries. 4.19M GI rays over 1M triangles: 4.66 ms, 4.90 with a vote and 5.11 with leaves as steps of
 // their own (which also drops the top level's stack: 5.45 ms before all of this). An any-hit walk, whose
@@ -750,7 +751,7 @@ RT_DEV void w8_top_node(const W8View& V, const uint4* cache, uint32_t cached, ui
 //
 // `lanes`: those of a warp that take rays, as in the FAST kernels (RayQueue).
 template <uint32_t LAYOUT, int AM, int BLOCK, bool COUNT, class Src, int SS = 0, bool LAZY = false>
-__global__ void __launch_bounds__(BLOCK, LAZY ? W8_TOP_BLOCKS : W8_FLAT_BLOCKS) k_wide8(const uint32_t* __restrict__ w, W8View V, const Src src,
+__global__ void __launch_bounds__(BLOCK, W8_BLOCKS) k_wide8(const uint32_t* __restrict__ w, W8View V, const Src src,
                                                  unsigned int* __restrict__ counter, uint32_t n, DevStatus* st,
                                                  unsigned long long* cnt, uint32_t refill, uint32_t lanes) {
   constexpr bool LEAF_STEPS = LAZY || AM == 1;
@@ -796,7 +797,7 @@ __global__ void __launch_bounds__(BLOCK, LAZY ? W8_TOP_BLOCKS : W8_FLAT_BLOCKS) 
       uint32_t bits = ey & 0xffu;  // a group: its first pending child now, the rest back on the stack
       const uint32_t imask = ey >> 8, k = __ffs(bits) - 1;
       bits &= bits - 1;
-      if (bits) tstack[L.tsp] = ex, tstack[L.tsp + 1] = bits | imask << 8, L.tsp += 2;
+      if (bits) tstack[L.tsp + 1] = bits | imask << 8, L.tsp += 2;
       const uint32_t slot = k ^ octant_of(L.ray.d);
       L.node = ex + __popc(imask & ((1u << slot) - 1u)), L.phase = PH_TOP;
       return;
