@@ -96,7 +96,9 @@ typedef struct rt_gi_hit {
 /* Where the WIDE8 per-ray walk keeps each lane's node-group stack (rt_tuning.wide8_stack,
  * rt_plan_desc.stack; 0 there means unchanged / the context's choice). No counterpart in the
  * reference, whose WGSL loops keep a fixed array per invocation. */
-#define RT_STACK_LOCAL 1u  /* 32 entries a lane in local memory, cached by L1 (the default) */
+#define RT_STACK_LOCAL 1u  /* 32 entries a lane in local memory, cached by L1 (the default, unless
+                            * no placement was ever set: then any-hit launches over flat scenes that
+                            * RT_STACK_SHARED fits take that one) */
 #define RT_STACK_SHARED 2u /* 16 entries a lane in shared memory: only for scenes whose 8-wide trees are
                             * at most 16 levels deep (else RT_ERR_UNSUPPORTED) */
 /* Launch parameters the autotuner chooses (renderlab_b200.tune); zero fields keep defaults. */

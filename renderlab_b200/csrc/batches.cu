@@ -74,7 +74,7 @@ cudaError_t enqueue(const rt_scene* scene, rt_kernel kernel, const rtk::BatchEnt
   const rtl::SceneView v = view_of(scene);
   if (kernel == RT_KERNEL_WIDE8)
     return rtl::launch_wide8_batches(v, d_table, entries, total, order, counter, st, s, refill, uniform,
-                                     stack == RT_STACK_SHARED ? 1u : 0u);
+                                     stack_of(stack, v, uniform == 1));
   if (kernel == RT_KERNEL_WIDE8_PACKET)
     return rtl::launch_wide8_packet_batches(v, d_table, entries, total, order, counter, st, s, uniform);
   return rtl::launch_fast_batches(v, d_table, entries, total, order, counter, st, s, refill, uniform);
@@ -124,12 +124,12 @@ rt_status rt_trace_batches(rt_ctx* ctx, const rt_scene* scene, rt_kernel kernel,
   RT_CUDA(ctx, cudaMemcpyAsync(d, h, sizeof(rtk::BatchEntry) * n_batches, cudaMemcpyHostToDevice, s));
   RT_CUDA(ctx, cudaEventRecord(ctx->table_done[slot], s));
   const uint32_t refill = kernel == RT_KERNEL_FAST ? ctx->tuning.fast_refill : ctx->tuning.wide8_refill;
-  if (kernel == RT_KERNEL_WIDE8 && ctx->tuning.wide8_stack == RT_STACK_SHARED && !rtl::shared_stack_fits(view_of(scene)))
+  if (kernel == RT_KERNEL_WIDE8 && chosen_stack(ctx) == RT_STACK_SHARED && !rtl::shared_stack_fits(view_of(scene)))
     return fail(ctx, RT_ERR_UNSUPPORTED, "the shared group stack holds 16 levels; this scene's 8-wide trees have %u",
                 scene->w8_depth);
   cudaError_t e = enqueue(scene, kernel, d, n_batches, (uint32_t)total, nullptr,
                           ctx->d_counters + (ctx->counter_seq++ % COUNTER_SLOTS), ctx->d_status, s, refill, uniform,
-                          ctx->tuning.wide8_stack);
+                          chosen_stack(ctx));
   if (e != cudaSuccess) return fail(ctx, RT_ERR_CUDA, "many-batch launch: %s", cudaGetErrorString(e));
   ctx->rays += total;
   ctx->launches += 1;
@@ -140,7 +140,7 @@ struct rt_plan {
   rt_ctx* ctx = nullptr;
   const rt_scene* scene = nullptr;
   rt_plan_desc desc{};
-  uint32_t entries = 0, total = 0, refill = 8, stack = RT_STACK_LOCAL;
+  uint32_t entries = 0, total = 0, refill = 8, stack = 0;  // stack 0: the launch's default (stack_of)
   int uniform = -1;
   rtk::BatchEntry* d_table = nullptr;
   unsigned int* d_counter = nullptr;
@@ -205,7 +205,7 @@ rt_status rt_plan_create(rt_ctx* ctx, const rt_scene* scene, const rt_batch* h_b
   p->h_table = table;
   p->refill = desc->refill ? desc->refill
                            : (desc->kernel == RT_KERNEL_FAST ? ctx->tuning.fast_refill : ctx->tuning.wide8_refill);
-  p->stack = desc->stack ? desc->stack : ctx->tuning.wide8_stack;
+  p->stack = desc->stack ? desc->stack : chosen_stack(ctx);
   if (desc->kernel == RT_KERNEL_WIDE8 && p->stack == RT_STACK_SHARED && !rtl::shared_stack_fits(view_of(scene))) {
     const uint32_t depth = scene->w8_depth;
     delete p;

@@ -40,12 +40,12 @@ rt_status dispatch(rt_ctx* ctx, const rt_scene* scene, rt_mode mode, rt_kernel k
     case RT_KERNEL_WIDE8:
       if (!scene->d_wide8)
         return fail(ctx, RT_ERR_UNSUPPORTED, "the WIDE8 kernel needs rt_scene_prepare(scene, RT_KERNEL_WIDE8) first");
-      if (ctx->tuning.wide8_stack == RT_STACK_SHARED && !rtl::shared_stack_fits(v))
+      if (chosen_stack(ctx) == RT_STACK_SHARED && !rtl::shared_stack_fits(v))
         return fail(ctx, RT_ERR_UNSUPPORTED, "the shared group stack holds 16 levels; this scene's 8-wide trees have %u",
                     v.w8_depth);
       e = rtl::launch_wide8(v, (uint32_t)mode, r, order, hits, n,
                             ctx->d_counters + (ctx->counter_seq++ % COUNTER_SLOTS), ctx->d_status, stream,
-                            ctx->tuning.wide8_refill, ctx->tuning.wide8_stack == RT_STACK_SHARED ? 1u : 0u);
+                            ctx->tuning.wide8_refill, stack_of(chosen_stack(ctx), v, mode != RT_CLOSEST));
       break;
     case RT_KERNEL_WIDE8_PACKET:
       if (!scene->d_wide8)
@@ -247,7 +247,7 @@ rt_status rt_ctx_set_tuning(rt_ctx* ctx, const rt_tuning* t) {
   if (t->wide8_entries > 1024) return fail(ctx, RT_ERR_INVALID_ARG, "top-level entries per instance are 1-1024");
   if (t->fast_refill) next.fast_refill = t->fast_refill;
   if (t->wide8_refill) next.wide8_refill = t->wide8_refill;
-  if (t->wide8_stack) next.wide8_stack = t->wide8_stack;
+  if (t->wide8_stack) next.wide8_stack = t->wide8_stack, ctx->stack_chosen = true;
   if (t->wide8_entries) next.wide8_entries = t->wide8_entries;
   ctx->tuning = next;
   return RT_OK;
@@ -939,7 +939,7 @@ rt_status rt_trace_gi_lights(rt_ctx* ctx, const rt_scene* scene, rt_kernel kerne
     e = rtl::launch_fast_lights(v, d_cells, n_cells, d_lights, n_lights, d_words, counter, ctx->d_status, st,
                                 ctx->tuning.fast_refill);
   } else {
-    const uint32_t stack = ctx->tuning.wide8_stack == RT_STACK_SHARED && rtl::shared_stack_fits(v) ? 1u : 0u;
+    const uint32_t stack = rtl::shared_stack_fits(v) ? stack_of(chosen_stack(ctx), v, true) : 0u;
     e = rtl::launch_wide8_lights(v, d_cells, n_cells, d_lights, n_lights, d_words, counter, ctx->d_status, st,
                                  ctx->tuning.wide8_refill, stack);
   }

@@ -78,3 +78,35 @@ def test_a_flat_plan_outlives_a_new_top_level(engine):
     finally:
         plan.close()
         scene.release()
+
+
+@pytest.mark.parametrize("layout", [A.LAYOUT_GI, A.LAYOUT_REFLECTION])
+def test_the_default_stack_gives_the_local_stack_results(layout):
+    """Where no placement was set, any-hit launches over a flat scene take the shared stack; the flags
+    are the local stack's through single launches, batches and plans (direct and captured)."""
+    import torch
+    mesh = S.clusters(20_000, stream=S.Stream(8))
+    words = A.pack_scene(layout, [A.Blas(mesh.positions, mesh.indices)], S.identity_instances(1))
+    rays = torch.from_numpy(H.random_rays(30_011, -120.0, 120.0, seed=6, tmax=300.0)).cuda()
+    batches = [(rays[:7], A.ANY_CASTERS), (rays[7:], A.ANY_SKY)]
+    got = {}
+    for stack in ("", "local"):
+        engine = A.Engine(0)
+        if stack:
+            engine.set_tuning(wide8_stack=A.STACKS[stack])
+        scene = engine.upload(layout, words)
+        scene.prepare("wide8")
+        assert scene.wide8_depth() <= 16 and engine.tuning()["wide8_stack"] == A.STACKS["local"]
+        out = [engine.trace(scene, rays, A.ANY_CASTERS, "wide8")] + engine.trace_batches(scene, batches, "wide8")
+        for graph in (False, True):
+            plan = engine.plan(scene, batches, "wide8", graph=graph)
+            plan.launch()
+            torch.cuda.synchronize()
+            out += [h.clone() for h in plan.hits]
+            plan.close()
+        assert engine.stats()["stack_overflows"] == 0
+        got[stack] = out
+        scene.release()
+        engine.close()
+    assert all(torch.equal(a, b) for a, b in zip(got[""], got["local"]))
+    assert any(bool(h.any()) for h in got[""])
