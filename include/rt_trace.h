@@ -227,7 +227,7 @@ rt_status rt_order_rays(rt_ctx* ctx, const rt_scene* scene, const rt_ray* d_rays
  * per BLAS reads its topology synchronously). Every instance of the BLAS sees the change. The
  * instance records and the top level are not touched: when the geometry leaves its records' world
  * boxes, rewrite them with rt_scene_update_records, as the reference refits and re-places its
- * instances. The scene's derived WIDE8 layout is dropped (rt_scene_prepare builds it again). */
+ * instances. Ordered against the scene's other calls as rt_scene_move_instances is. The scene's derived WIDE8 layout is dropped (rt_scene_prepare builds it again). */
 rt_status rt_scene_refit(rt_ctx* ctx, rt_scene* scene, uint32_t instance, const float* d_positions,
                          uint32_t n_positions, const uint32_t* d_indices, uint32_t n_indices, void* stream);
 /* Copies words [first, first + n) of the scene's device buffer to host memory (synchronous). */
@@ -481,8 +481,13 @@ rt_status rt_move_instances_host(rt_layout layout, uint32_t* words, size_t n_wor
 /* The same on an uploaded scene, on the device (records, top-level refit in one launch,
  * the rebuild after 64 refits, scene bounds), with rt_move_instances_host's words bit for bit:
  * the per-frame instance update of the reference (instance_words + instance_bvh::place,
- * src/instance_bvh.rs:162-275) without a host round trip. Host arrays; it reads, on the first
- * call, the top level's topology synchronously. */
+ * src/instance_bvh.rs:162-275) without a host round trip. Host arrays, read before
+ * it returns; on the first call it reads the top level's topology synchronously. Asynchronous on
+ * `stream`, after the default stream's work: every later call of this interface on the scene, on any
+ * stream or none (host buffers, rt_scene_read_words, rt_scene_update_records, rt_scene_prepare,
+ * another move or refit), sees the moved scene without a wait of the caller's. A traversal still
+ * running on another stream than the default one is the caller's to order before it. Not in a stream
+ * capture (RT_ERR_CUDA). */
 rt_status rt_scene_move_instances(rt_ctx* ctx, rt_scene* scene, const rt_instance* instances, uint32_t n,
                                   const float* mesh_boxes, uint32_t n_meshes, void* stream);
 

@@ -114,6 +114,7 @@ rt_status rt_trace_batches(rt_ctx* ctx, const rt_scene* scene, rt_kernel kernel,
   rt_status st = make_table(ctx, scene, kernel, h_batches, n_batches, h, total, uniform);
   if (st != RT_OK || total == 0) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  RT_CUDA(ctx, after_changes(scene, s));
   if (kernel == RT_KERNEL_PLAIN) {
     cudaError_t e = enqueue_plain(scene, h, n_batches, ctx->d_status, s);
     if (e != cudaSuccess) return fail(ctx, RT_ERR_CUDA, "plain batch launch: %s", cudaGetErrorString(e));
@@ -256,6 +257,7 @@ rt_status rt_plan_launch(rt_plan* p, void* stream) {
   rt_ctx* ctx = p->ctx;
   RT_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  RT_CUDA(ctx, after_changes(p->scene, s));
   if (p->exec) {
     RT_CUDA(ctx, cudaGraphLaunch(p->exec, s));
   } else {

@@ -54,6 +54,15 @@ struct rt_scene {
   size_t move_bytes = 0;
   uint32_t* d_top_tree = nullptr;
   uint32_t top_nodes = 0;  // nodes the links cover; 0: not made yet
+
+  // rt_scene_move_instances and rt_scene_refit return with their work queued on the caller's stream
+  // (see after_changes): `changed` is recorded after the last of it, on the stream with the id
+  // `change_stream`; `changes` counts such calls and `settled` is the last of them known to be over.
+  // `legacy` orders a change after the default stream's work.
+  cudaEvent_t changed = nullptr, legacy = nullptr;
+  std::atomic<unsigned long long> change_stream{0};
+  std::atomic<uint64_t> changes{0};
+  mutable std::atomic<uint64_t> settled{0};
 };
 
 struct rt_blas {
@@ -148,6 +157,87 @@ inline rt_status fail(rt_ctx* ctx, rt_status s, const char* fmt, ...) {
     cudaError_t e_ = (call);                                                                   \
     if (e_ != cudaSuccess) return fail(ctx, RT_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); \
   } while (0)
+
+// Event calls about work outside any stream capture, also while this thread captures.
+class OutsideCapture {
+ public:
+  OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+  ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+
+ private:
+  cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
+
+// The host waits for the scene's last move or refit. For the calls that read or write the scene's
+// words by synchronous copies, which wait for no non-blocking stream.
+inline cudaError_t wait_changes(const rt_scene* scene) {
+  const uint64_t n = scene->changes.load(std::memory_order_acquire);
+  if (scene->settled.load(std::memory_order_relaxed) >= n) return cudaSuccess;
+  OutsideCapture guard;
+  const cudaError_t e = cudaEventSynchronize(scene->changed);
+  if (e == cudaSuccess) scene->settled.store(n, std::memory_order_relaxed);
+  return e;
+}
+
+// What is queued on `s` from here on runs after the scene's last move or refit, whichever stream that
+// took: every launch that reads the scene's words is ordered so. A launch being captured runs
+// later, on any stream, so there the host waits. Once the change is known to be over, two loads.
+inline cudaError_t after_changes(const rt_scene* scene, cudaStream_t s) {
+  const uint64_t n = scene->changes.load(std::memory_order_acquire);
+  if (scene->settled.load(std::memory_order_relaxed) >= n) return cudaSuccess;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return wait_changes(scene);
+  }
+  unsigned long long id = 0;
+  cudaError_t e = cudaStreamGetId(s, &id);
+  if (e != cudaSuccess || id == scene->change_stream.load(std::memory_order_relaxed)) return e;
+  OutsideCapture guard;
+  e = cudaEventQuery(scene->changed);
+  if (e == cudaSuccess) scene->settled.store(n, std::memory_order_relaxed);
+  if (e != cudaErrorNotReady) return e;
+  cudaGetLastError();
+  return cudaStreamWaitEvent(s, scene->changed, 0);
+}
+
+// Around the launches that change a scene's words on `s` (the caller holds the context's lock):
+// start() queues them after earlier changes and after the default stream's work (a traversal there
+// that still reads the words), and the end of the scope marks them as the last change, on every
+// return path.
+class Change {
+ public:
+  Change(rt_scene* scene, cudaStream_t s) : scene_(scene), s_(s) {}
+  Change(const Change&) = delete;
+  Change& operator=(const Change&) = delete;
+  cudaError_t start() {
+    for (cudaEvent_t* ev : {&scene_->changed, &scene_->legacy})
+      if (!*ev) {
+        const cudaError_t e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+        if (e != cudaSuccess) return e;
+      }
+    cudaError_t e = cudaStreamGetId(s_, &id_);
+    if (e == cudaSuccess) e = after_changes(scene_, s_);
+    if (e == cudaSuccess && s_ != nullptr && s_ != cudaStreamLegacy) {
+      e = cudaEventRecord(scene_->legacy, cudaStreamLegacy);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(s_, scene_->legacy, 0);
+    }
+    started_ = e == cudaSuccess;
+    return e;
+  }
+  ~Change() {
+    if (!started_) return;
+    cudaEventRecord(scene_->changed, s_);
+    scene_->change_stream.store(id_, std::memory_order_relaxed);
+    scene_->changes.fetch_add(1, std::memory_order_release);
+  }
+
+ private:
+  rt_scene* scene_;
+  cudaStream_t s_;
+  unsigned long long id_ = 0;
+  bool started_ = false;
+};
 
 inline size_t hit_bytes(uint32_t layout, uint32_t mode) {
   if (mode != 0) return ANY_HIT_BYTES;

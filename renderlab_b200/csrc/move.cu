@@ -208,6 +208,10 @@ extern "C" rt_status rt_scene_move_instances(rt_ctx* ctx, rt_scene* scene, const
   const uint32_t layout = scene->layout;
   std::lock_guard<std::mutex> lock(ctx->mu);
   RT_CUDA(ctx, cudaSetDevice(ctx->device));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  RT_CUDA(ctx, cudaStreamIsCapturing(s, &capture));
+  if (capture != cudaStreamCaptureStatusNone) return fail(ctx, RT_ERR_CUDA, "a move cannot be captured: it reads host arrays");
   const uint32_t* head = scene->head;
   const uint32_t count = head[0];
   if (n != count || (layout == 0 && head[4] > count))  // GI word 4: a see-through tail
@@ -224,6 +228,7 @@ extern "C" rt_status rt_scene_move_instances(rt_ctx* ctx, rt_scene* scene, const
   scene->w8_top_valid = false;  // the instances move: the packed top level until re-prepared
   const size_t need = sizeof(rt_instance) * n + 24 * (size_t)n_meshes;
   if (need > scene->move_bytes) {
+    RT_CUDA(ctx, wait_changes(scene));
     RT_CUDA(ctx, cudaFree(scene->d_move));
     scene->d_move = nullptr;
     scene->device_bytes -= scene->move_bytes;
@@ -237,7 +242,6 @@ extern "C" rt_status rt_scene_move_instances(rt_ctx* ctx, rt_scene* scene, const
     scene->device_bytes += need;
     ctx->scene_bytes += need;
   }
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   rt_instance* d_moved = static_cast<rt_instance*>(scene->d_move);
   float* d_boxes = reinterpret_cast<float*>(d_moved + n);
   const size_t base = layout == 0 ? head[1] : (head[1] & ~3u);
@@ -246,8 +250,11 @@ extern "C" rt_status rt_scene_move_instances(rt_ctx* ctx, rt_scene* scene, const
   if (top && base + span > scene->n_words) return fail(ctx, RT_ERR_LAYOUT, "top level exceeds the scene's words");
   if (layout == 1 && (size_t)head[4] + 8 > scene->n_words) return fail(ctx, RT_ERR_LAYOUT, "scene bounds exceed the words");
   const uint32_t refits = !top ? head[3] : (rebuild ? 0u : head[3] + 1);
-  // one copy, from pageable memory of the scene's own: it is staged before the call returns, whatever
-  // memory the caller's arrays are in
+  Change change(scene, s);
+  RT_CUDA(ctx, change.start());
+  // one copy, from memory of the scene's own, whatever memory the caller's arrays are in; the last
+  // call's copy has to have read it
+  RT_CUDA(ctx, wait_changes(scene));
   scene->move_stage.resize(need);
   std::memcpy(scene->move_stage.data(), instances, sizeof(rt_instance) * n);
   if (n_meshes) std::memcpy(scene->move_stage.data() + sizeof(rt_instance) * n, mesh_boxes, 24 * (size_t)n_meshes);

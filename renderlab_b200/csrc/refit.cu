@@ -50,6 +50,7 @@ rt_status levels_of(rt_ctx* ctx, rt_scene* scene, const uint32_t* rec, RefitLeve
   if (root & LEAF) return RT_OK;  // a single leaf: nothing to refit
   const uint32_t n = root + 1;    // postorder: the root is the last node
   std::vector<uint32_t> w(16 * (size_t)n);
+  RT_CUDA(ctx, wait_changes(scene));
   RT_CUDA(ctx, cudaMemcpy(w.data(), scene->d_words + nodes, w.size() * 4, cudaMemcpyDeviceToHost));
   uint32_t tris = 0;
   for (uint32_t k = 0; k < n; ++k) {
@@ -109,8 +110,14 @@ rt_status rt_scene_refit(rt_ctx* ctx, rt_scene* scene, uint32_t instance, const 
   if (!gi && !d_indices) return fail(ctx, RT_ERR_INVALID_ARG, "the reflection layout refits from the triangle list");
   std::lock_guard<std::mutex> lock(ctx->mu);
   RT_CUDA(ctx, cudaSetDevice(ctx->device));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  RT_CUDA(ctx, cudaStreamIsCapturing(s, &capture));
   uint32_t rec[24] = {};
   std::copy_n(scene->blas_words.begin() + 6 * (size_t)instance, 6, rec + 18);
+  if (capture != cudaStreamCaptureStatusNone)  // refused where the capture allows no synchronous call
+    RT_CUDA(ctx, cudaMemcpy(rec, scene->d_words + (gi ? 16 + 32 * (size_t)instance : 8 + 24 * (size_t)instance), sizeof rec,
+                            cudaMemcpyDeviceToHost));
   const uint32_t base = gi ? rec[18] : (rec[18] & ~3u);
   auto it = scene->refit.find(base);
   if (it == scene->refit.end()) {
@@ -131,7 +138,8 @@ rt_status rt_scene_refit(rt_ctx* ctx, rt_scene* scene, uint32_t instance, const 
     ctx->scene_bytes -= scene->wide8_bytes;
     scene->wide8_bytes = 0;
   }
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  Change change(scene, s);
+  if (capture == cudaStreamCaptureStatusNone) RT_CUDA(ctx, change.start());  // a captured refit is the replay's caller's to order
   View v{};
   v.w = scene->d_words;
   v.layout = scene->layout;
@@ -159,6 +167,7 @@ rt_status rt_scene_read_words(rt_ctx* ctx, const rt_scene* scene, size_t first, 
   if (!ctx || !scene || (n && !out)) return fail(ctx, RT_ERR_INVALID_ARG, "null argument");
   if (first > scene->n_words || n > scene->n_words - first) return fail(ctx, RT_ERR_INVALID_ARG, "words out of range");
   RT_CUDA(ctx, cudaSetDevice(ctx->device));
+  RT_CUDA(ctx, wait_changes(scene));
   if (n) RT_CUDA(ctx, cudaMemcpy(out, scene->d_words + first, n * 4, cudaMemcpyDeviceToHost));
   return RT_OK;
 }

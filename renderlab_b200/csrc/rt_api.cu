@@ -26,7 +26,8 @@ rt_status dispatch(rt_ctx* ctx, const rt_scene* scene, rt_mode mode, rt_kernel k
                    const uint32_t* order, void* hits, uint32_t n, cudaStream_t stream) {
   const rtl::SceneView v = view_of(scene);
   const float4* r = reinterpret_cast<const float4*>(rays);
-  cudaError_t e;
+  cudaError_t e = after_changes(scene, stream);
+  if (e != cudaSuccess) return fail(ctx, RT_ERR_CUDA, "scene changes: %s", cudaGetErrorString(e));
   switch (kernel) {
     case RT_KERNEL_PLAIN:
       if (order) return fail(ctx, RT_ERR_UNSUPPORTED, "the PLAIN kernel takes no ray order");
@@ -317,6 +318,7 @@ rt_status rt_scene_update_records(rt_ctx* ctx, rt_scene* scene, const uint32_t* 
   // Validate the whole buffer as it will be: the new leading words over the old mesh words.
   std::vector<uint32_t> all(scene->n_words);
   RT_CUDA(ctx, cudaSetDevice(ctx->device));
+  RT_CUDA(ctx, wait_changes(scene));
   RT_CUDA(ctx, cudaMemcpy(all.data(), scene->d_words, scene->n_words * 4, cudaMemcpyDeviceToHost));
   // the old records, to tell whether the 8-wide instance table still holds
   const size_t header = scene->layout == 0 ? 16 : 8, stride = scene->layout == 0 ? 32 : 24;
@@ -355,6 +357,7 @@ rt_status rt_scene_prepare(rt_ctx* ctx, rt_scene* scene, rt_kernel kernel) {
   if (scene->d_wide8 && (scene->w8_top_valid || scene->info.top == 0)) return RT_OK;
   std::vector<uint32_t> words(scene->n_words);
   RT_CUDA(ctx, cudaSetDevice(ctx->device));
+  RT_CUDA(ctx, wait_changes(scene));
   RT_CUDA(ctx, cudaMemcpy(words.data(), scene->d_words, scene->n_words * 4, cudaMemcpyDeviceToHost));
   if (scene->d_wide8) return prepare_top(ctx, scene, words);  // the BLASes stand; the instances moved
   rtb::Wide8Scene w8;
@@ -474,6 +477,7 @@ rt_status rt_scene_tune_top(rt_ctx* ctx, rt_scene* scene, const uint32_t* budget
       return fail(ctx, RT_ERR_LAYOUT, "the scene has no finite world box to probe");
   std::vector<uint32_t> words(scene->n_words);
   RT_CUDA(ctx, cudaSetDevice(ctx->device));
+  RT_CUDA(ctx, wait_changes(scene));
   RT_CUDA(ctx, cudaMemcpy(words.data(), scene->d_words, scene->n_words * 4, cudaMemcpyDeviceToHost));
   rtb::Wide8Scene top;
   rt_status s = read_wide8_blas(ctx, scene, words[0], top);
@@ -534,6 +538,9 @@ rt_status rt_scene_tune_top(rt_ctx* ctx, rt_scene* scene, const uint32_t* budget
 rt_status rt_scene_release(rt_ctx* ctx, rt_scene* scene) {
   if (!ctx || !scene) return fail(ctx, RT_ERR_INVALID_ARG, "null argument");
   cudaSetDevice(ctx->device);
+  wait_changes(scene);
+  for (cudaEvent_t e : {scene->changed, scene->legacy})
+    if (e) cudaEventDestroy(e);
   cudaFree(scene->d_words);
   cudaFree(scene->d_wide8);
   cudaFree(scene->d_w8_top);
@@ -577,7 +584,9 @@ rt_status rt_trace_split(rt_ctx* ctx, const rt_scene* scene, rt_mode mode, const
     return fail(ctx, RT_ERR_INVALID_ARG, "hits must be 4-byte aligned");
   const rtk::SplitRays src{rays->d_o, rays->d_d, rays->d_tmin, rays->d_tmax, rays->tmin, rays->tmax, rays->o_stride,
                            rays->d_stride, d_out, clear ? 1u : 0u};
-  const cudaError_t e = rtl::launch_plain_split(view_of(scene), (uint32_t)mode, src, n, ctx->d_status, static_cast<cudaStream_t>(stream));
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  cudaError_t e = after_changes(scene, st);
+  if (e == cudaSuccess) e = rtl::launch_plain_split(view_of(scene), (uint32_t)mode, src, n, ctx->d_status, st);
   if (e != cudaSuccess) return fail(ctx, RT_ERR_CUDA, "traversal launch: %s", cudaGetErrorString(e));
   ctx->rays += n;
   ctx->launches += 1;
@@ -596,6 +605,7 @@ rt_status rt_trace_counted(rt_ctx* ctx, const rt_scene* scene, rt_mode mode, rt_
   unsigned long long* d_cnt = nullptr;
   RT_CUDA(ctx, cudaMalloc(&d_cnt, 8 * sizeof(unsigned long long)));
   cudaError_t e = cudaMemset(d_cnt, 0, 8 * sizeof(unsigned long long));
+  if (e == cudaSuccess) e = after_changes(scene, nullptr);
   if (e == cudaSuccess)
     e = rtl::count_wide8(view_of(scene), (uint32_t)mode, reinterpret_cast<const float4*>(d_rays), d_hits, n,
                          ctx->d_counters + (ctx->counter_seq++ % COUNTER_SLOTS), ctx->d_status, d_cnt, nullptr);
@@ -904,6 +914,7 @@ rt_status rt_trace_gi_cells(rt_ctx* ctx, const rt_scene* scene, rt_mode mode, co
   if (n_cells > (1u << 25)) return fail(ctx, RT_ERR_INVALID_ARG, "at most 2^25 cells a call");
   if (reinterpret_cast<uintptr_t>(d_hits) % 4 != 0) return fail(ctx, RT_ERR_INVALID_ARG, "hits must be 4-byte aligned");
   RT_CUDA(ctx, cudaSetDevice(ctx->device));
+  RT_CUDA(ctx, after_changes(scene, static_cast<cudaStream_t>(stream)));
   cudaError_t e = rtl::launch_fast_cells(view_of(scene), (uint32_t)mode, d_cells, n_cells, (flags & RT_GI_ROTATE) ? 1u : 0u,
                                          d_hits, ctx->d_counters + (ctx->counter_seq++ % COUNTER_SLOTS), ctx->d_status,
                                          static_cast<cudaStream_t>(stream), ctx->tuning.fast_refill);
@@ -934,6 +945,7 @@ rt_status rt_trace_gi_lights(rt_ctx* ctx, const rt_scene* scene, rt_kernel kerne
   const rtl::SceneView v = view_of(scene);
   unsigned int* counter = ctx->d_counters + (ctx->counter_seq++ % COUNTER_SLOTS);
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  RT_CUDA(ctx, after_changes(scene, st));
   cudaError_t e;
   if (kernel == RT_KERNEL_FAST) {
     e = rtl::launch_fast_lights(v, d_cells, n_cells, d_lights, n_lights, d_words, counter, ctx->d_status, st,
