@@ -22,6 +22,9 @@ struct RefitLevels {
   uint32_t tri_count = 0;       // reflection layout: packed triangles of the BLAS
   uint32_t position_count = 0;  // GI layout: position records of the BLAS
   uint32_t* d_tree = nullptr;   // per node: its parent, a counter, and (bytes) its inner children
+  // Instead, where the nodes are not one tree: d_tree holds node ids by height above the leaves, height
+  // h at [level_start[h], level_start[h + 1]).
+  std::vector<uint32_t> level_start;
 };
 
 struct rt_scene {

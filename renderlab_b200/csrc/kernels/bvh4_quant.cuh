@@ -147,7 +147,14 @@ inline __device__ void refit_node(const View& v, uint32_t node, unsigned quad, i
   }
 }
 
-constexpr uint8_t NEVER = 0xff;  // inner children of a node that is not refit
+constexpr uint8_t NEVER = 0xff;  // inner children of a node that the climb does not come to
+
+// Nodes of one height above the leaves, four lanes each.
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK) k_refit_level(View v, const uint32_t* __restrict__ order, uint32_t count) {
+  const uint32_t i = (blockIdx.x * BLOCK + threadIdx.x) / 4;
+  if (i < count) refit_node(v, order[i], 0xfu << (threadIdx.x & 28), threadIdx.x & 3);
+}
 
 // Every node of a BLAS, children before parents, in one launch: four lanes start at each node without
 // inner children (inner[node] == 0) and climb; of a node's inner children, the last one done takes

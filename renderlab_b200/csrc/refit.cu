@@ -42,32 +42,46 @@ __global__ void k_refit_triangles(View v, uint32_t n_tris) {
   }
 }
 
-// The BLAS's topology (once per BLAS): node heights, triangle / position counts.
+// Whether a leaf that no instance's root reaches lies inside the scene's words, as the upload's
+// admission checks those that one does (`words`: the scene's, read for the GI layout alone).
+bool leaf_inside(const rt_scene* scene, const uint32_t* rec, uint32_t c, const std::vector<uint32_t>& words) {
+  const size_t n = scene->n_words;
+  if (scene->layout != 0) return (rec[19] & ~3u) + 12 * ((size_t)((c & ~LEAF) >> 4) + (c & 15u)) <= n;
+  const size_t l = rec[19] + 2 * (size_t)(c & ~LEAF);
+  if (l + 2 > n) return false;
+  const size_t first = rec[21] + (size_t)words[l], count = words[l + 1];
+  if (first + count > n) return false;
+  for (size_t k = first; k < first + count; ++k)
+    if (rec[20] + 3 * (size_t)words[k] + 3 > n) return false;
+  return true;
+}
+
+// The BLAS's topology (once per BLAS): what the refit's launches need, triangle / position counts.
+// Every node up to the highest root that an instance enters the BLAS at is refit, as the host's
+// refit does, reached from a root or not (a file of several levels holds such nodes, and other
+// instances may enter at them).
 rt_status levels_of(rt_ctx* ctx, rt_scene* scene, const uint32_t* rec, RefitLevels& out) {
   const bool gi = scene->layout == 0;
   const size_t nodes = gi ? rec[18] : (rec[18] & ~3u);
-  const uint32_t root = gi ? rec[22] : rec[20];
-  if (root & LEAF) return RT_OK;  // a single leaf: nothing to refit
-  const uint32_t n = root + 1;    // postorder: the root is the last node
+  uint32_t n = 0;
+  for (size_t i = 0; i < scene->info.instances; ++i) {
+    const uint32_t* r = scene->blas_words.data() + 6 * i;
+    const uint32_t root = gi ? r[4] : r[2];
+    if ((gi ? r[0] : (r[0] & ~3u)) == nodes && !(root & LEAF)) n = std::max(n, root + 1);  // postorder: the root is the last node
+  }
+  if ((gi ? rec[22] : rec[20]) & LEAF) return RT_OK;  // a single leaf: nothing to refit
   std::vector<uint32_t> w(16 * (size_t)n);
   RT_CUDA(ctx, wait_changes(scene));
   RT_CUDA(ctx, cudaMemcpy(w.data(), scene->d_words + nodes, w.size() * 4, cudaMemcpyDeviceToHost));
-  uint32_t tris = 0;
-  for (uint32_t k = 0; k < n; ++k) {
+  for (uint32_t k = 0; k < n; ++k)
     for (int s = 0; s < 4; ++s) {
       const uint32_t c = w[16 * (size_t)k + 6 + s];
-      if (c == EMPTY) continue;
-      if (c & LEAF) {
-        if (!gi) tris = std::max(tris, ((c & ~LEAF) >> 4) + (c & 15u));
-      } else if (c >= k) {
-        return fail(ctx, RT_ERR_LAYOUT, "refit: BLAS children must precede their parent");
-      }
+      if (c != EMPTY && !(c & LEAF) && c >= k) return fail(ctx, RT_ERR_LAYOUT, "refit: BLAS children must precede their parent");
     }
-  }
-  // the tree from the root: each node's parent and inner children (a node it does not reach is left)
+  // the tree from the last root: each node's parent and inner children
   std::vector<uint32_t> parent(n, EMPTY);
   std::vector<uint8_t> inner(n, rtq::NEVER);
-  inner[root] = 0;
+  inner[n - 1] = 0;
   for (uint32_t k = n; k-- > 0;) {
     if (inner[k] == rtq::NEVER) continue;
     for (int s = 0; s < 4; ++s) {
@@ -76,20 +90,52 @@ rt_status levels_of(rt_ctx* ctx, rt_scene* scene, const uint32_t* rec, RefitLeve
       parent[c] = k, inner[c] = 0, ++inner[k];
     }
   }
+  const bool tree = std::find(inner.begin(), inner.end(), rtq::NEVER) == inner.end();
+  std::vector<uint32_t> words, height(tree ? 0 : n, 0), order;
+  if (!tree && gi) {
+    words.resize(scene->n_words);
+    RT_CUDA(ctx, cudaMemcpy(words.data(), scene->d_words, 4 * words.size(), cudaMemcpyDeviceToHost));
+  }
+  uint32_t tris = 0, top = 0;
+  for (uint32_t k = 0; k < n; ++k) {
+    uint32_t h = 1, most = 0;
+    for (int s = 0; s < 4; ++s) {
+      const uint32_t c = w[16 * (size_t)k + 6 + s];
+      if (c == EMPTY) continue;
+      if (c & LEAF) {
+        if (!gi) most = std::max(most, ((c & ~LEAF) >> 4) + (c & 15u));
+        if (!tree && inner[k] == rtq::NEVER && !leaf_inside(scene, rec, c, words)) h = 0;
+      } else if (!tree) {
+        h = h && height[c] ? std::max(h, height[c] + 1) : 0;
+      }
+    }
+    if (h == 0) continue;  // leaves outside the words below it: no ray enters here, and it stays as it is
+    tris = std::max(tris, most);
+    if (!tree) height[k] = h, top = std::max(top, h);
+  }
   out.node_count = n;
   out.tri_count = tris;
   if (gi) {  // the packer lays a mesh's positions (3 words each) right before its indices
     if (rec[21] < rec[20] || (rec[21] - rec[20]) % 3 != 0) return fail(ctx, RT_ERR_LAYOUT, "refit: GI position words");
     out.position_count = (rec[21] - rec[20]) / 3;
   }
-  // one allocation: parents, counters of a launch, inner child counts
-  if (cudaMalloc(&out.d_tree, 9 * (size_t)n) != cudaSuccess) {
+  if (!tree) {
+    out.level_start.assign(1, 0);
+    for (uint32_t h = 1; h <= top; ++h) {
+      for (uint32_t k = 0; k < n; ++k)
+        if (height[k] == h) order.push_back(k);
+      out.level_start.push_back((uint32_t)order.size());
+    }
+  }
+  // one allocation: parents, counters of a launch, inner child counts; or the order
+  if (cudaMalloc(&out.d_tree, tree ? 9 * (size_t)n : 4 * std::max<size_t>(order.size(), 1)) != cudaSuccess) {
     cudaGetLastError();
     out.d_tree = nullptr;
     return fail(ctx, RT_ERR_OOM, "refit tree");
   }
-  cudaError_t e = cudaMemcpy(out.d_tree, parent.data(), 4 * (size_t)n, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(out.d_tree + 2 * (size_t)n, inner.data(), n, cudaMemcpyHostToDevice);
+  cudaError_t e = tree ? cudaMemcpy(out.d_tree, parent.data(), 4 * (size_t)n, cudaMemcpyHostToDevice)
+                       : cudaMemcpy(out.d_tree, order.data(), 4 * order.size(), cudaMemcpyHostToDevice);
+  if (tree && e == cudaSuccess) e = cudaMemcpy(out.d_tree + 2 * (size_t)n, inner.data(), n, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cudaFree(out.d_tree);
     out.d_tree = nullptr;
@@ -153,10 +199,15 @@ rt_status rt_scene_refit(rt_ctx* ctx, rt_scene* scene, uint32_t instance, const 
     if (lv.tri_count) k_refit_triangles<<<(lv.tri_count + 255) / 256, 256, 0, s>>>(v, lv.tri_count);
   }
   RT_CUDA(ctx, cudaGetLastError());
-  if (lv.node_count) {
+  const auto blocks = [](uint64_t nodes) { return (uint32_t)((4 * nodes + REFIT_BLOCK - 1) / REFIT_BLOCK); };
+  for (size_t h = 0; h + 1 < lv.level_start.size(); ++h) {
+    const uint32_t first = lv.level_start[h], n = lv.level_start[h + 1] - first;
+    if (n) k_refit_level<REFIT_BLOCK><<<blocks(n), REFIT_BLOCK, 0, s>>>(v, lv.d_tree + first, n);
+  }
+  if (lv.node_count && lv.level_start.empty()) {
     const uint32_t n = lv.node_count;
     RT_CUDA(ctx, cudaMemsetAsync(lv.d_tree + n, 0, 4 * (size_t)n, s));
-    k_refit_up<REFIT_BLOCK><<<(uint32_t)((4 * (uint64_t)n + REFIT_BLOCK - 1) / REFIT_BLOCK), REFIT_BLOCK, 0, s>>>(
+    k_refit_up<REFIT_BLOCK><<<blocks(n), REFIT_BLOCK, 0, s>>>(
         v, n, lv.d_tree, reinterpret_cast<const uint8_t*>(lv.d_tree + 2 * (size_t)n), lv.d_tree + n);
   }
   RT_CUDA(ctx, cudaGetLastError());

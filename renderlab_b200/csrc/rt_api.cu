@@ -344,7 +344,12 @@ rt_status rt_scene_update_records(rt_ctx* ctx, rt_scene* scene, const uint32_t* 
     scene->d_top_tree = nullptr, scene->top_nodes = 0;
   }
   scene->info = info;
+  const std::vector<uint32_t> blas = scene->blas_words;
   keep_records(scene, all.data(), all.size());
+  if (blas != scene->blas_words) {  // other roots or BLASes: the refits' topology is read again
+    for (auto& kv : scene->refit) cudaFree(kv.second.d_tree);
+    scene->refit.clear();
+  }
   scene->w8_top_valid = false;  // the instances' boxes may have moved: the packed top level until re-prepared
   return RT_OK;
 }
