@@ -63,13 +63,21 @@ bool leaf_inside(const rt_scene* scene, const uint32_t* rec, uint32_t c, const s
 rt_status levels_of(rt_ctx* ctx, rt_scene* scene, const uint32_t* rec, RefitLevels& out) {
   const bool gi = scene->layout == 0;
   const size_t nodes = gi ? rec[18] : (rec[18] & ~3u);
-  uint32_t n = 0;
+  uint32_t n = 0, tris = 0;
   for (size_t i = 0; i < scene->info.instances; ++i) {
     const uint32_t* r = scene->blas_words.data() + 6 * i;
     const uint32_t root = gi ? r[4] : r[2];
-    if ((gi ? r[0] : (r[0] & ~3u)) == nodes && !(root & LEAF)) n = std::max(n, root + 1);  // postorder: the root is the last node
+    if ((gi ? r[0] : (r[0] & ~3u)) != nodes || root == EMPTY) continue;
+    if (!(root & LEAF)) n = std::max(n, root + 1);  // postorder: the root is the last node
+    else if (!gi) tris = std::max(tris, ((root & ~LEAF) >> 4) + (root & 15u));  // a single leaf: its triangles alone
   }
-  if ((gi ? rec[22] : rec[20]) & LEAF) return RT_OK;  // a single leaf: nothing to refit
+  out.node_count = n;
+  out.tri_count = tris;
+  if (gi) {  // the packer lays a mesh's positions (3 words each) right before its indices
+    if (rec[21] < rec[20] || (rec[21] - rec[20]) % 3 != 0) return fail(ctx, RT_ERR_LAYOUT, "refit: GI position words");
+    out.position_count = (rec[21] - rec[20]) / 3;
+  }
+  if (n == 0) return RT_OK;
   std::vector<uint32_t> w(16 * (size_t)n);
   RT_CUDA(ctx, wait_changes(scene));
   RT_CUDA(ctx, cudaMemcpy(w.data(), scene->d_words + nodes, w.size() * 4, cudaMemcpyDeviceToHost));
@@ -96,7 +104,7 @@ rt_status levels_of(rt_ctx* ctx, rt_scene* scene, const uint32_t* rec, RefitLeve
     words.resize(scene->n_words);
     RT_CUDA(ctx, cudaMemcpy(words.data(), scene->d_words, 4 * words.size(), cudaMemcpyDeviceToHost));
   }
-  uint32_t tris = 0, top = 0;
+  uint32_t top = 0;
   for (uint32_t k = 0; k < n; ++k) {
     uint32_t h = 1, most = 0;
     for (int s = 0; s < 4; ++s) {
@@ -113,12 +121,7 @@ rt_status levels_of(rt_ctx* ctx, rt_scene* scene, const uint32_t* rec, RefitLeve
     tris = std::max(tris, most);
     if (!tree) height[k] = h, top = std::max(top, h);
   }
-  out.node_count = n;
   out.tri_count = tris;
-  if (gi) {  // the packer lays a mesh's positions (3 words each) right before its indices
-    if (rec[21] < rec[20] || (rec[21] - rec[20]) % 3 != 0) return fail(ctx, RT_ERR_LAYOUT, "refit: GI position words");
-    out.position_count = (rec[21] - rec[20]) / 3;
-  }
   if (!tree) {
     out.level_start.assign(1, 0);
     for (uint32_t h = 1; h <= top; ++h) {
