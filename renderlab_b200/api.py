@@ -896,6 +896,8 @@ def _seam(engine: Engine, scene: Scene, origin, direction, tmin, tmax, mode: int
     for x in (origin, direction):
         if type(x) is not torch.Tensor or not x.is_cuda or x.dtype != torch.float32 or x.dim() != 2 or x.shape[1] != 3:
             return None
+        if x.is_neg():  # the memory holds the negated values
+            return None
     n, device = origin.shape[0], origin.device
     strides = origin.stride(), direction.stride()
     if n == 0 or direction.shape[0] != n or direction.device != device:
@@ -909,7 +911,7 @@ def _seam(engine: Engine, scene: Scene, origin, direction, tmin, tmax, mode: int
                 return None
             ranges.append((None, x))
         elif (type(x) is torch.Tensor and x.is_cuda and x.dtype == torch.float32 and x.dim() == 1 and x.shape[0] == n
-              and x.device == device and x.is_contiguous()):
+              and x.device == device and x.is_contiguous() and not x.is_neg()):
             ranges.append((x.data_ptr(), 0.0))
         else:
             return None
