@@ -836,7 +836,10 @@ __global__ void __launch_bounds__(BLOCK, W8_BLOCKS) k_wide8(const uint32_t* __re
       L.flat = 0;
       L.tsp = 0;
       if (top8) {  // the root as a group of one: slot 0 of an all-inner group at node 0
-        tstack[0] = 0, tstack[1] = (1u << octant_of(L.ray.d)) | 0xffu << 8, L.tsp = 2;
+        tstack[0] = 0, tstack[1] = (1u << octant_of(L.ray.d)) | 0xffu << 8;
+        // nothing lies in a range with a NaN, but w8_box_hits takes a NaN difference for a hit: a ray of
+        // NaN alone would walk every instance (from a list or a packed top level it enters none)
+        L.tsp = isnan(L.ray.tmin) || isnan(L.ray.tmax) ? 0 : 2;
       } else if (top != 0 && count != 0) {
         tstack[L.tsp++] = root;
       }
