@@ -56,6 +56,7 @@ struct rt_scene {
   void* d_move = nullptr;
   size_t move_bytes = 0;
   uint32_t* d_top_tree = nullptr;
+  size_t top_cap = 0;      // nodes d_top_tree has room for
   uint32_t top_nodes = 0;  // nodes the links cover; 0: not made yet
 
   // rt_scene_move_instances and rt_scene_refit return with their work queued on the caller's stream

@@ -67,9 +67,8 @@ __device__ Box instance_box(uint32_t layout, const float* m, const float* obj) {
 }
 
 __global__ void k_move_records(uint32_t* __restrict__ w, uint32_t layout, const rt_instance* __restrict__ moved, uint32_t n,
-                               const float* __restrict__ mesh_boxes, uint32_t refits) {
+                               const float* __restrict__ mesh_boxes) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) w[3] = refits;
   if (i >= n) return;
   const rt_instance& g = moved[i];
   uint32_t* r = w + (layout == 0 ? 16 + 32 * (size_t)i : 8 + 24 * (size_t)i);
@@ -84,12 +83,14 @@ constexpr uint8_t NEVER = 0xff;  // inner children of a node that is not refit
 // from the nodes without inner children; of a node's inner children the last one done takes the
 // node (done[], zeroed before the launch; nothing waits). An inner child's box is grown in slot order
 // as instance_bvh::refit_wide does. 2,500 instances, 6 heights: 40 us as a launch per height with a
-// thread a node, 16 so (the whole call, its copies included: 144 -> 62 us).
+// thread a node, 16 so (the whole call, its copies included: 144 -> 62 us). `refits`: the header's count.
 constexpr int TOP_BLOCK = 128;
 __global__ void __launch_bounds__(TOP_BLOCK) k_refit_top(uint32_t* __restrict__ w, uint32_t layout, size_t base, uint32_t n,
                                                          const uint32_t* __restrict__ parent,
-                                                         const uint8_t* __restrict__ inner, uint32_t* __restrict__ done) {
+                                                         const uint8_t* __restrict__ inner, uint32_t* __restrict__ done,
+                                                         uint32_t refits) {
   const uint32_t i = (blockIdx.x * TOP_BLOCK + threadIdx.x) / 4;
+  if (blockIdx.x == 0 && threadIdx.x == 0) w[3] = refits;
   if (i >= n || inner[i] != 0) return;
   const int c = threadIdx.x & 3;
   const unsigned quad = 0xfu << (threadIdx.x & 28);
@@ -131,10 +132,13 @@ __global__ void __launch_bounds__(TOP_BLOCK) k_refit_top(uint32_t* __restrict__ 
   }
 }
 
-// Parents and inner child counts of a tree built on the device (nodes 0 to n - 1, the root first).
-__global__ void k_top_links(const uint32_t* __restrict__ nodes, uint32_t n, uint32_t* __restrict__ parent,
+// Parents and inner child counts of a tree built on the device (nodes 0 to n - 1, the root first), and the
+// header's refit count, 0 from here.
+__global__ void k_top_links(uint32_t* __restrict__ w, size_t base, uint32_t n, uint32_t* __restrict__ parent,
                             uint8_t* __restrict__ inner) {
+  const uint32_t* nodes = w + base;
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) w[3] = 0;
   if (i >= n) return;
   uint32_t kids = 0;
   for (int c = 0; c < 4; ++c) {
@@ -180,23 +184,27 @@ __global__ void __launch_bounds__(BOUNDS_THREADS) k_scene_bounds(uint32_t* __res
 }
 
 // Parents and inner child counts of the top level's nodes reachable from the root (the reserve may
-// hold unused space: NEVER); false when a node names a child outside it.
-bool top_links(const std::vector<uint32_t>& nodes, std::vector<uint32_t>& parent, std::vector<uint8_t>& inner) {
+// hold unused space: NEVER). Returns how many nodes it has to see: at most those given when it is done.
+size_t top_links(const std::vector<uint32_t>& nodes, std::vector<uint32_t>& parent, std::vector<uint8_t>& inner) {
   const size_t nn = nodes.size() / TOP_WORDS;
+  size_t need = nn;
   parent.assign(nn, EMPTY);
   inner.assign(nn, NEVER);
-  if (nn == 0) return true;
   inner[0] = 0;
   for (size_t i = 0; i < nn; ++i) {  // children follow their parents
     if (inner[i] == NEVER) continue;
     for (int c = 0; c < 4; ++c) {
       const uint32_t id = nodes[i * TOP_WORDS + 24 + c];
       if (id == EMPTY || (id & LEAF)) continue;
-      if (id >= nn || id <= i) return false;
+      if (id >= nn) {
+        need = std::max<size_t>(need, (size_t)id + 1);
+        continue;
+      }
+      if (id <= i || inner[id] != NEVER) continue;  // words that are no tree from node 0: the child's box as it stands
       parent[id] = (uint32_t)i, inner[id] = 0, ++inner[i];
     }
   }
-  return true;
+  return need;
 }
 
 }  // namespace
@@ -225,7 +233,13 @@ extern "C" rt_status rt_scene_move_instances(rt_ctx* ctx, rt_scene* scene, const
     if (rtb::is_singular(p)) return fail(ctx, RT_ERR_LAYOUT, "instance %u: singular placement", i);
   }
   if (n == 0) return RT_OK;
-  scene->w8_top_valid = false;  // the instances move: the packed top level until re-prepared
+  // All that can be refused or fail comes before the first launch, and the refit count is written where
+  // the refit or the rebuild is: a call that fails in between leaves the count as it was.
+  const size_t base = layout == 0 ? head[1] : (head[1] & ~3u);
+  const bool top = head[1] != 0 && count >= 2, rebuild = top && head[3] >= rtb::TLAS_REFITS;
+  const size_t span = top ? rtb::tlas_reserve(count) : 0;
+  if (top && base + span > scene->n_words) return fail(ctx, RT_ERR_LAYOUT, "top level exceeds the scene's words");
+  if (layout == 1 && (size_t)head[4] + 8 > scene->n_words) return fail(ctx, RT_ERR_LAYOUT, "scene bounds exceed the words");
   const size_t need = sizeof(rt_instance) * n + 24 * (size_t)n_meshes;
   if (need > scene->move_bytes) {
     RT_CUDA(ctx, wait_changes(scene));
@@ -242,14 +256,42 @@ extern "C" rt_status rt_scene_move_instances(rt_ctx* ctx, rt_scene* scene, const
     scene->device_bytes += need;
     ctx->scene_bytes += need;
   }
+  // the top level's links, per node its parent, a counter, and (bytes) its inner children; the tree's
+  // topology is read once (a rebuild keeps its own)
+  std::vector<uint32_t> nodes, up;
+  std::vector<uint8_t> kids;
+  if (top && (scene->top_nodes == 0 || rebuild)) {
+    size_t cap = span / TOP_WORDS;  // a rebuild's most
+    if (!rebuild) {
+      RT_CUDA(ctx, wait_changes(scene));
+      for (size_t seen = 0; seen < cap;) {
+        seen = cap;
+        nodes.resize(cap * TOP_WORDS);
+        RT_CUDA(ctx, cudaMemcpy(nodes.data(), scene->d_words + base, 4 * nodes.size(), cudaMemcpyDeviceToHost));
+        cap = std::min(top_links(nodes, up, kids), (scene->n_words - base) / TOP_WORDS);
+      }
+    }
+    if (cap > scene->top_cap) {
+      RT_CUDA(ctx, wait_changes(scene));
+      RT_CUDA(ctx, cudaFree(scene->d_top_tree));
+      scene->d_top_tree = nullptr, scene->top_cap = 0, scene->top_nodes = 0;
+      if (cudaMalloc(&scene->d_top_tree, 9 * cap) != cudaSuccess) {
+        cudaGetLastError();
+        scene->d_top_tree = nullptr;
+        return fail(ctx, RT_ERR_OOM, "top-level links");
+      }
+      scene->top_cap = cap;
+    }
+  }
+  uint32_t *parent = scene->d_top_tree, *done = parent + scene->top_cap;
+  uint8_t* inner = reinterpret_cast<uint8_t*>(done + scene->top_cap);
+  if (!up.empty()) {
+    RT_CUDA(ctx, cudaMemcpy(parent, up.data(), 4 * up.size(), cudaMemcpyHostToDevice));
+    RT_CUDA(ctx, cudaMemcpy(inner, kids.data(), kids.size(), cudaMemcpyHostToDevice));
+    scene->top_nodes = (uint32_t)up.size();
+  }
   rt_instance* d_moved = static_cast<rt_instance*>(scene->d_move);
   float* d_boxes = reinterpret_cast<float*>(d_moved + n);
-  const size_t base = layout == 0 ? head[1] : (head[1] & ~3u);
-  const bool top = head[1] != 0 && count >= 2, rebuild = top && head[3] >= rtb::TLAS_REFITS;
-  const size_t span = top ? rtb::tlas_reserve(count) : 0;
-  if (top && base + span > scene->n_words) return fail(ctx, RT_ERR_LAYOUT, "top level exceeds the scene's words");
-  if (layout == 1 && (size_t)head[4] + 8 > scene->n_words) return fail(ctx, RT_ERR_LAYOUT, "scene bounds exceed the words");
-  const uint32_t refits = !top ? head[3] : (rebuild ? 0u : head[3] + 1);
   Change change(scene, s);
   RT_CUDA(ctx, change.start());
   // one copy, from memory of the scene's own, whatever memory the caller's arrays are in; the last
@@ -258,47 +300,28 @@ extern "C" rt_status rt_scene_move_instances(rt_ctx* ctx, rt_scene* scene, const
   scene->move_stage.resize(need);
   std::memcpy(scene->move_stage.data(), instances, sizeof(rt_instance) * n);
   if (n_meshes) std::memcpy(scene->move_stage.data() + sizeof(rt_instance) * n, mesh_boxes, 24 * (size_t)n_meshes);
+  scene->w8_top_valid = false;  // the instances move: the packed top level until re-prepared
   RT_CUDA(ctx, cudaMemcpyAsync(d_moved, scene->move_stage.data(), need, cudaMemcpyHostToDevice, s));
-  k_move_records<<<(n + 127) / 128, 128, 0, s>>>(scene->d_words, layout, d_moved, n, d_boxes, refits);
+  k_move_records<<<(n + 127) / 128, 128, 0, s>>>(scene->d_words, layout, d_moved, n, d_boxes);
   RT_CUDA(ctx, cudaGetLastError());
-  scene->head[3] = refits;
-  if (top) {
-    // per node: its parent, a counter, and (bytes) its inner children; span / TOP_WORDS nodes at most
-    const size_t cap = span / TOP_WORDS;
-    if (!scene->d_top_tree && cudaMalloc(&scene->d_top_tree, 9 * cap) != cudaSuccess) {
-      cudaGetLastError();
-      scene->d_top_tree = nullptr;
-      return fail(ctx, RT_ERR_OOM, "top-level links");
-    }
-    uint32_t *parent = scene->d_top_tree, *done = parent + cap;
-    uint8_t* inner = reinterpret_cast<uint8_t*>(done + cap);
-    if (rebuild) {
-      // Rebuilt on the device from the records' new boxes (instance_bvh::place for a moved set).
-      const size_t header = layout == 0 ? 16 : 8, stride = layout == 0 ? 32 : 24;
-      uint32_t n_nodes = 0;
-      scene->top_nodes = 0;
-      const rt_status st = tlas_build_device(ctx, scene->d_words + header + 12, stride, n, true, scene->d_words + base, span,
-                                             &n_nodes, s);
-      if (st != RT_OK) return st;
-      k_top_links<<<(n_nodes + 127) / 128, 128, 0, s>>>(scene->d_words + base, n_nodes, parent, inner);
-      RT_CUDA(ctx, cudaGetLastError());
-      scene->top_nodes = n_nodes;
-    } else {
-      if (scene->top_nodes == 0) {  // the tree's topology, once (a rebuild keeps its own)
-        std::vector<uint32_t> nodes(span), up;
-        std::vector<uint8_t> kids;
-        RT_CUDA(ctx, cudaMemcpyAsync(nodes.data(), scene->d_words + base, 4 * span, cudaMemcpyDeviceToHost, s));
-        RT_CUDA(ctx, cudaStreamSynchronize(s));
-        if (!top_links(nodes, up, kids)) return fail(ctx, RT_ERR_LAYOUT, "move: top-level children out of order");
-        RT_CUDA(ctx, cudaMemcpy(parent, up.data(), 4 * up.size(), cudaMemcpyHostToDevice));
-        RT_CUDA(ctx, cudaMemcpy(inner, kids.data(), kids.size(), cudaMemcpyHostToDevice));
-        scene->top_nodes = (uint32_t)up.size();
-      }
-      RT_CUDA(ctx, cudaMemsetAsync(done, 0, 4 * cap, s));
-      k_refit_top<<<(4 * scene->top_nodes + TOP_BLOCK - 1) / TOP_BLOCK, TOP_BLOCK, 0, s>>>(
-          scene->d_words, layout, base, scene->top_nodes, parent, inner, done);
-      RT_CUDA(ctx, cudaGetLastError());
-    }
+  if (rebuild) {
+    // Rebuilt on the device from the records' new boxes (instance_bvh::place for a moved set).
+    const size_t header = layout == 0 ? 16 : 8, stride = layout == 0 ? 32 : 24;
+    uint32_t n_nodes = 0;
+    scene->top_nodes = 0;
+    const rt_status st = tlas_build_device(ctx, scene->d_words + header + 12, stride, n, true, scene->d_words + base, span,
+                                           &n_nodes, s);
+    if (st != RT_OK) return st;
+    k_top_links<<<(n_nodes + 127) / 128, 128, 0, s>>>(scene->d_words, base, n_nodes, parent, inner);
+    RT_CUDA(ctx, cudaGetLastError());
+    scene->head[3] = 0;
+    scene->top_nodes = n_nodes;
+  } else if (top) {
+    RT_CUDA(ctx, cudaMemsetAsync(done, 0, 4 * (size_t)scene->top_nodes, s));
+    k_refit_top<<<(4 * scene->top_nodes + TOP_BLOCK - 1) / TOP_BLOCK, TOP_BLOCK, 0, s>>>(
+        scene->d_words, layout, base, scene->top_nodes, parent, inner, done, scene->head[3] + 1);
+    RT_CUDA(ctx, cudaGetLastError());
+    scene->head[3] += 1;
   }
   if (layout == 1) {
     k_scene_bounds<<<1, BOUNDS_THREADS, 0, s>>>(scene->d_words, n);

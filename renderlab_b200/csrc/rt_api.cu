@@ -339,10 +339,7 @@ rt_status rt_scene_update_records(rt_ctx* ctx, rt_scene* scene, const uint32_t* 
   // records that name other BLASes, or another instance count, void the 8-wide instance table
   if (scene->d_wide8 && !same_instances(scene->layout, before.data(), all.data())) drop_wide8(ctx, scene);
   RT_CUDA(ctx, cudaMemcpy(scene->d_words, words, n_words * 4, cudaMemcpyHostToDevice));
-  if (!same_top) {
-    cudaFree(scene->d_top_tree);
-    scene->d_top_tree = nullptr, scene->top_nodes = 0;
-  }
+  if (!same_top) scene->top_nodes = 0;
   scene->info = info;
   const std::vector<uint32_t> blas = scene->blas_words;
   keep_records(scene, all.data(), all.size());
