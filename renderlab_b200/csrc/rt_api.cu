@@ -315,6 +315,7 @@ rt_status rt_scene_validate(rt_layout layout, const uint32_t* words, size_t n_wo
 rt_status rt_scene_update_records(rt_ctx* ctx, rt_scene* scene, const uint32_t* words, size_t n_words) {
   if (!ctx || !scene || !words) return fail(ctx, RT_ERR_INVALID_ARG, "null argument");
   if (n_words > scene->n_words) return fail(ctx, RT_ERR_INVALID_ARG, "record words exceed the scene");
+  std::lock_guard<std::mutex> lock(ctx->mu);  // moves and refits read what this rewrites under it
   // Validate the whole buffer as it will be: the new leading words over the old mesh words.
   std::vector<uint32_t> all(scene->n_words);
   RT_CUDA(ctx, cudaSetDevice(ctx->device));
