@@ -122,11 +122,14 @@ RT_DEV F3 unit_normal(F3 n) {
   return {mul(s.x, k), mul(s.y, k), mul(s.z, k)};
 }
 
-// The closest hit so far: the record's identity words and normal are made once, when the ray ends.
+// The closest hit so far: the record's identity words and normal are made once, when the ray ends. The
+// triangle is kept as a place in its mesh's index list (at most 2^32 - 1 long), not as a word of the
+// buffer, which may lie past 2^32: 64 bits for it cost FAST's closest hits 1.5 % (1M GI rays over 250k
+// triangles 1,087 us against 1,064).
 struct GiNear {
   float t, u, v;
   uint32_t inst;  // EMPTY: none
-  uint32_t at;    // word of the triangle's three indices
+  uint32_t at;    // the triangle's first index, in the mesh's list
 };
 RT_DEV float gi_limit(const GiNear& b, uint32_t i) { return (b.inst != EMPTY && i < b.inst) ? next_up(b.t) : b.t; }
 
@@ -161,7 +164,8 @@ RT_DEV void gi_finish(const uint32_t* __restrict__ w, const GiLane<AM>& L, const
   if (b.inst != EMPTY) {
     const size_t r = 16 + (size_t)b.inst * 32;
     const uint32_t positions = ld(w, r + 20), indices = ld(w, r + 21), prim_base = ld(w, r + 28);
-    tri[0] = ld(w, b.at), tri[1] = ld(w, (size_t)b.at + 1), tri[2] = ld(w, (size_t)b.at + 2);
+    const size_t x = (size_t)indices + b.at;
+    tri[0] = ld(w, x), tri[1] = ld(w, x + 1), tri[2] = ld(w, x + 2);
     const F3 a = ld3(w, positions + (size_t)tri[0] * 3), bb = ld3(w, positions + (size_t)tri[1] * 3),
              c = ld3(w, positions + (size_t)tri[2] * 3);
     const F3 cr = cross3(sub3(bb, a), sub3(c, a));
@@ -169,7 +173,7 @@ RT_DEV void gi_finish(const uint32_t* __restrict__ w, const GiLane<AM>& L, const
     n = unit_normal({add(add(mul(__uint_as_float(q0.x), cr.x), mul(__uint_as_float(q1.x), cr.y)), mul(__uint_as_float(q2.x), cr.z)),
                      add(add(mul(__uint_as_float(q0.y), cr.x), mul(__uint_as_float(q1.y), cr.y)), mul(__uint_as_float(q2.y), cr.z)),
                      add(add(mul(__uint_as_float(q0.z), cr.x), mul(__uint_as_float(q1.z), cr.y)), mul(__uint_as_float(q2.z), cr.z))});
-    if (prim_base != 0) tri[0] = ld(w, prim_base + (b.at - indices) / 3), tri[1] = 0, tri[2] = 0;
+    if (prim_base != 0) tri[0] = ld(w, (size_t)prim_base + b.at / 3), tri[1] = 0, tri[2] = 0;
   }
   o[0] = __float_as_uint(b.t), o[1] = b.inst, o[2] = tri[0], o[3] = tri[1], o[4] = tri[2];
   o[5] = __float_as_uint(b.u), o[6] = __float_as_uint(b.v);
@@ -204,9 +208,9 @@ RT_DEV bool gi_leaf(const uint32_t* __restrict__ w, GiLane<AM>& L, uint32_t chil
   const uint32_t first = ld(w, l), count = ld(w, l + 1);
   const uint32_t i = L.inst;
   for (uint32_t k = 0; k < count; k += 6) {
-    const uint32_t x = L.indices + first + k;
+    const size_t x = (size_t)L.indices + first + k;  // past 2^32 where a buffer's last mesh crosses it
     const bool two = k + 3 < count;
-    const uint32_t y = two ? x + 3 : x;
+    const size_t y = two ? x + 3 : x;
     const uint32_t ia = ld(w, x), ib = ld(w, x + 1), ic = ld(w, x + 2);
     const uint32_t ja = ld(w, y), jb = ld(w, y + 1), jc = ld(w, y + 2);
     const F3 a = ld3(w, L.positions + (size_t)ia * 3), b = ld3(w, L.positions + (size_t)ib * 3),
@@ -215,11 +219,11 @@ RT_DEV bool gi_leaf(const uint32_t* __restrict__ w, GiLane<AM>& L, uint32_t chil
              c2 = ld3(w, L.positions + (size_t)jc * 3);
     float t, u, v;
     if (gi_triangle(L.o, L.d, a, b, c, L.ray.tmin, gi_limit(L.best, i), t, u, v)) {
-      L.best = GiNear{t, u, v, i, x};
+      L.best = GiNear{t, u, v, i, first + k};
       if (any_of<AM>(L)) return true;
     }
     if (two && gi_triangle(L.o, L.d, a2, b2, c2, L.ray.tmin, gi_limit(L.best, i), t, u, v)) {
-      L.best = GiNear{t, u, v, i, y};
+      L.best = GiNear{t, u, v, i, first + k + 3};
       if (any_of<AM>(L)) return true;
     }
   }
