@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(TOP_BLOCK) k_refit_top(uint32_t* __restrict__ 
       last = atomicAdd(&done[up], 1u) + 1u == inner[up] ? 1u : 0u;
       __threadfence();
     }
+    __syncwarp(quad);  // what lane 0's fence has made visible, the other lanes may read (a shuffle orders no memory)
     if (!__shfl_sync(quad, last, 0, 4)) return;
     at = up;
   }
