@@ -303,14 +303,31 @@ _INSTANCE_DTYPE = np.dtype([("model", np.float32, 12), ("rows", np.float32, 12),
                             ("casts_shadow", np.uint32), ("near_base", np.uint32), ("extra", np.uint32, 8)])
 
 
+def _array(values):
+    """The values as one array, or None where numpy would not hold each as it is (lists that mix
+    types or lengths, mappings, tensors on a device)."""
+    if isinstance(values, np.ndarray):
+        return values
+    try:
+        a = np.asarray(values)
+    except Exception:
+        return None
+    return a if a.dtype.kind in "iub" or (a.dtype.kind == "f" and not isinstance(values, (list, tuple))) else None
+
+
 def _words32(values, n: int) -> np.ndarray:
-    """The first n values (of any numeric type, truncated) as 32-bit words, as ctypes stores them."""
-    v = np.asarray(values)[:n]
-    if len(v) < n:
-        raise IndexError(f"{len(v)} values for {n} instances")
-    if v.dtype.kind == "f" and not np.isfinite(v).all():
-        raise ValueError("an instance field is not finite")
-    return v if v.dtype == np.uint32 else (v.astype(np.int64) & 0xFFFFFFFF).astype(np.uint32)
+    """The first n values as 32-bit words, as ctypes stores int(value): arrays of numbers at once,
+    anything else value by value."""
+    a = _array(values)
+    if a is not None and a.ndim == 1:
+        if len(a) < n:
+            raise IndexError(f"{len(a)} values for {n} instances")
+        a = a[:n]
+        if a.dtype.kind == "f" and (np.abs(a) < 2.0 ** 62).all():
+            a = a.astype(np.int64)
+        if a.dtype.kind in "iub":
+            return a.astype(np.uint32)
+    return np.array([int(values[i]) & 0xFFFFFFFF for i in range(n)], np.uint32)
 
 
 def _instance_array(layout: int, instances):
@@ -325,12 +342,19 @@ def _instance_array(layout: int, instances):
     extra = getattr(instances, "extra", None)
     rec["mesh"][:n] = _words32(instances.mesh, n)
     rec["slot"][:n] = np.arange(n) if slot is None else _words32(slot, n)
-    rec["casts_shadow"][:n] = 1 if casts is None else _words32(np.asarray(casts).astype(bool), n)
+    if casts is None:
+        rec["casts_shadow"][:n] = 1
+    else:
+        flags = _array(casts)
+        plain = flags is not None and flags.ndim == 1 and len(flags) >= n
+        rec["casts_shadow"][:n] = flags[:n] != 0 if plain else [bool(casts[i]) for i in range(n)]
     if near is not None:
         rec["near_base"][:n] = _words32(near, n)
     if extra is not None:
-        if n:
-            rec["extra"][:n] = np.stack([_words32(extra, n)[:, k] for k in range(8)], axis=1)
+        rows = _array(extra)
+        plain = rows is not None and rows.ndim == 2 and rows.shape[1] >= 8
+        for k in range(8):
+            rec["extra"][:n, k] = _words32(rows[:, k] if plain else [extra[i][k] for i in range(n)], n)
     elif casts is not None and layout == LAYOUT_GI:
         rec["extra"][:n, 3] = 1 - rec["casts_shadow"][:n]
     return (RtInstance * len(rec)).from_buffer(rec), n
