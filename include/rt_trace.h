@@ -383,6 +383,11 @@ typedef struct rt_host_batch {
 rt_status rt_trace_host_batches(rt_ctx* ctx, const rt_scene* scene, const rt_host_batch* batches,
                                 uint32_t n_batches);
 rt_status rt_ctx_reserve(rt_ctx* ctx, uint32_t max_rays);
+/* Gives back the device memory that rt_blas_build_device keeps between builds (two workspaces of at most
+ * 64 MiB each; in no count of rt_get_stats or of a server's) and reports its bytes in *freed (may be
+ * NULL). The library does so itself when a server is made or given a scene and when an allocation
+ * finds no room. */
+rt_status rt_ctx_trim(rt_ctx* ctx, uint64_t* freed);
 /* rt_trace_ex in an instrumented build that counts, over the batch, into counts[8]:
  * rays, top-level nodes, instance box tests, BLAS nodes, leaves, triangles tested, f64
  * re-tests, f64 final refinements (RT_KERNEL_WIDE8; the bit-exact kernels visit exactly what

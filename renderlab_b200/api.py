@@ -106,7 +106,7 @@ class RtTuning(ctypes.Structure):
 EXPORTS = ("rt_abi_version", "rt_ctx_create", "rt_ctx_destroy", "rt_get_last_error", "rt_get_stats",
            "rt_ctx_set_tuning", "rt_ctx_get_tuning",
            "rt_selftest", "rt_scene_upload", "rt_scene_update_records", "rt_scene_release",
-           "rt_scene_device_bytes", "rt_scene_validate", "rt_scene_prepare", "rt_trace", "rt_trace_ex", "rt_trace_split", "rt_trace_host", "rt_trace_host_batches", "rt_ctx_reserve", "rt_trace_counted", "rt_order_rays",
+           "rt_scene_device_bytes", "rt_scene_validate", "rt_scene_prepare", "rt_trace", "rt_trace_ex", "rt_trace_split", "rt_trace_host", "rt_trace_host_batches", "rt_ctx_reserve", "rt_ctx_trim", "rt_trace_counted", "rt_order_rays",
            "rt_trace_batches", "rt_plan_create", "rt_plan_launch", "rt_plan_info", "rt_plan_destroy",
            "rt_scene_refit", "rt_scene_read_words", "rt_scene_tune_top", "rt_gi_cell_rays", "rt_trace_gi_cells", "rt_trace_gi_lights", "rt_server_create", "rt_server_add_scene", "rt_server_remove_scene", "rt_server_submit",
            "rt_server_wait", "rt_server_get_stats", "rt_server_fail_next", "rt_server_destroy",
@@ -159,6 +159,7 @@ def lib() -> ctypes.CDLL:
     L.rt_trace_host.argtypes = [_vp, _vp, ctypes.c_int, ctypes.c_int, _vp, _vp, ctypes.c_uint32]
     L.rt_trace_host_batches.argtypes = [_vp, _vp, ctypes.POINTER(RtHostBatch), ctypes.c_uint32]
     L.rt_ctx_reserve.argtypes = [_vp, ctypes.c_uint32]
+    L.rt_ctx_trim.argtypes = [_vp, ctypes.POINTER(ctypes.c_uint64)]
     L.rt_order_rays.argtypes = [_vp, _vp, _vp, ctypes.c_uint32, ctypes.c_int, _vp, _vp]
     L.rt_trace_batches.argtypes = [_vp, _vp, ctypes.c_int, ctypes.POINTER(RtBatch), ctypes.c_uint32, _vp]
     L.rt_plan_create.argtypes = [_vp, _vp, ctypes.POINTER(RtBatch), ctypes.c_uint32, ctypes.POINTER(RtPlanDesc),
@@ -846,6 +847,12 @@ class Engine:
 
     def reserve(self, max_rays: int):
         self._check(lib().rt_ctx_reserve(self.ctx, max_rays))
+
+    def trim(self) -> int:
+        """rt_ctx_trim: gives back what device builds keep between calls; returns its bytes."""
+        freed = ctypes.c_uint64()
+        self._check(lib().rt_ctx_trim(self.ctx, ctypes.byref(freed)))
+        return int(freed.value)
 
 
 STATIC_MAX_RAYS = 1 << 31

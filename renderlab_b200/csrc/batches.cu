@@ -97,7 +97,7 @@ rt_status rt_trace_batches(rt_ctx* ctx, const rt_scene* scene, rt_kernel kernel,
   RT_CUDA(ctx, cudaSetDevice(ctx->device));
   if (!ctx->h_tables) {
     const size_t bytes = sizeof(rtk::BatchEntry) * RT_MAX_BATCHES * rt_ctx::TABLE_SLOTS;
-    if (cudaMallocHost(&ctx->h_tables, bytes) != cudaSuccess || cudaMalloc(&ctx->d_tables, bytes) != cudaSuccess) {
+    if (cudaMallocHost(&ctx->h_tables, bytes) != cudaSuccess || device_alloc(ctx, &ctx->d_tables, bytes, true) != cudaSuccess) {
       cudaGetLastError();
       cudaFreeHost(ctx->h_tables);
       ctx->h_tables = nullptr;
@@ -220,13 +220,13 @@ rt_status rt_plan_create(rt_ctx* ctx, const rt_scene* scene, const rt_batch* h_b
     return fail(ctx, RT_ERR_OOM, "plan %s (%zu bytes)", what, bytes);
   };
   const size_t table_bytes = sizeof(rtk::BatchEntry) * table.size();
-  if (cudaMalloc(&p->d_table, table_bytes) != cudaSuccess) return oom("batch table", table_bytes);
-  if (cudaMalloc(&p->d_counter, 256) != cudaSuccess) return oom("ray counter", 256);
+  if (device_alloc(ctx, &p->d_table, table_bytes) != cudaSuccess) return oom("batch table", table_bytes);
+  if (device_alloc(ctx, &p->d_counter, 256) != cudaSuccess) return oom("ray counter", 256);
   p->device_bytes = table_bytes + 256;
   if (desc->order != RT_ORDER_NONE && total > 0) {
     p->sort_bytes = rtl::order_scratch_bytes(p->total);
-    if (cudaMalloc(&p->d_order, sizeof(uint32_t) * total) != cudaSuccess) return oom("ray order", 4 * total);
-    if (cudaMalloc(&p->d_sort, p->sort_bytes) != cudaSuccess) return oom("sort scratch", p->sort_bytes);
+    if (device_alloc(ctx, &p->d_order, sizeof(uint32_t) * total) != cudaSuccess) return oom("ray order", 4 * total);
+    if (device_alloc(ctx, &p->d_sort, p->sort_bytes) != cudaSuccess) return oom("sort scratch", p->sort_bytes);
     p->device_bytes += sizeof(uint32_t) * total + p->sort_bytes;
   }
   cudaError_t e = cudaMemcpy(p->d_table, table.data(), table_bytes, cudaMemcpyHostToDevice);

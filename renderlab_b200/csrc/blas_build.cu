@@ -622,7 +622,14 @@ class Arena {
     auto& kept = ctx_->build_space[slot_];
     if (size_ > BUILD_KEEP) {
       own_ = true;
-      return cudaMalloc(&base_, size_);
+      cudaError_t e = cudaMalloc(&base_, size_);
+      if (e == cudaErrorMemoryAllocation && kept.p) {  // without this slot's kept one; the other may be in use
+        cudaGetLastError();
+        cudaFree(kept.p);
+        kept.p = nullptr, kept.bytes = 0;
+        e = cudaMalloc(&base_, size_);
+      }
+      return e;
     }
     if (size_ > kept.bytes) {
       cudaFree(kept.p);

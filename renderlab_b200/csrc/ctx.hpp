@@ -84,7 +84,8 @@ struct rt_rnf {
 #define RT_HOST_STAGES 4
 #endif
 
-// Bytes of each BLAS build workspace that a context keeps (meshes of about 300k triangles).
+// Bytes of each BLAS build workspace that a context keeps (meshes of about 300k triangles) until
+// rt_ctx_trim, a server on the context, an allocation that finds no room, or its end.
 constexpr size_t BUILD_KEEP = 64u << 20;
 
 struct rt_ctx {
@@ -242,6 +243,31 @@ class Change {
   unsigned long long id_ = 0;
   bool started_ = false;
 };
+
+// Gives the kept build workspaces back (no build runs: the caller holds the context's lock, as a build
+// does throughout). Returns their bytes.
+inline size_t drop_build_space(rt_ctx* ctx) {
+  size_t bytes = 0;
+  for (auto& b : ctx->build_space) {
+    cudaFree(b.p);
+    bytes += b.bytes;
+    b.p = nullptr, b.bytes = 0;
+  }
+  return bytes;
+}
+
+// cudaMalloc for what a caller asks for: where the device has no room, again without the kept build
+// workspaces. `held`: the caller holds the context's lock.
+template <class T>
+cudaError_t device_alloc(rt_ctx* ctx, T** p, size_t bytes, bool held = false) {
+  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  std::unique_lock<std::mutex> lock(ctx->mu, std::defer_lock);
+  if (!held) lock.lock();
+  if (drop_build_space(ctx) == 0) return e;
+  cudaGetLastError();
+  return cudaMalloc(reinterpret_cast<void**>(p), bytes);
+}
 
 inline size_t hit_bytes(uint32_t layout, uint32_t mode) {
   if (mode != 0) return ANY_HIT_BYTES;

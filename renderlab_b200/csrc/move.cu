@@ -249,7 +249,7 @@ extern "C" rt_status rt_scene_move_instances(rt_ctx* ctx, rt_scene* scene, const
     scene->device_bytes -= scene->move_bytes;
     ctx->scene_bytes -= scene->move_bytes;
     scene->move_bytes = 0;
-    if (cudaMalloc(&scene->d_move, need) != cudaSuccess) {
+    if (device_alloc(ctx, &scene->d_move, need, true) != cudaSuccess) {
       cudaGetLastError();
       return fail(ctx, RT_ERR_OOM, "move staging (%zu bytes)", need);
     }
@@ -276,7 +276,7 @@ extern "C" rt_status rt_scene_move_instances(rt_ctx* ctx, rt_scene* scene, const
       RT_CUDA(ctx, wait_changes(scene));
       RT_CUDA(ctx, cudaFree(scene->d_top_tree));
       scene->d_top_tree = nullptr, scene->top_cap = 0, scene->top_nodes = 0;
-      if (cudaMalloc(&scene->d_top_tree, 9 * cap) != cudaSuccess) {
+      if (device_alloc(ctx, &scene->d_top_tree, 9 * cap, true) != cudaSuccess) {
         cudaGetLastError();
         scene->d_top_tree = nullptr;
         return fail(ctx, RT_ERR_OOM, "top-level links");

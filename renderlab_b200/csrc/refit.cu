@@ -131,7 +131,7 @@ rt_status levels_of(rt_ctx* ctx, rt_scene* scene, const uint32_t* rec, RefitLeve
     }
   }
   // one allocation: parents, counters of a launch, inner child counts; or the order
-  if (cudaMalloc(&out.d_tree, tree ? 9 * (size_t)n : 4 * std::max<size_t>(order.size(), 1)) != cudaSuccess) {
+  if (device_alloc(ctx, &out.d_tree, tree ? 9 * (size_t)n : 4 * std::max<size_t>(order.size(), 1), true) != cudaSuccess) {
     cudaGetLastError();
     out.d_tree = nullptr;
     return fail(ctx, RT_ERR_OOM, "refit tree");

@@ -89,7 +89,7 @@ rt_status upload_top(rt_ctx* ctx, rt_scene* scene, const std::vector<uint32_t>& 
   if (nodes.empty()) return RT_OK;
   const size_t items_at = nodes.size(), total = items_at + std::max<size_t>(items.size(), 1);
   void* d = nullptr;
-  if (cudaMalloc(&d, total * 4) != cudaSuccess) {
+  if (device_alloc(ctx, &d, total * 4) != cudaSuccess) {
     cudaGetLastError();
     return fail(ctx, RT_ERR_OOM, "device allocation of %zu bytes for the 8-wide top level failed", total * 4);
   }
@@ -217,7 +217,7 @@ void rt_ctx_destroy(rt_ctx* ctx) {
   cudaFree(ctx->d_rays);
   cudaFree(ctx->d_hits);
   cudaFree(ctx->d_order_scratch);
-  for (auto& b : ctx->build_space) cudaFree(b.p);
+  drop_build_space(ctx);
   cudaFree(ctx->d_tables);
   cudaFreeHost(ctx->h_tables);
   for (cudaEvent_t e : ctx->table_done)
@@ -280,7 +280,7 @@ rt_status rt_scene_upload(rt_ctx* ctx, rt_layout layout, const uint32_t* words, 
     return fail(ctx, RT_ERR_LAYOUT, "scene rejected: %s", err.c_str());
   RT_CUDA(ctx, cudaSetDevice(ctx->device));
   const size_t bytes = std::max<size_t>(n_words, 4) * 4;
-  if (cudaMalloc(&s->d_words, bytes) != cudaSuccess) {
+  if (device_alloc(ctx, &s->d_words, bytes) != cudaSuccess) {
     cudaGetLastError();
     return fail(ctx, RT_ERR_OOM, "device allocation of %zu bytes failed", bytes);
   }
@@ -373,7 +373,7 @@ rt_status rt_scene_prepare(rt_ctx* ctx, rt_scene* scene, rt_kernel kernel) {
   const size_t nodes_at = 0, tris_at = up4(w8.nodes.size()), inst_at = tris_at + up4(w8.tris.size());
   const size_t total = inst_at + up4(std::max<size_t>(w8.inst.size(), 1));
   void* d = nullptr;
-  if (cudaMalloc(&d, total * 4) != cudaSuccess) {
+  if (device_alloc(ctx, &d, total * 4) != cudaSuccess) {
     cudaGetLastError();
     return fail(ctx, RT_ERR_OOM, "device allocation of %zu bytes for the 8-wide layout failed", total * 4);
   }
@@ -497,7 +497,7 @@ rt_status rt_scene_tune_top(rt_ctx* ctx, rt_scene* scene, const uint32_t* budget
     cudaFree(d_rays);
     cudaFree(d_hits);
   };
-  if (cudaMalloc(&d_rays, rays.size() * 4) != cudaSuccess || cudaMalloc(&d_hits, hit_words * 4 * (size_t)n) != cudaSuccess ||
+  if (device_alloc(ctx, &d_rays, rays.size() * 4) != cudaSuccess || device_alloc(ctx, &d_hits, hit_words * 4 * (size_t)n) != cudaSuccess ||
       cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess || cudaEventCreate(&e0) != cudaSuccess ||
       cudaEventCreate(&e1) != cudaSuccess || cudaMemcpy(d_rays, rays.data(), rays.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess) {
     cudaGetLastError();
@@ -628,7 +628,7 @@ rt_status ensure_order_scratch(rt_ctx* ctx, uint32_t n) {
   cudaFree(ctx->d_order_scratch);
   ctx->d_order_scratch = nullptr;
   ctx->order_scratch_bytes = 0;
-  if (cudaMalloc(&ctx->d_order_scratch, need) != cudaSuccess) {
+  if (device_alloc(ctx, &ctx->d_order_scratch, need, true) != cudaSuccess) {
     cudaGetLastError();
     return fail(ctx, RT_ERR_OOM, "ordering scratch of %zu bytes", need);
   }
@@ -658,6 +658,15 @@ rt_status rt_order_rays(rt_ctx* ctx, const rt_scene* scene, const rt_ray* d_rays
   return RT_OK;
 }
 
+rt_status rt_ctx_trim(rt_ctx* ctx, uint64_t* freed) {
+  if (!ctx) return RT_ERR_INVALID_ARG;
+  std::lock_guard<std::mutex> lock(ctx->mu);
+  RT_CUDA(ctx, cudaSetDevice(ctx->device));
+  const size_t bytes = drop_build_space(ctx);
+  if (freed) *freed = bytes;
+  return RT_OK;
+}
+
 rt_status rt_ctx_reserve(rt_ctx* ctx, uint32_t max_rays) {
   if (!ctx) return RT_ERR_INVALID_ARG;
   std::lock_guard<std::mutex> lock(ctx->mu);
@@ -673,8 +682,8 @@ rt_status rt_ctx_reserve(rt_ctx* ctx, uint32_t max_rays) {
   cudaFree(ctx->d_hits);
   ctx->d_rays = ctx->d_hits = nullptr;
   ctx->stage_rays = 0;
-  if (cudaMalloc(&ctx->d_rays, RT_HOST_STAGES * want * RAY_BYTES) != cudaSuccess ||
-      cudaMalloc(&ctx->d_hits, RT_HOST_STAGES * want * GI_HIT_BYTES) != cudaSuccess) {
+  if (device_alloc(ctx, &ctx->d_rays, RT_HOST_STAGES * want * RAY_BYTES, true) != cudaSuccess ||
+      device_alloc(ctx, &ctx->d_hits, RT_HOST_STAGES * want * GI_HIT_BYTES, true) != cudaSuccess) {
     cudaGetLastError();
     return fail(ctx, RT_ERR_OOM, "staging allocation for %zu rays failed", want);
   }

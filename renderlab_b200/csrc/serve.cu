@@ -258,6 +258,7 @@ rt_status rt_server_create(rt_ctx* ctx, const rt_server_desc* desc, rt_server** 
     return fail(ctx, RT_ERR_OOM, "the launch slots alone (%zu bytes) exceed the HBM budget", srv->slot_bytes * desc->slots);
   }
   RT_CUDA(ctx, cudaSetDevice(ctx->device));
+  rt_ctx_trim(ctx, nullptr);  // the budget knows scenes and slots alone
   srv->slots.resize(desc->slots);
   for (uint32_t i = 0; i < desc->slots; ++i) {
     Slot& s = srv->slots[i];
@@ -265,8 +266,8 @@ rt_status rt_server_create(rt_ctx* ctx, const rt_server_desc* desc, rt_server** 
     s.id = i;
     const size_t hit_bytes = srv->slot_bytes - (size_t)desc->launch_rays * sizeof(rt_ray);
     if (cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc(&s.d_rays, (size_t)desc->launch_rays * sizeof(rt_ray)) != cudaSuccess ||
-        cudaMalloc(&s.d_hits, hit_bytes) != cudaSuccess) {
+        device_alloc(ctx, &s.d_rays, (size_t)desc->launch_rays * sizeof(rt_ray)) != cudaSuccess ||
+        device_alloc(ctx, &s.d_hits, hit_bytes) != cudaSuccess) {
       cudaGetLastError();
       free_slots(srv);
       delete srv;
@@ -284,6 +285,7 @@ rt_status rt_server_add_scene(rt_server* srv, rt_layout layout, const uint32_t* 
   rt_ctx* ctx = srv->ctx;
   if (layout == RT_LAYOUT_REFLECTION_BVH2 && srv->desc.kernel != RT_KERNEL_PLAIN)
     return fail(ctx, RT_ERR_UNSUPPORTED, "the legacy BVH2 layout is served by a PLAIN-kernel server");
+  rt_ctx_trim(ctx, nullptr);  // as rt_server_create
   rt_scene* scene = nullptr;
   rt_status st = rt_scene_upload(ctx, layout, words, n_words, &scene);
   if (st != RT_OK) return st;

@@ -379,7 +379,7 @@ __global__ void k_words(const Seg* __restrict__ segs, const uint32_t* __restrict
 
 class Scratch {
  public:
-  explicit Scratch(cudaStream_t s) : s_(s) {}
+  Scratch(rt_ctx* ctx, cudaStream_t s) : ctx_(ctx), s_(s) {}
   ~Scratch() {
     if (base_) {
       cudaStreamSynchronize(s_);
@@ -394,9 +394,10 @@ class Scratch {
     used_ += (n * sizeof(T) + 255) & ~(size_t)255;
     return p;
   }
-  cudaError_t allocate() { return cudaMalloc(&base_, size_); }
+  cudaError_t allocate() { return device_alloc(ctx_, &base_, size_, true); }
 
  private:
+  rt_ctx* ctx_;
   cudaStream_t s_;
   void* base_ = nullptr;
   size_t size_ = 0, used_ = 0;
@@ -423,7 +424,7 @@ rt_status tlas_build_device(rt_ctx* ctx, const uint32_t* d_box_words, size_t str
     RT_CUDA(ctx, cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, u32, u32, (int)(seg_cap + 1), st));
     RT_CUDA(ctx, cub::DeviceSegmentedSort::SortKeys(nullptr, sort_bytes, u64, u64, (int)n, (int)seg_cap, u32, u32, st));
   }
-  Scratch sc(st);
+  Scratch sc(ctx, st);
   sc.plan<uint32_t>(n);                  // instance permutation
   sc.plan<uint32_t>(n);                  // partition scratch
   sc.plan<Seg>(seg_cap);
@@ -570,7 +571,7 @@ rt_status rt_tlas_build_device(rt_ctx* ctx, const float* boxes, uint32_t n, int 
   } end{st};
   const size_t cap = (size_t)(n - 1) * NODE_WORDS;
   uint32_t* d = nullptr;
-  if (cudaMalloc(&d, 24 * (size_t)n + 4 * cap) != cudaSuccess) {
+  if (device_alloc(ctx, &d, 24 * (size_t)n + 4 * cap, true) != cudaSuccess) {
     cudaGetLastError();
     return fail(ctx, RT_ERR_OOM, "top-level build buffers for %u instances", n);
   }
