@@ -266,26 +266,110 @@ RT_DEV uint32_t gi_node(const uint32_t* __restrict__ w, GiLane<AM>& L, uint32_t 
   return next;
 }
 
+// gi_instance (gi_rays_software.wgsl:98-207) for an any-hit ray of a launch whose warps are full: true when
+// something in it blocks the ray. A loop of its own, every surviving child on the stack and words loaded
+// one by one: the shared steps took 2,477 us against 2,228 for 1M incoherent rays over 20 listed
+// instances, 919 against 869 over one mesh, 2,163 against 1,903 for camera rays under a top level of 500
+// (and 627 against 705 for 90,000 of them). Where few rays are spread over warps the wait for each load
+// counts, and the shared steps, which keep the next child in a register, are ahead (300 rays over one
+// mesh 76 us against 81, 20,000 under the top level 653 against 689).
+RT_DEV bool gi_blocked(const uint32_t* __restrict__ w, uint32_t i, const Ray& ray, F3 world_inv, uint32_t* stack, DevStatus* st) {
+  const size_t r = 16 + (size_t)i * 32;
+  if ((ld(w, r + 27) & 1u) != 0) return false;
+  const float lim = ray.tmax;  // nothing met yet
+  if (!(slab_near(ray.o, world_inv, ld3(w, r + 12), ld3(w, r + 15), ray.tmin, lim) <= lim)) return false;
+  const float r00 = ldf(w, r), r01 = ldf(w, r + 1), r02 = ldf(w, r + 2), r03 = ldf(w, r + 3);
+  const float r10 = ldf(w, r + 4), r11 = ldf(w, r + 5), r12 = ldf(w, r + 6), r13 = ldf(w, r + 7);
+  const float r20 = ldf(w, r + 8), r21 = ldf(w, r + 9), r22 = ldf(w, r + 10), r23 = ldf(w, r + 11);
+  const F3 o = {dot4p(r00, r01, r02, r03, ray.o), dot4p(r10, r11, r12, r13, ray.o), dot4p(r20, r21, r22, r23, ray.o)};
+  const F3 d = {dot3({r00, r01, r02}, ray.d), dot3({r10, r11, r12}, ray.d), dot3({r20, r21, r22}, ray.d)};
+  const F3 inv = safe_inverse(d);
+  const uint32_t nodes = ld(w, r + 18), leaves = ld(w, r + 19), positions = ld(w, r + 20), indices = ld(w, r + 21);
+  stack[0] = ld(w, r + 22);
+  uint32_t sp = 1;
+  while (sp > 0) {
+    const uint32_t child = stack[--sp];
+    if (child & LEAF) {
+      const size_t l = leaves + (size_t)(child & ~LEAF) * 2;
+      const uint32_t first = ld(w, l), count = ld(w, l + 1);
+      for (uint32_t k = 0; k < count; k += 6) {
+        const size_t x = (size_t)indices + first + k;
+        const bool two = k + 3 < count;
+        const size_t y = two ? x + 3 : x;
+        const uint32_t ia = ld(w, x), ib = ld(w, x + 1), ic = ld(w, x + 2);
+        const uint32_t ja = ld(w, y), jb = ld(w, y + 1), jc = ld(w, y + 2);
+        const F3 a = ld3(w, positions + (size_t)ia * 3), b = ld3(w, positions + (size_t)ib * 3),
+                 c = ld3(w, positions + (size_t)ic * 3);
+        const F3 a2 = ld3(w, positions + (size_t)ja * 3), b2 = ld3(w, positions + (size_t)jb * 3),
+                 c2 = ld3(w, positions + (size_t)jc * 3);
+        float t, u, v;
+        if (gi_triangle(o, d, a, b, c, ray.tmin, lim, t, u, v)) return true;
+        if (two && gi_triangle(o, d, a2, b2, c2, ray.tmin, lim, t, u, v)) return true;
+      }
+      continue;
+    }
+    const size_t n = nodes + (size_t)child * 16;
+    const F3 oq = ld3(w, n), step = ld3(w, n + 3);
+    uint32_t c[4] = {ld(w, n + 6), ld(w, n + 7), ld(w, n + 8), ld(w, n + 9)};
+    const uint32_t lx = ld(w, n + 10), ly = ld(w, n + 11), lz = ld(w, n + 12);
+    const uint32_t hx = ld(w, n + 13), hy = ld(w, n + 14), hz = ld(w, n + 15);
+    uint32_t tb[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      tb[s] = __float_as_uint(BIG);
+      if (c[s] == EMPTY) continue;
+      const uint32_t sh = 8 * s;
+      const F3 lo = {add(oq.x, mul(step.x, (float)((lx >> sh) & 0xffu))), add(oq.y, mul(step.y, (float)((ly >> sh) & 0xffu))),
+                     add(oq.z, mul(step.z, (float)((lz >> sh) & 0xffu)))};
+      const F3 hi = {add(oq.x, mul(step.x, (float)((hx >> sh) & 0xffu))), add(oq.y, mul(step.y, (float)((hy >> sh) & 0xffu))),
+                     add(oq.z, mul(step.z, (float)((hz >> sh) & 0xffu)))};
+      tb[s] = __float_as_uint(slab_near(o, inv, lo, hi, ray.tmin, lim));
+    }
+    // (distance bits, child), descending: gi_rays_software.wgsl:191-197
+#define RT_SW(a, b)                          \
+  if (tb[a] < tb[b]) {                       \
+    uint32_t x = tb[a]; tb[a] = tb[b]; tb[b] = x; \
+    x = c[a]; c[a] = c[b]; c[b] = x;         \
+  }
+    RT_SW(0, 1) RT_SW(2, 3) RT_SW(0, 2) RT_SW(1, 3) RT_SW(1, 2)
+#undef RT_SW
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      if (__uint_as_float(tb[s]) <= lim && c[s] != EMPTY) {
+        if (sp < STACK) stack[sp++] = c[s];
+        else atomicAdd(&st->stack_drops, 1ull);
+      }
+    }
+  }
+  return false;
+}
+
 // gi_traverse (gi_rays_software.wgsl:217-279) of one ray.
-template <int AM>
+template <int AM, bool SPREAD>
 RT_DEV void gi_traverse(const uint32_t* __restrict__ w, GiLane<AM>& L, DevStatus* st) {
   L.world_inv = safe_inverse(L.ray.d);
   L.best = GiNear{L.ray.tmax, 0.0f, 0.0f, EMPTY, 0u};
   uint32_t stack[STACK];
   auto instance = [&](uint32_t i) {  // true when an any-hit ray is blocked
-    if (!gi_enter<AM>(w, L, i)) return false;
-    for (;;) {
-      uint32_t next = EMPTY;
-      if (L.cur & LEAF) {
-        if (gi_leaf<AM>(w, L, L.cur)) return true;
-      } else {
-        next = gi_node<AM>(w, L, L.cur, stack, st);
+    if constexpr (AM == 1 && !SPREAD) {
+      if (!gi_blocked(w, i, L.ray, L.world_inv, stack, st)) return false;
+      L.best.inst = i;
+      return true;
+    } else {
+      if (!gi_enter<AM>(w, L, i)) return false;
+      for (;;) {
+        uint32_t next = EMPTY;
+        if (L.cur & LEAF) {
+          if (gi_leaf<AM>(w, L, L.cur)) return true;
+        } else {
+          next = gi_node<AM>(w, L, L.cur, stack, st);
+        }
+        if (next == EMPTY) {
+          if (L.sp == 0) return false;
+          next = stack[--L.sp];
+        }
+        L.cur = next;
       }
-      if (next == EMPTY) {
-        if (L.sp == 0) return false;
-        next = stack[--L.sp];
-      }
-      L.cur = next;
     }
   };
   const uint32_t instances = ld(w, 0), top = ld(w, 1);
@@ -311,7 +395,7 @@ RT_DEV void gi_traverse(const uint32_t* __restrict__ w, GiLane<AM>& L, DevStatus
 // Resident blocks of 128 threads an SM. Closest hits (72 registers): 6, 7 and 8 give 2.17, 2.10 and 2.15
 // ms for 1M GI rays over 250k triangles, 559, 538 and 539 us for 1M camera rays there (reflection).
 // Any hit (64 registers): 7, 8, 9 and 10 give 1.87, 1.76, 1.75 and 1.79 ms for 1M shadow rays there.
-constexpr int PLAIN_MIN_BLOCKS = 7, PLAIN_ANY_BLOCKS = 8;
+constexpr int PLAIN_MIN_BLOCKS = 7, PLAIN_ANY_BLOCKS = 8, PLAIN_FEW_BLOCKS = 5;  // FEW: see run_gi_closest
 
 // The ray of this thread: `width` rays to a warp, in its first lanes (n: none).
 RT_DEV uint32_t plain_ray(uint32_t width, uint32_t n) {
@@ -320,14 +404,15 @@ RT_DEV uint32_t plain_ray(uint32_t width, uint32_t n) {
   return lane < width && i < n ? (uint32_t)i : n;
 }
 
-template <int AM, class Src>
-__global__ void __launch_bounds__(128, AM ? PLAIN_ANY_BLOCKS : PLAIN_MIN_BLOCKS) k_gi_plain(const uint32_t* __restrict__ w, const Src src, uint32_t n, uint32_t width,
-                                                  DevStatus* st) {
+// SPREAD: its warps hold few rays each.
+template <int AM, class Src, int BLOCKS, bool SPREAD = false>
+__global__ void __launch_bounds__(128, BLOCKS) k_gi_plain(const uint32_t* __restrict__ w, const Src src, uint32_t n, uint32_t width,
+                                                          DevStatus* st) {
   const uint32_t i = plain_ray(width, n);
   if (i == n) return;
   GiLane<AM> L;
   L.ray = fetch(src, i, L);
-  gi_traverse<AM>(w, L, st);
+  gi_traverse<AM, SPREAD>(w, L, st);
   gi_finish<AM>(w, L, src);
 }
 

@@ -1,58 +1,26 @@
 // Launchers for the FAST kernels: persistent grids sized to fill every SM once.
 #include <cuda_runtime.h>
 
-#include <map>
-#include <mutex>
-
 #include "kernels/cells.cuh"
 #include "kernels/fast.cuh"
 #include "launch.hpp"
+#include "spread.hpp"
 
 namespace rtl {
 
 namespace {
 constexpr int FAST_BLOCK = 128;
 
-// Resident blocks of `kernel` on the current device, cached per (kernel, device) under a lock:
-// kernels of one signature share this template instance but can differ in registers, and
-// rt_trace_static calls arrive from any thread without a context lock.
-template <class K>
-cudaError_t resident_blocks(K kernel, uint32_t& out) {
-  static std::mutex mu;
-  static std::map<std::pair<const void*, int>, uint32_t> cached;
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  const auto key = std::make_pair(reinterpret_cast<const void*>(kernel), dev);
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = cached.find(key);
-    if (it != cached.end()) {
-      out = it->second;
-      return cudaSuccess;
-    }
-  }
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, FAST_BLOCK, 0)) != cudaSuccess) return e;
-  out = (uint32_t)sms * (uint32_t)(per_sm > 0 ? per_sm : 1);
-  std::lock_guard<std::mutex> lock(mu);
-  cached[key] = out;
-  return cudaSuccess;
-}
-
-// The launch's grid and the lanes of each warp that take rays. A launch that does not fill the GPU
-// is bound by its longest rays' chains of loads, and a warp's lanes delay one another where they
-// part; so its rays are spread over half of the resident warps, in as few lanes each as hold them.
-// 4,096 GI rays over a 250k-triangle scene: 159 us against 196 with all 32 lanes; 10,000 (GI
-// layout): 151 against 162; from about 65,000 rays on both are the same.
+// The launch's grid and the lanes of each warp that take rays: rays are spread over half of the
+// resident warps (spread_width). 4,096 GI rays over a 250k-triangle scene: 159 us against 196 with
+// all 32 lanes; 10,000 (GI layout): 151 against 162; from about 65,000 rays on both are the same.
 template <class K>
 cudaError_t grid_for(K kernel, uint32_t n, dim3& grid, uint32_t& width) {
   uint32_t full = 0;
-  cudaError_t e = resident_blocks(kernel, full);
+  cudaError_t e = resident_blocks(kernel, FAST_BLOCK, full);
   if (e != cudaSuccess) return e;
   constexpr uint32_t warps = FAST_BLOCK / 32;
-  width = 1;
-  while (width < 32 && (uint64_t)full * warps * width < 2 * (uint64_t)n) width *= 2;
+  width = spread_width((uint64_t)full * warps / 2, n);
   const uint32_t need = (uint32_t)(((uint64_t)n + warps * width - 1) / (warps * width));
   grid = dim3(need < full ? need : full);
   return cudaSuccess;

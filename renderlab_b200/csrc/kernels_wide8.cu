@@ -1,10 +1,8 @@
 // Launchers for the WIDE8 kernels.
-#include <map>
-#include <mutex>
-
 #include "kernels/cells.cuh"
 #include "kernels/wide8.cuh"
 #include "launch.hpp"
+#include "spread.hpp"
 
 namespace rtl {
 
@@ -12,45 +10,16 @@ namespace {
 constexpr int W8_BLOCK = 128;
 }
 
-// Resident blocks of `kernel` on the current device: one cache per kernel, since instances of one
-// signature (the same function-pointer type) can differ in registers and shared memory.
-template <class K>
-cudaError_t resident(K kernel, uint32_t& out) {
-  static std::mutex mu;
-  static std::map<std::pair<const void*, int>, uint32_t> cached;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  const auto key = std::make_pair(reinterpret_cast<const void*>(kernel), dev);
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = cached.find(key);
-    if (it != cached.end()) {
-      out = it->second;
-      return cudaSuccess;
-    }
-  }
-  int sms = 0, per_sm = 0;
-  e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, W8_BLOCK, 0);
-  if (e != cudaSuccess) return e;
-  out = (uint32_t)sms * (uint32_t)(per_sm > 0 ? per_sm : 1);
-  std::lock_guard<std::mutex> lock(mu);
-  cached[key] = out;
-  return cudaSuccess;
-}
-
 template <class K, class Src>
 cudaError_t run(K kernel, const uint32_t* words, const rtk::W8View& v, const Src& src, unsigned int* counter, uint32_t n,
                 rtk::DevStatus* st, cudaStream_t stream, unsigned long long* cnt, uint32_t refill) {
   uint32_t full = 0;
-  cudaError_t e = resident(kernel, full);
+  cudaError_t e = resident_blocks(kernel, W8_BLOCK, full);
   if (e != cudaSuccess) return e;
-  // a launch that does not fill the resident warps spreads its rays over half of them, in as few lanes
-  // each as hold them (3,000 GI rays over 250k triangles: 97 -> 81 us, 20,000: 117 -> 114)
+  // rays spread over half of the resident warps (spread_width): 3,000 GI rays over 250k triangles 97 -> 81
+  // us, 20,000 117 -> 114
   constexpr uint32_t warps = W8_BLOCK / 32;
-  uint32_t width = 1;
-  while (width < 32 && (uint64_t)full * warps * width < 2 * (uint64_t)n) width *= 2;
+  const uint32_t width = spread_width((uint64_t)full * warps / 2, n);
   const uint32_t need = (uint32_t)(((uint64_t)n + warps * width - 1) / (warps * width));
   if ((e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), stream)) != cudaSuccess) return e;
   kernel<<<need < full ? need : full, W8_BLOCK, 0, stream>>>(words, v, src, counter, n, st, cnt, refill < width ? refill : width,
@@ -189,7 +158,7 @@ template <class K, class Src>
 cudaError_t run_packet(K kernel, const uint32_t* words, const rtk::W8View& v, const Src& src, unsigned int* counter,
                        uint32_t n, rtk::DevStatus* st, cudaStream_t stream) {
   uint32_t full = 0;
-  cudaError_t e = resident(kernel, full);
+  cudaError_t e = resident_blocks(kernel, W8_BLOCK, full);
   if (e != cudaSuccess) return e;
   const uint32_t need = (n + W8_BLOCK - 1) / W8_BLOCK;
   if ((e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), stream)) != cudaSuccess) return e;
