@@ -207,14 +207,53 @@ __device__ __forceinline__ void write_children(Seg* segs, uint32_t lv0, uint32_t
   segs[next + 2 * r + 1] = Seg{mid, g.e, g.depth + 1, own};
 }
 
+// A barrier of the `warps` warps that share a range (group `g` of the block).
+__device__ __forceinline__ void group_sync(uint32_t g, uint32_t warps) {
+  asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(warps * 32) : "memory");
+}
+
 // A range of at most SMALL triangles split down to its leaves by one block, level by level in shared
 // memory, a warp to a range. (A launch per level with a block to a range and one thread sweeping
-// the planes: 20 launches and 975 us of a 250k-triangle build; one launch and 430 us so.)
+// the planes: 20 launches and 975 us of a 250k-triangle build; one launch and 430 us so.) A median split
+// sorts its range, which is too long for one warp while a level has few: up to half as many ranges as
+// warps share the warps evenly. Median builds of 2,048 and 8,000
+// triangles: 1,132 -> 685 and 1,527 -> 1,079 us (a launch per level: 834 and 1,232).
 struct SmallRange {
   uint32_t b, e, seg, owner;
 };
+
+// Sorts n keys by the threads `at` of `step`, `sync` between the steps: bitonic, the places past the range
+// left out.
+template <class Sync>
+__device__ __forceinline__ void bitonic_sort(unsigned long long* key, uint32_t n, uint32_t at, uint32_t step, Sync sync) {
+  uint32_t n2 = 1;
+  while (n2 < n) n2 <<= 1;
+  for (uint32_t size = 2; size <= n2; size <<= 1)
+    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+      for (uint32_t k = at; k < n; k += step) {
+        const uint32_t p = stride == size >> 1 ? k ^ (size - 1) : k ^ stride;  // each merge starts mirrored
+        if (p > k && p < n) {
+          const unsigned long long u = key[k], v = key[p];
+          if (u > v) key[k] = v, key[p] = u;
+        }
+      }
+      sync();
+    }
+}
+
+// The two halves of a range of the block: their records, and those that split again in the next list.
+__device__ __forceinline__ void push_halves(Seg* segs, uint32_t* seg_count, uint32_t base, uint32_t depth, const SmallRange& x,
+                                            uint32_t mid, SmallRange* list, uint32_t* count) {
+  const uint32_t at = atomicAdd(seg_count, 2u), own = (depth & 1u) ? x.owner : x.seg;
+  segs[at] = Seg{base + x.b, base + mid, depth + 1, own};
+  segs[at + 1] = Seg{base + mid, base + x.e, depth + 1, own};
+  if (mid - x.b > LEAF_TRIS) list[atomicAdd(count, 1u)] = SmallRange{x.b, mid, at, own};
+  if (x.e - mid > LEAF_TRIS) list[atomicAdd(count, 1u)] = SmallRange{mid, x.e, at + 1, own};
+}
+
+template <bool SAH>
 __global__ void __launch_bounds__(SMALL_WARPS * 32) k_split_small(Seg* __restrict__ segs, const float* __restrict__ cen,
-                                                                  const uint32_t* __restrict__ tbk, uint32_t* __restrict__ perm, int sah,
+                                                                  const uint32_t* __restrict__ tbk, uint32_t* __restrict__ perm,
                                                                   uint32_t* __restrict__ seg_count, uint32_t* __restrict__ too_deep) {
   constexpr uint32_t MOST = SMALL / (LEAF_TRIS + 1) + 1;  // ranges of one level that split
   const Seg g = segs[blockIdx.x];
@@ -224,18 +263,49 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32) k_split_small(Seg* __restric
   __shared__ unsigned long long skey[SMALL];  // a median split's keys; an SAH one's scattered triangles
   __shared__ uint32_t cnt[SMALL_WARPS][3 * BINS], bl[SMALL_WARPS][3 * BINS * 3], bh[SMALL_WARPS][3 * BINS * 3];
   __shared__ SmallRange list[2][MOST];
-  __shared__ uint32_t count[2];
+  __shared__ uint32_t count[2], box[SMALL_WARPS][6];
   const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid & 31;
   for (uint32_t k = tid; k < len; k += SMALL_WARPS * 32) sp[k] = perm[g.b + k];
   if (tid == 0) list[0][0] = SmallRange{0, len, blockIdx.x, g.owner}, count[0] = 1, count[1] = 0;
   __syncthreads();
   uint32_t cur = 0;
   for (uint32_t depth = g.depth; count[cur] != 0; ++depth, cur ^= 1) {
-    if (sah && depth >= TOO_DEEP) {
+    if (SAH && depth >= TOO_DEEP) {
       if (tid == 0) *too_deep = 1;
       return;
     }
-    for (uint32_t r = warp; r < count[cur]; r += SMALL_WARPS) {
+    uint32_t groups = 1;  // warps of a group: SMALL_WARPS / groups
+    while (!SAH && groups < count[cur]) groups *= 2;
+    const bool shared = !SAH && groups <= SMALL_WARPS / 2;
+    const uint32_t warps = shared ? SMALL_WARPS / groups : 1, group = warp / warps;
+    if (shared && group < count[cur]) {
+      const SmallRange x = list[cur][group];
+      const uint32_t n = x.e - x.b, at = tid - group * warps * 32, step = warps * 32;
+      uint32_t l[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, h[3] = {0u, 0u, 0u};
+      for (uint32_t k = x.b + at; k < x.e; k += step)
+        for (int a = 0; a < 3; ++a) {
+          const uint32_t v = okey(cen[3 * (size_t)sp[k] + a]);
+          l[a] = min(l[a], v), h[a] = max(h[a], v);
+        }
+      for (int a = 0; a < 3; ++a) {
+        l[a] = __reduce_min_sync(0xffffffffu, l[a]), h[a] = __reduce_max_sync(0xffffffffu, h[a]);
+        if (lane == 0) box[warp][a] = l[a], box[warp][3 + a] = h[a];
+      }
+      group_sync(group, warps);
+      float lo[3], hi[3];
+      for (int a = 0; a < 3; ++a) {
+        for (uint32_t v = group * warps; v < (group + 1) * warps; ++v) l[a] = min(l[a], box[v][a]), h[a] = max(h[a], box[v][3 + a]);
+        lo[a] = unkey(l[a]), hi[a] = unkey(h[a]);
+      }
+      const int axis = choose(lo, hi, nullptr, nullptr, nullptr, n, false).axis;
+      unsigned long long* key = skey + x.b;
+      for (uint32_t k = at; k < n; k += step) key[k] = median_key(cen, sp[x.b + k], axis);
+      group_sync(group, warps);
+      bitonic_sort(key, n, at, step, [&] { group_sync(group, warps); });
+      for (uint32_t k = at; k < n; k += step) sp[x.b + k] = (uint32_t)key[k];
+      if (at == 0) push_halves(segs, seg_count, g.b, depth, x, x.b + n / 2, list[cur ^ 1], &count[cur ^ 1]);
+    }
+    for (uint32_t r = shared ? count[cur] : warp; r < count[cur]; r += SMALL_WARPS) {
       const SmallRange x = list[cur][r];
       const uint32_t n = x.e - x.b;
       uint32_t l[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, h[3] = {0u, 0u, 0u};
@@ -246,7 +316,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32) k_split_small(Seg* __restric
         }
       float lo[3], hi[3];
       for (int a = 0; a < 3; ++a) lo[a] = unkey(__reduce_min_sync(0xffffffffu, l[a])), hi[a] = unkey(__reduce_max_sync(0xffffffffu, h[a]));
-      if (sah) {
+      if (SAH) {
         for (uint32_t k = lane; k < 3 * BINS * 3; k += 32) {
           bl[warp][k] = 0xffffffffu, bh[warp][k] = 0u;
           if (k < 3 * BINS) cnt[warp][k] = 0u;
@@ -266,7 +336,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32) k_split_small(Seg* __restric
         }
         __syncwarp();
       }
-      const Choice c = choose(lo, hi, cnt[warp], bl[warp], bh[warp], n, sah != 0);
+      const Choice c = choose(lo, hi, cnt[warp], bl[warp], bh[warp], n, SAH);
       uint32_t mid;
       if (c.kind == KIND_SAH) {  // stable partition, 32 triangles at a time
         uint32_t* tmp = reinterpret_cast<uint32_t*>(skey + x.b);  // in the range's own part
@@ -284,34 +354,16 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32) k_split_small(Seg* __restric
         __syncwarp();
         for (uint32_t k = lane; k < n; k += 32) sp[x.b + k] = tmp[k];
         mid = x.b + c.left;
-      } else {  // bitonic sort of (centroid key, triangle), the places past the range left out
+      } else {  // sorted by (centroid key, triangle)
         unsigned long long* key = skey + x.b;
         for (uint32_t k = lane; k < n; k += 32) key[k] = median_key(cen, sp[x.b + k], c.axis);
         __syncwarp();
-        uint32_t n2 = 1;
-        while (n2 < n) n2 <<= 1;
-        for (uint32_t size = 2; size <= n2; size <<= 1)
-          for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-            for (uint32_t k = lane; k < n; k += 32) {
-              const uint32_t p = stride == size >> 1 ? k ^ (size - 1) : k ^ stride;  // each merge starts mirrored
-              if (p > k && p < n) {
-                const unsigned long long u = key[k], v = key[p];
-                if (u > v) key[k] = v, key[p] = u;
-              }
-            }
-            __syncwarp();
-          }
+        bitonic_sort(key, n, lane, 32, [] { __syncwarp(); });
         for (uint32_t k = lane; k < n; k += 32) sp[x.b + k] = (uint32_t)key[k];
         mid = x.b + n / 2;
       }
       __syncwarp();
-      if (lane == 0) {
-        const uint32_t at = atomicAdd(seg_count, 2u), own = (depth & 1u) ? x.owner : x.seg;
-        segs[at] = Seg{g.b + x.b, g.b + mid, depth + 1, own};
-        segs[at + 1] = Seg{g.b + mid, g.b + x.e, depth + 1, own};
-        if (mid - x.b > LEAF_TRIS) list[cur ^ 1][atomicAdd(&count[cur ^ 1], 1u)] = SmallRange{x.b, mid, at, own};
-        if (x.e - mid > LEAF_TRIS) list[cur ^ 1][atomicAdd(&count[cur ^ 1], 1u)] = SmallRange{mid, x.e, at + 1, own};
-      }
+      if (lane == 0) push_halves(segs, seg_count, g.b, depth, x, mid, list[cur ^ 1], &count[cur ^ 1]);
     }
     __syncthreads();
     if (tid == 0) count[cur] = 0;
@@ -843,7 +895,8 @@ rt_status rt_blas_build_device(rt_ctx* ctx, const float* positions, uint32_t n_p
     if (!over[1]) {
       over[0] = lv0 + width;
       RT_CUDA(ctx, cudaMemcpyAsync(d_count + 2, over, 8, cudaMemcpyHostToDevice, st));
-      k_split_small<<<over[0], SMALL_WARPS * 32, 0, st>>>(d_segs, d_cen, d_tbk, d_perm, sah ? 1 : 0, d_count + 2, d_count + 3);
+      (sah ? k_split_small<true> : k_split_small<false>)<<<over[0], SMALL_WARPS * 32, 0, st>>>(d_segs, d_cen, d_tbk, d_perm, d_count + 2,
+                                                                                               d_count + 3);
       RT_CUDA(ctx, cudaGetLastError());
       RT_CUDA(ctx, cudaMemcpyAsync(over, d_count + 2, 8, cudaMemcpyDeviceToHost, st));
       RT_CUDA(ctx, cudaStreamSynchronize(st));
