@@ -42,8 +42,10 @@ constexpr uint32_t W8_SSTACK = 16;
 // memory at 7; smaller batches over 200 and 600 instances 1,198 and 994 us against 1,278 and 1,099.
 // The packet walk (W8P_MIN_BLOCKS, 72 registers, both in local memory, about 140 bytes of spills):
 // 3.01, 2.93, 2.88 and 3.12 ms for 4.19M camera rays at 5, 6, 7 and 8 blocks, and 3.2 ms at 5 to 7 with
-// both in registers.
-constexpr int W8_BLOCKS = 5, W8P_MIN_BLOCKS = 7;
+// both in registers. Its reflection any-hit instance spills 168 bytes at 7, where the others spill 140, and
+// takes 6 blocks (80 registers): 1M rays over one mesh 1,554 -> 1,405 us, over 500 instances 15.5 -> 15.3 ms,
+// 5,000 there 1,403 -> 1,298.
+constexpr int W8_BLOCKS = 5, W8P_MIN_BLOCKS = 7, W8P_RS_ANY_BLOCKS = 6;
 
 // Opt-in device counters of the WIDE8 walk (diagnostics and the bytes-per-ray roofline).
 enum W8Count { W8C_RAYS, W8C_TOP_NODES, W8C_INSTANCE_TESTS, W8C_NODES, W8C_LEAVES, W8C_TRIS, W8C_RETESTS, W8C_FINAL64, W8C_N };
@@ -1052,7 +1054,7 @@ RT_DEV uint32_t w8_packet_top(const uint32_t* __restrict__ w, size_t n, const W8
 // the visit order (conservative boxes, ties resolved in f64 on (t, instance, triangle)), so each
 // ray gets the hit the per-ray walk finds.
 template <uint32_t LAYOUT, int AM, int BLOCK, class Src>
-__global__ void __launch_bounds__(BLOCK, W8P_MIN_BLOCKS) k_wide8_packet(const uint32_t* __restrict__ w, W8View V, const Src src,
+__global__ void __launch_bounds__(BLOCK, LAYOUT == 1 && AM == 1 ? W8P_RS_ANY_BLOCKS : W8P_MIN_BLOCKS) k_wide8_packet(const uint32_t* __restrict__ w, W8View V, const Src src,
                                                            unsigned int* __restrict__ counter, uint32_t n, DevStatus* st) {
   __shared__ W8Decoded decoded[BLOCK / 32];
   W8Decoded& D = decoded[threadIdx.x / 32];
