@@ -16,7 +16,7 @@ cudaError_t run_gi_closest(const SceneView& s, const Src& src, uint32_t n, rtk::
   if (e == cudaSuccess) e = resident_blocks(few, PLAIN_BLOCK, full_few);
   if (e != cudaSuccess) return e;
   const uint64_t warps = (uint64_t)full * (PLAIN_BLOCK / 32), warps_few = (uint64_t)full_few * (PLAIN_BLOCK / 32);
-  const uint32_t width = spread_width(warps, n), width_few = spread_width(warps_few, n);
+  const uint32_t width = plain_width(warps, n), width_few = spread_width(warps_few, n);
   if (n <= warps_few * width_few && (width_few == width || width_few >= 16))
     return run_plain_at(few, width_few, s, src, n, st, stream);
   return run_plain_at(many, width, s, src, n, st, stream);
@@ -28,7 +28,7 @@ cudaError_t run_gi_any(const SceneView& s, const Src& src, uint32_t n, rtk::DevS
   uint32_t full = 0;
   const cudaError_t e = resident_blocks(full_warps, PLAIN_BLOCK, full);
   if (e != cudaSuccess) return e;
-  const uint32_t width = spread_width((uint64_t)full * (PLAIN_BLOCK / 32), n);
+  const uint32_t width = plain_width((uint64_t)full * (PLAIN_BLOCK / 32), n);
   if (width < 16) return run_plain_at(rtk::k_gi_plain<1, Src, rtk::PLAIN_ANY_BLOCKS, true>, width, s, src, n, st, stream);
   return run_plain_at(full_warps, width, s, src, n, st, stream);
 }

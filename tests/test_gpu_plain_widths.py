@@ -15,8 +15,8 @@ from .test_gpu_wide8_schedule import _words
 pytestmark = pytest.mark.gpu
 
 SMS = 148
-# rays at which 5, 7 and 8 blocks of 4 warps an SM are full with 1, 8, 16 and 32 rays a warp
-EDGES = sorted({SMS * 4 * blocks * width for blocks in (5, 7, 8) for width in (1, 8, 16, 32)})
+# rays at which 5, 7 and 8 blocks of 4 warps an SM are full with 1 (and a quarter more), 8, 16 and 32 rays a warp
+EDGES = sorted({int(SMS * 4 * blocks * width) for blocks in (5, 7, 8) for width in (1, 1.25, 8, 16, 32)})
 
 
 @pytest.mark.parametrize("layout", [A.LAYOUT_GI, A.LAYOUT_REFLECTION])
