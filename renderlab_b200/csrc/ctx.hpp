@@ -184,6 +184,17 @@ inline cudaError_t wait_changes(const rt_scene* scene) {
   return e;
 }
 
+// after_changes on a stream, with this id, that does not capture; `n`: the changes so far.
+inline cudaError_t after_changes_on(const rt_scene* scene, cudaStream_t s, unsigned long long id, uint64_t n) {
+  if (id == scene->change_stream.load(std::memory_order_relaxed)) return cudaSuccess;  // in the stream's own order
+  OutsideCapture guard;
+  const cudaError_t e = cudaEventQuery(scene->changed);
+  if (e == cudaSuccess) scene->settled.store(n, std::memory_order_relaxed);
+  if (e != cudaErrorNotReady) return e;
+  cudaGetLastError();
+  return cudaStreamWaitEvent(s, scene->changed, 0);
+}
+
 // What is queued on `s` from here on runs after the scene's last move or refit, whichever stream that
 // took: every launch that reads the scene's words is ordered so. A launch being captured runs
 // later, on any stream, so there the host waits. Once the change is known to be over, two loads.
@@ -196,19 +207,13 @@ inline cudaError_t after_changes(const rt_scene* scene, cudaStream_t s) {
     return wait_changes(scene);
   }
   unsigned long long id = 0;
-  cudaError_t e = cudaStreamGetId(s, &id);
-  if (e != cudaSuccess || id == scene->change_stream.load(std::memory_order_relaxed)) return e;
-  OutsideCapture guard;
-  e = cudaEventQuery(scene->changed);
-  if (e == cudaSuccess) scene->settled.store(n, std::memory_order_relaxed);
-  if (e != cudaErrorNotReady) return e;
-  cudaGetLastError();
-  return cudaStreamWaitEvent(s, scene->changed, 0);
+  const cudaError_t e = cudaStreamGetId(s, &id);
+  return e != cudaSuccess ? e : after_changes_on(scene, s, id, n);
 }
 
 // Around the launches that change a scene's words on `s` (the caller holds the context's lock):
-// start() queues them after earlier changes and after the default stream's work (a traversal there
-// that still reads the words), and the end of the scope marks them as the last change, on every
+// start(), on a stream that does not capture, queues them after earlier changes and after the default
+// stream's work (a traversal there that still reads the words), and the end of the scope marks them as the last change, on every
 // return path.
 class Change {
  public:
@@ -222,7 +227,8 @@ class Change {
         if (e != cudaSuccess) return e;
       }
     cudaError_t e = cudaStreamGetId(s_, &id_);
-    if (e == cudaSuccess) e = after_changes(scene_, s_);
+    const uint64_t n = scene_->changes.load(std::memory_order_relaxed);
+    if (e == cudaSuccess && scene_->settled.load(std::memory_order_relaxed) < n) e = after_changes_on(scene_, s_, id_, n);
     if (e == cudaSuccess && s_ != nullptr && s_ != cudaStreamLegacy) {
       e = cudaEventRecord(scene_->legacy, cudaStreamLegacy);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(s_, scene_->legacy, 0);

@@ -101,7 +101,8 @@ constexpr uint32_t TLAS_REFITS = 64;  // instance_bvh.rs:94
 bool move_instances(uint32_t layout, uint32_t* words, size_t n_words, const std::vector<Placement>& inst,
                     const std::vector<Aabb>& mesh_boxes, std::string& err);
 // A placement the packers skip or refuse: a zero determinant or a non-finite row (pack.cpp).
-bool is_singular(const Placement& g);
+bool is_singular(const float* model, const float* rows);
+inline bool is_singular(const Placement& g) { return is_singular(g.model, g.rows); }
 // The world box (with the layout's margin) of a placement of an object box (pack.cpp), as the
 // packers write instance words 12-17.
 void instance_box(uint32_t layout, const float* model, const Aabb& obj, float lo[3], float hi[3]);

@@ -29,14 +29,13 @@ void to_world(const float* m, const float* p, float* out) {
 
 }  // namespace
 
-bool is_singular(const Placement& g) {
-  const float* m = g.model;
+bool is_singular(const float* m, const float* rows) {
   double det = (double)m[0] * ((double)m[5] * m[10] - (double)m[6] * m[9]) -
                (double)m[1] * ((double)m[4] * m[10] - (double)m[6] * m[8]) +
                (double)m[2] * ((double)m[4] * m[9] - (double)m[5] * m[8]);
   if (det == 0.0) return true;
-  for (float r : g.rows)
-    if (!std::isfinite(r)) return true;
+  for (int k = 0; k < 12; ++k)
+    if (!std::isfinite(rows[k])) return true;
   return false;
 }
 

@@ -227,11 +227,8 @@ extern "C" rt_status rt_scene_move_instances(rt_ctx* ctx, rt_scene* scene, const
     return fail(ctx, RT_ERR_INVALID_ARG, "moved instances must be the scene's %u instances, in record order", count);
   for (uint32_t i = 0; i < n; ++i) {
     const rt_instance& s = instances[i];
-    rtb::Placement p;
-    std::copy(s.model, s.model + 12, p.model);
-    std::copy(s.rows, s.rows + 12, p.rows);
     if (s.mesh >= n_meshes) return fail(ctx, RT_ERR_INVALID_ARG, "instance %u: mesh %u of %u", i, s.mesh, n_meshes);
-    if (rtb::is_singular(p)) return fail(ctx, RT_ERR_LAYOUT, "instance %u: singular placement", i);
+    if (rtb::is_singular(s.model, s.rows)) return fail(ctx, RT_ERR_LAYOUT, "instance %u: singular placement", i);
   }
   if (n == 0) return RT_OK;
   // All that can be refused or fail comes before the first launch, and the refit count is written where
