@@ -1,16 +1,22 @@
 // GPU build of one mesh's BVH4-Q8 (near_field::build_bvh_sah / build_bvh, near_field.rs:172-436)
 // whose records equal the host builder's (host/blas.cpp), word for word.
 //
-// The host builder recurses depth first; this one splits level by level. Both give the same
-// tree, for four reasons:
+// The host builder recurses depth first; this one splits all large ranges of a level at once, and a range
+// of at most SMALL triangles down to its leaves by one block. Both give the same tree, for four reasons:
 //  * a split depends only on its own range of the triangle permutation, and its halves keep
 //    their input order (near_field.rs:361-364), so every range of one level splits in parallel
 //    and the permutation ends up as the host's, leaves in depth-first order;
 //  * the centroid and bin boxes are min/max reductions, taken here in any order through
 //    order-preserving integer keys. They can differ from the host's only in the sign of a zero
 //    bound, and that changes no bin, extent test, cost comparison or split;
-//  * the cost sweep runs on one thread per split, with the host's operations in the host's order;
+//  * the cost sweep runs on a warp, a bin to a lane. The boxes and counts on each side of a plane are
+//    scans of minima, maxima and integer sums, which no order changes but for the sign of a zero
+//    bound; each plane's cost is then formed by the host's operations in their order, and the choice
+//    keeps the host's rules for equal costs (the lowest axis and bin), infinities and NaN (a first NaN
+//    cost is replaced by none);
 //  * a median split sorts by (centroid, triangle), a key with no ties.
+// A block appends its ranges to the table in whatever order its warps finish: nothing is read from that
+// order, since ids and slots come from the ranges themselves (below).
 // A split of a range is a node group when its binary depth is even: its halves, and the halves of
 // those halves, are the node's children (near_field.rs:286-306). The node ids follow postorder,
 // which is the order of (range end, range length). A child's slot is its order by range start.

@@ -13,11 +13,12 @@
 // lanes waiting as well was slower (6.78, 6.35 and 6.23 against 6.08 ms there), and so were weights
 // by a step's length. Each is resident 7 times an SM (72 registers): 4, 5, 6 and 8 blocks gave 6.65,
 // 6.63, 6.10 and 6.12 against 6.09 ms; the closest hit therefore keeps no more than t, u, v and where
-// its triangle is, and the record is made when the ray ends. Together, before and after (us):
-//   gather of 16,384 cells over 400 instances, closest   9,530 -> 6,160
-//   16,384 cells x 40 lights, 250k triangles, any hit      508 ->   438
-//   1M GI rays, 250k triangles, GI / reflection          1,876 / 1,455 -> 1,320 / 1,000
-//   1M camera rays, the same scene                         989 /   765 ->   765 /   600
+// its triangle is, and the record is made when the ray ends. Together, before and after (us; the first two
+// by perf/cases.py, whose scenes differ by seed: the counters above are of another seed):
+//   gather of 16,384 cells over 400 instances, closest          12,288 -> 7,319
+//   16,384 cells x 40 lights, 250k triangles, any hit              533 ->   450
+//   1M rays, uniform directions, 250k cluster triangles, closest, GI / reflection  1,531 / 1,188 -> 1,066 / 837
+//   1M camera rays, the same scene                               1,053 /   811 ->   768 / 614
 #pragma once
 #include "plain.cuh"
 
@@ -50,10 +51,6 @@ RT_DEV uint32_t take_ray(const RayQueue& q, bool need, bool& drained) {
   return ((want >> lane & 1u) && idx < q.n) ? idx : EMPTY;
 }
 
-// ---------------------------------------------------------------- the walk's schedule
-
-// ---------------------------------------------------------------- reflection layout
-
 // The next item of the top level (or of the flat instance list).
 template <class Lane>
 RT_DEV void next_top(Lane& L, const uint32_t* top_stack, bool flat, uint32_t instances) {
@@ -74,6 +71,8 @@ RT_DEV void next_top(Lane& L, const uint32_t* top_stack, bool flat, uint32_t ins
   L.cur = item & ~LEAF;
   L.phase = (item & LEAF) ? PH_ENTER : PH_TOP;
 }
+
+// ---------------------------------------------------------------- reflection layout
 
 template <int AM, int BLOCK, class Src>
 __global__ void __launch_bounds__(BLOCK, FAST_MIN_BLOCKS)

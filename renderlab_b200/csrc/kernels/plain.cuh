@@ -6,10 +6,11 @@
 // restatement. Two safety rules the WGSL leaves to robust buffer access: a child id EMPTY is
 // never pushed, and a push onto a full stack is dropped and counted (DevStatus::stack_drops).
 //
-// The steps of a walk (instance entry, node, leaf) are shared with the FAST kernels: records and
-// nodes in 16-byte loads, slabs two children to an instruction, the GI hit record made when the
-// ray ends. 1M camera rays over 120,000 cube triangles (GI) 230 -> 191 us, over 250k cluster
-// triangles (reflection) 625 -> 541, 1M GI rays there (GI) 2,387 -> 2,160.
+// The steps of a walk (instance entry, node, leaf) are shared with the FAST kernels (but for GI any hits in
+// full warps: gi_blocked): records and nodes in 16-byte loads, slabs two children to an instruction,
+// the GI hit record made when the ray ends. Closest hits, 1M camera rays over 120,000 cube triangles (GI)
+// 234 -> 192 us, over 250k cluster triangles (reflection) 651 -> 553, 1M rays of uniform directions there
+// 2,221 -> 1,803 (GI) and 1,688 -> 1,410.
 #pragma once
 #include "common.cuh"
 
