@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <array>
 #include <atomic>
 #include <cstdarg>
 #include <map>
@@ -49,7 +50,7 @@ struct rt_scene {
   bool w8_top_valid = false;
   uint32_t w8_entries = 0;  // the top level's entries per instance (rt_scene_tune_top); 0: the context's
 
-  std::map<uint32_t, RefitLevels> refit;  // by the BLAS's node base word
+  std::map<std::array<uint32_t, 4>, RefitLevels> refit;  // by the words that name the BLAS's parts (see blas_of)
   // rt_scene_move_instances: staging for the moved instances and mesh boxes, and the top level's
   // links (see k_refit_top), made by the first move and by each rebuild.
   std::vector<char> move_stage;

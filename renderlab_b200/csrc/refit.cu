@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cfloat>
 #include <cmath>
 #include <vector>
@@ -42,6 +43,13 @@ __global__ void k_refit_triangles(View v, uint32_t n_tris) {
   }
 }
 
+// The words of a record that say where its BLAS's nodes, leaves, positions and indices (GI) or nodes and
+// triangles (reflection) lie; `r`: words 18 on.
+std::array<uint32_t, 4> blas_of(bool gi, const uint32_t* r) {
+  if (gi) return {r[0], r[1], r[2], r[3]};
+  return {r[0] & ~3u, r[1] & ~3u, 0u, 0u};
+}
+
 // Whether a leaf that no instance's root reaches lies inside the scene's words, as the upload's
 // admission checks those that one does (`words`: the scene's, read for the GI layout alone).
 bool leaf_inside(const rt_scene* scene, const uint32_t* rec, uint32_t c, const std::vector<uint32_t>& words) {
@@ -67,7 +75,7 @@ rt_status levels_of(rt_ctx* ctx, rt_scene* scene, const uint32_t* rec, RefitLeve
   for (size_t i = 0; i < scene->info.instances; ++i) {
     const uint32_t* r = scene->blas_words.data() + 6 * i;
     const uint32_t root = gi ? r[4] : r[2];
-    if ((gi ? r[0] : (r[0] & ~3u)) != nodes || root == EMPTY) continue;
+    if (blas_of(gi, r) != blas_of(gi, rec + 18) || root == EMPTY) continue;
     if (!(root & LEAF)) n = std::max(n, root + 1);  // postorder: the root is the last node
     else if (!gi) tris = std::max(tris, ((root & ~LEAF) >> 4) + (root & 15u));  // a single leaf: its triangles alone
   }
@@ -168,12 +176,13 @@ rt_status rt_scene_refit(rt_ctx* ctx, rt_scene* scene, uint32_t instance, const 
     RT_CUDA(ctx, cudaMemcpy(rec, scene->d_words + (gi ? 16 + 32 * (size_t)instance : 8 + 24 * (size_t)instance), sizeof rec,
                             cudaMemcpyDeviceToHost));
   const uint32_t base = gi ? rec[18] : (rec[18] & ~3u);
-  auto it = scene->refit.find(base);
+  const std::array<uint32_t, 4> key = blas_of(gi, rec + 18);
+  auto it = scene->refit.find(key);
   if (it == scene->refit.end()) {
     RefitLevels lv;
     rt_status st = levels_of(ctx, scene, rec, lv);
     if (st != RT_OK) return st;
-    it = scene->refit.emplace(base, std::move(lv)).first;
+    it = scene->refit.emplace(key, std::move(lv)).first;
   }
   const RefitLevels& lv = it->second;
   if (gi && n_positions != lv.position_count)

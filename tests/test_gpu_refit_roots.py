@@ -55,3 +55,37 @@ def test_every_root_is_refit(engine, layout, case):
             assert np.array_equal(got[after:], want[after:])
     finally:
         scene.release()
+
+
+def test_another_meshes_parts_are_left(engine):
+    """Two GI instances over the same nodes, the second with leaves and positions of its own: a refit of the
+    first, which enters a subtree, reads and writes its own parts alone."""
+    import torch
+    mesh = S.clusters(3000, stream=S.Stream(13))
+    blas = A.Blas(mesh.positions, mesh.indices)
+    inst = S.identity_instances(2)
+    inst.mesh[:] = 0
+    w = A.pack_scene(A.LAYOUT_GI, [blas], inst, tlas_mode=0)
+    base, leaves, root = int(w[16 + 18]), int(w[16 + 19]), int(w[16 + 22])
+    node = w[base:leaves].reshape(-1, 16)
+    sub = next(int(c) for c in node[root, 6:10] if 0 < c < root)
+    own = len(w)  # a second copy of all behind the nodes
+    w = np.concatenate([w, w[leaves:]])
+    w[16 + 22] = sub
+    w[48 + 19:48 + 22] += own - leaves
+    scene = engine.upload(A.LAYOUT_GI, w)
+    try:
+        for k in range(2):  # the second time from the kept topology
+            new = (mesh.positions * np.float32(1.5 + k)).astype(np.float32)
+            blas.refit(new)
+            want = A.pack_scene(A.LAYOUT_GI, [blas], inst, tlas_mode=0)
+            scene.refit(0, torch.from_numpy(new).cuda())
+            got, low = scene.words(), base + 16 * (sub + 1)
+            assert np.array_equal(got[base:low], want[base:low])
+            assert np.array_equal(got[low:leaves], w[low:leaves]) and np.array_equal(got[own:], w[own:])
+            assert np.array_equal(got[leaves:own], want[leaves:own])
+        scene.refit(1, torch.from_numpy(new).cuda())
+        got = scene.words()
+        assert np.array_equal(got[base:own], want[base:own]) and np.array_equal(got[own:], want[leaves:own])
+    finally:
+        scene.release()
