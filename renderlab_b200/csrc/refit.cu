@@ -131,12 +131,15 @@ rt_status levels_of(rt_ctx* ctx, rt_scene* scene, const uint32_t* rec, RefitLeve
   }
   out.tri_count = tris;
   if (!tree) {
-    out.level_start.assign(1, 0);
-    for (uint32_t h = 1; h <= top; ++h) {
-      for (uint32_t k = 0; k < n; ++k)
-        if (height[k] == h) order.push_back(k);
-      out.level_start.push_back((uint32_t)order.size());
-    }
+    std::vector<uint32_t>& start = out.level_start;  // height h + 1 at start[h] on
+    start.assign(top + 1, 0);
+    for (uint32_t h : height)
+      if (h) ++start[h];
+    for (uint32_t h = 1; h <= top; ++h) start[h] += start[h - 1];
+    order.resize(start[top]);
+    std::vector<uint32_t> next(start.begin(), start.end());
+    for (uint32_t k = 0; k < n; ++k)
+      if (height[k]) order[next[height[k] - 1]++] = k;
   }
   // one allocation: parents, counters of a launch, inner child counts; or the order
   if (device_alloc(ctx, &out.d_tree, tree ? 9 * (size_t)n : 4 * std::max<size_t>(order.size(), 1), true) != cudaSuccess) {
