@@ -83,7 +83,8 @@ constexpr uint8_t NEVER = 0xff;  // inner children of a node that is not refit
 // from the nodes without inner children; of a node's inner children the last one done takes the
 // node (done[], zeroed before the launch; nothing waits). An inner child's box is grown in slot order
 // as instance_bvh::refit_wide does. 2,500 instances, 6 heights: 40 us as a launch per height with a
-// thread a node, 16 so (the whole call, its copies included: 144 -> 62 us). `refits`: the header's count.
+// thread a node, 16 so (the whole call until the device is done: 144 -> 90 us, 52 of them on the host).
+// `refits`: the header's count.
 constexpr int TOP_BLOCK = 128;
 __global__ void __launch_bounds__(TOP_BLOCK) k_refit_top(uint32_t* __restrict__ w, uint32_t layout, size_t base, uint32_t n,
                                                          const uint32_t* __restrict__ parent,
